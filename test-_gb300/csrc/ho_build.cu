@@ -224,6 +224,218 @@ int launch_setup(ho_context* c) {
 }
 
 // ---------------------------------------------------------------------------
+// Isosurface exclusion certificates (iso_excluded reads them).
+//
+// For an element with map x(xi), let K be the inverse Jacobian of its
+// trilinear part at 0, x0 = x(0) and G(xi) = K (x(xi) - x0), and let beta bound
+// the infinity norm of G' - I over the cube |xi| <= R. A point x of the padded
+// box has |y| <= Y, y = K (x - x0).
+//  * xi -> xi - (G(xi) - y) contracts by beta on |xi| <= rho = Y / (1 - beta),
+//    so for rho <= R exactly one xi* in the cube maps to x, with |xi*| <= rho
+//    and |xi* - y| = |xi* - G(xi*)| <= beta rho = delta.
+//  * a Newton step from xi moves to an error of at most q |xi - xi*|, q =
+//    2 beta / (1 - beta), while the segment from xi to xi* stays in the cube.
+//    So from any start with |xi| <= S where rho + q (S + rho) <= R (the cold
+//    start 0 is one) the iterates approach xi*: where they stop, they are at
+//    xi*. No sample of a certified element converges anywhere else.
+// The field there is its trilinear part, exactly interpolated by the test,
+// plus the higher modes, at most H = sum |c_ijk| V_i V_j V_k over |xi| <= rho.
+// The bounds on the modes and their derivatives over [-r, r], r >= 1, follow
+// from phi_i = (i-1) / (2 (2i-1)) (L_{i-2} - L_i) and phi_i' = -(i-1)/2
+// L_{i-1} with Legendre polynomials L, which are largest at the end outside
+// [-1, 1] and at most 1 within. Margins of 0.01 in Y and rho, 5e-4 in delta and 1e-5
+// relative in H cover FP32 rounding here, in the test and in the solves.
+// ---------------------------------------------------------------------------
+constexpr int kCullWarps = 4;
+
+// Largest |phi_i| and |phi_i'| over [-r, r], r >= 1.
+__device__ __forceinline__ void mode_bounds(int i, float r, float& v, float& d) {
+  if (i < 2) {
+    v = 0.5f * (1.f + r);
+    d = 0.5f;
+    return;
+  }
+  float a = 1.f, b = r, c = r;  // L_{i-2}, L_{i-1}, L_i at r
+  for (int m = 2; m <= i; ++m) {
+    c = (static_cast<float>(2 * m - 1) * r * b - static_cast<float>(m - 1) * a) / static_cast<float>(m);
+    if (m < i) {
+      a = b;
+      b = c;
+    }
+  }
+  const float w = static_cast<float>(i - 1) / static_cast<float>(2 * i - 1);
+  // within [-1, 1]: 1/4 exactly for i = 2, and |L_{i-2} - L_i| <= 2
+  v = fmaxf(i == 2 ? 0.25f : w, 0.5f * w * (c - a));
+  d = 0.5f * static_cast<float>(i - 1) * b;
+}
+
+// One warp per element, its lanes over the coefficients; once per scene.
+template <int N>
+__global__ void __launch_bounds__(32 * kCullWarps) cull_kernel(const float* __restrict__ rec,
+                                                               const float* __restrict__ box, int64_t n_elem,
+                                                               float* __restrict__ cull) {
+  constexpr int S = N * N * N, RS = row_stride(N), BF = block_floats(N);
+  __shared__ float vb[kCullWarps][N], db[kCullWarps][N];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int64_t e = static_cast<int64_t>(blockIdx.x) * kCullWarps + wib;
+  if (e >= n_elem) return;
+  const float* r = rec + e * record_floats(N);
+  const auto wsum = [](float x) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    return x;
+  };
+  const auto fill = [&](float rad) {
+    __syncwarp();
+    if (lane < N) mode_bounds(lane, rad, vb[wib][lane], db[wib][lane]);
+    __syncwarp();
+  };
+  float c[3][8], f[8];
+  for (int v = 0; v < 8; ++v) {
+    const int at = (((v >> 2) * N + ((v >> 1) & 1)) * RS) + (v & 1);
+    for (int a = 0; a < 3; ++a) c[a][v] = r[a * BF + at];
+    f[v] = r[3 * BF + at];
+  }
+  float J[9], K[9];
+  for (int a = 0; a < 3; ++a)
+    for (int q = 0; q < 3; ++q) {
+      float s = 0.f;
+      for (int v = 0; v < 8; ++v) s += ((v >> q) & 1) ? c[a][v] : -c[a][v];
+      J[3 * a + q] = 0.125f * s;
+    }
+  invert3(J, K);
+  // x(0): phi_i(0) of the modes through vb
+  __syncwarp();
+  {
+    float b0[N];
+    basis_val<N>(0.f, b0);
+    if (lane == 0)
+      for (int i = 0; i < N; ++i) vb[wib][i] = b0[i];
+  }
+  __syncwarp();
+  float x0[3] = {0.f, 0.f, 0.f};
+  for (int q = lane; q < S; q += 32) {
+    const int i = q % N, j = (q / N) % N, k = q / (N * N);
+    const float w = vb[wib][i] * vb[wib][j] * vb[wib][k];
+    for (int a = 0; a < 3; ++a) x0[a] = fmaf(r[a * BF + (k * N + j) * RS + i], w, x0[a]);
+  }
+  for (int a = 0; a < 3; ++a) x0[a] = wsum(x0[a]);
+  const float* b = box + 6 * e;
+  float Y = 0.f;
+  bool ok = true;  // false for a NaN too (fmaxf drops one)
+  for (int a = 0; a < 3; ++a) {
+    float mid = 0.f, half = 0.f;
+    for (int q = 0; q < 3; ++q) {
+      mid += K[3 * a + q] * (0.5f * (b[q] + b[3 + q]) - x0[q]);
+      half += fabsf(K[3 * a + q]) * 0.5f * (b[3 + q] - b[q]);
+    }
+    ok = ok && fabsf(mid) + half < 20.f;
+    Y = fmaxf(Y, fabsf(mid) + half);
+  }
+  Y = 1.001f * Y + 0.01f;
+  float delta = -1.f, rho = 0.f, start = 0.f;
+  for (int attempt = 0; attempt < 3 && ok && delta < 0.f; ++attempt) {
+    const float R = fmaxf(1.f, Y * (attempt == 0 ? 1.2f : (attempt == 1 ? 1.5f : 2.f)));
+    fill(R);
+    float E[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int q = lane; q < S; q += 32) {
+      const int i = q % N, j = (q / N) % N, k = q / (N * N);
+      if (i < 2 && j < 2 && k < 2) continue;
+      const float* p = r + (k * N + j) * RS + i;
+      const float cx = p[0], cy = p[BF], cz = p[2 * BF];
+      const float vi = vb[wib][i], vj = vb[wib][j], vk = vb[wib][k];
+      const float w0 = db[wib][i] * vj * vk, w1 = vi * db[wib][j] * vk, w2 = vi * vj * db[wib][k];
+      for (int a = 0; a < 3; ++a) {
+        const float g = fabsf(K[3 * a] * cx + K[3 * a + 1] * cy + K[3 * a + 2] * cz);
+        E[3 * a] += g * w0;
+        E[3 * a + 1] += g * w1;
+        E[3 * a + 2] += g * w2;
+      }
+    }
+    float beta = 0.f;
+    bool tame = true;
+    for (int a = 0; a < 3; ++a) {
+      float row = 0.f;
+      for (int q = 0; q < 3; ++q) {
+        // the trilinear part's derivative along q: bilinear in the other two
+        // directions, so its extremes over the cube are at its edges
+        const int q1 = q == 0 ? 1 : 0, q2 = q == 2 ? 1 : 2;
+        float dv[4];
+        for (int s = 0; s < 4; ++s) {
+          const int lo = ((s & 1) << q1) | ((s >> 1) << q2), hi = lo | (1 << q);
+          dv[s] = 0.5f * (K[3 * a] * (c[0][hi] - c[0][lo]) + K[3 * a + 1] * (c[1][hi] - c[1][lo]) +
+                          K[3 * a + 2] * (c[2][hi] - c[2][lo]));
+        }
+        const float one = a == q ? 1.f : 0.f;
+        float m = 0.f;
+        for (int s = 0; s < 4; ++s) {
+          const float u = 0.5f + ((s & 1) ? 0.5f : -0.5f) * R, v = 0.5f + ((s >> 1) ? 0.5f : -0.5f) * R;
+          const float lo = dv[0] + u * (dv[1] - dv[0]), hi = dv[2] + u * (dv[3] - dv[2]);
+          const float dev = fabsf(lo + v * (hi - lo) - one);
+          tame = tame && dev < 0.3f;
+          m = fmaxf(m, dev);
+        }
+        row += m + wsum(E[3 * a + q]);
+      }
+      tame = tame && 1.001f * row + 1e-5f < 0.3f;
+      beta = fmaxf(beta, 1.001f * row + 1e-5f);
+    }
+    if (!tame) continue;
+    const float q = 2.f * beta / (1.f - beta);
+    rho = Y / (1.f - beta) + 0.01f;
+    start = fminf(R, (R - rho) / q - rho);
+    if (start >= 0.f) delta = beta * rho + 5e-4f;
+  }
+  float H = 0.f;
+  if (delta >= 0.f) {
+    const float rad = fmaxf(1.f, rho);
+    fill(rad);
+    for (int q = lane; q < S; q += 32) {
+      const int i = q % N, j = (q / N) % N, k = q / (N * N);
+      if (i < 2 && j < 2 && k < 2) continue;
+      H = fmaf(fabsf(r[3 * BF + (k * N + j) * RS + i]), vb[wib][i] * vb[wib][j] * vb[wib][k], H);
+    }
+    H = wsum(H);
+    float tri = 0.f;
+    for (int v = 0; v < 8; ++v) tri += fabsf(f[v]);
+    const float w = 0.5f * (1.f + rad);
+    H = 1.001f * H + 1e-5f * (tri * w * w * w + H) + 1e-7f;
+  }
+  if (lane == 0) {
+    float* o = cull + e * kCullFloats;
+    for (int q = 0; q < 9; ++q) o[q] = K[q];
+    for (int a = 0; a < 3; ++a) o[9 + a] = x0[a];
+    o[12] = delta;
+    o[13] = H;
+    o[14] = start;
+    o[15] = 0.f;
+    for (int v = 0; v < 8; ++v) o[16 + v] = f[v];
+  }
+}
+
+template <int N>
+static cudaError_t launch_cull_n(ho_context* c) {
+  const int64_t blocks = (c->n_elem + kCullWarps - 1) / kCullWarps;
+  cull_kernel<N><<<static_cast<unsigned>(blocks), 32 * kCullWarps, 0, c->stream>>>(c->d_rec, c->d_box, c->n_elem,
+                                                                                    c->d_cull);
+  return cudaGetLastError();
+}
+
+int launch_cull(ho_context* c) {
+  switch (c->N) {
+    case 2: return int(launch_cull_n<2>(c));
+    case 3: return int(launch_cull_n<3>(c));
+    case 4: return int(launch_cull_n<4>(c));
+    case 5: return int(launch_cull_n<5>(c));
+    case 6: return int(launch_cull_n<6>(c));
+    case 7: return int(launch_cull_n<7>(c));
+    case 8: return int(launch_cull_n<8>(c));
+    case 9: return int(launch_cull_n<9>(c));
+    default: return int(cudaErrorInvalidValue);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // LBVH
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {

@@ -48,6 +48,7 @@ void free_scene(ho_context* c) {
   cudaFree(c->d_box);
   cudaFree(c->d_hull);
   cudaFree(c->d_fbox);
+  cudaFree(c->d_cull);
   cudaFree(c->d_flags);
   cudaFree(c->d_own);
   cudaFree(c->d_nodes);
@@ -60,7 +61,7 @@ void free_scene(ho_context* c) {
   c->d_cord = nullptr;
   c->orders = 0;
   c->d_desc = nullptr;
-  c->d_rec = c->d_box = c->d_hull = c->d_fbox = nullptr;
+  c->d_rec = c->d_box = c->d_hull = c->d_fbox = c->d_cull = nullptr;
   c->d_flags = nullptr;
   c->d_own = nullptr;
   c->d_nodes = nullptr;
@@ -545,6 +546,7 @@ int ho_build_bvh(ho_context* c) {
   CK(cudaMalloc(&c->d_box, ne * 6 * sizeof(float)), "cudaMalloc(box)");
   CK(cudaMalloc(&c->d_hull, ne * 6 * sizeof(float)), "cudaMalloc(hull)");
   CK(cudaMalloc(&c->d_fbox, ne * ho::kFaceBoxFloats * sizeof(float)), "cudaMalloc(face boxes)");
+  CK(cudaMalloc(&c->d_cull, ne * ho::kCullFloats * sizeof(float)), "cudaMalloc(certificates)");
   CK(cudaMemcpyAsync(c->d_rec, rec.data(), rec.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream), "upload");
   CK(cudaMemcpyAsync(c->d_flags, flags.data(), ne * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream), "upload");
   CK(cudaMemcpyAsync(c->d_own, own.data(), ne * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream), "upload");
@@ -573,6 +575,8 @@ int ho_build_bvh(ho_context* c) {
   }
   rc = ho::launch_setup(c);
   if (rc) return cuda_fail(c, rc, "setup kernel");
+  rc = ho::launch_cull(c);
+  if (rc) return cuda_fail(c, rc, "certificate kernel");
   rc = ho::build_lbvh(c);
   if (rc) return cuda_fail(c, rc, "LBVH build");
   CK(cudaMalloc(&c->d_desc, ne * ho::kDescFloats * sizeof(float)), "cudaMalloc(descriptors)");
@@ -580,7 +584,7 @@ int ho_build_bvh(ho_context* c) {
   if (rc) return cuda_fail(c, rc, "descriptor kernel");
   if (c->bvh_depth + 2 > 64) return fail(c, HO_ERR_RANGE, "BVH deeper than the traversal stack");
   CK(cudaStreamSynchronize(c->stream), "sync");
-  c->device_bytes += static_cast<int64_t>(rec.size() * sizeof(float)) + ne * (4 + 4 + 1 + 24 + 24 + 144) +
+  c->device_bytes += static_cast<int64_t>(rec.size() * sizeof(float)) + ne * (4 + 4 + 1 + 24 + 24 + 144 + 4 * ho::kCullFloats) +
                      c->n_nodes * static_cast<int64_t>(sizeof(ho::BNode));
   c->built = true;
   return HO_OK;

@@ -667,6 +667,76 @@ __device__ bool find_iso_warp(const Elem<N, SM>& e, float3 o, float3 d, float t0
   return found;
 }
 
+// True when the isosurface search of a candidate's segment [te, tx] cannot
+// find a sign change, from the element's certificate (cull_kernel in
+// ho_build.cu has the proof): every sample whose Newton solve converges has
+// xi within delta of y = K (x - x0), which is linear in t, and a field value
+// within H of the trilinear interpolant of the element's corner values there.
+// So u - iso keeps one sign over the segment when those bounds clear the
+// isovalue on one side over the boxes around its four quarters (a trilinear
+// function on a box has its extremes at the box's corners), and the 17
+// samples, whatever subset of them converges, bracket nothing. A NaN
+// anywhere fails the comparisons: the search then runs.
+__device__ __forceinline__ bool iso_excluded(const float* __restrict__ cull, int elem, float3 o, float3 d, float te,
+                                             float tx, float iso, bool warm, const Pred& pr) {
+  const float4* c4 = reinterpret_cast<const float4*>(cull + static_cast<int64_t>(elem) * kCullFloats);
+  const float4 k0 = __ldg(c4), k1 = __ldg(c4 + 1), k2 = __ldg(c4 + 2), k3 = __ldg(c4 + 3);
+  if (!(k3.x >= 0.f)) return false;
+  if (warm) {  // the network's starts must lie where the certificate's Newton bound holds
+    const float3 a = pr.at(te), b = pr.at(tx);
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(b.x))),
+                          fmaxf(fabsf(b.y), fabsf(b.z)));
+    if (!(m <= k3.z)) return false;
+  }
+  const float K[9] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w, k2.x};
+  const float3 q = make_float3(o.x - k2.y, o.y - k2.z, o.z - k2.w);
+  // rounding of the sample points o + t d and of y (the candidate's box keeps
+  // a margin of 0.01 in y for it)
+  const float kn = fmaxf(fabsf(K[0]) + fabsf(K[1]) + fabsf(K[2]),
+                         fmaxf(fabsf(K[3]) + fabsf(K[4]) + fabsf(K[5]), fabsf(K[6]) + fabsf(K[7]) + fabsf(K[8])));
+  const float big = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z))) + fmaxf(fabsf(te), fabsf(tx)) *
+                        fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
+  const float slop = 1e-6f * big * kn;
+  if (!(slop <= 5e-3f)) return false;
+  const float dl = k3.x + slop;
+  float y0[3], ys[3];  // y at te, and over a quarter of the segment
+  const float qt = 0.25f * (tx - te);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    y0[a] = K[3 * a] * (q.x + te * d.x) + K[3 * a + 1] * (q.y + te * d.y) + K[3 * a + 2] * (q.z + te * d.z);
+    ys[a] = (K[3 * a] * d.x + K[3 * a + 1] * d.y + K[3 * a + 2] * d.z) * qt;
+  }
+  const float4 f0 = __ldg(c4 + 4), f1 = __ldg(c4 + 5);
+  const float lim_lo = iso - k3.y, lim_hi = iso + k3.y;
+  bool above = true, below = true;
+#pragma unroll 1
+  for (int s = 0; s < 4 && (above || below); ++s) {
+    float w[3][2];  // interpolation weights of the box's two sides per axis
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float p = y0[a] + s * ys[a], r = p + ys[a];
+      w[a][0] = 0.5f + 0.5f * (fminf(p, r) - dl);
+      w[a][1] = 0.5f + 0.5f * (fmaxf(p, r) + dl);
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const float e0 = f0.x + w[0][x] * (f0.y - f0.x), e1 = f0.z + w[0][x] * (f0.w - f0.z),
+                  e2 = f1.x + w[0][x] * (f1.y - f1.x), e3 = f1.z + w[0][x] * (f1.w - f1.z);
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const float g0 = e0 + w[1][y] * (e1 - e0), g1 = e2 + w[1][y] * (e3 - e2);
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const float v = g0 + w[2][z] * (g1 - g0);
+          above = above && v > lim_hi;
+          below = below && v < lim_lo;
+        }
+      }
+    }
+  }
+  return above || below;
+}
+
 // Slab test clipped to [tmin, tmax] (high_order.h:115-152).
 __device__ __forceinline__ bool ray_box(float3 o, float3 d, const float* lo, const float* hi, float tmin, float tmax,
                                         float& te, float& tx) {

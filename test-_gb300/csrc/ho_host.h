@@ -163,6 +163,7 @@ struct ho_context {
   float* d_box = nullptr;         // n_elem * 6 padded sampled boxes
   float* d_hull = nullptr;        // n_elem * 6 Bernstein hull boxes
   float* d_fbox = nullptr;        // n_elem * 36 face hull boxes
+  float* d_cull = nullptr;        // n_elem * kCullFloats isosurface exclusion certificates
   uint32_t* d_flags = nullptr;    // n_elem
   int32_t* d_own = nullptr;       // n_elem
   ho::BNode* d_nodes = nullptr;   // max(1, n_elem - 1)
@@ -241,6 +242,7 @@ struct ho_context {
 namespace ho {
 // Kernel launchers (ho_build.cu / ho_trace.cu). Return cudaError_t as int.
 int launch_setup(ho_context* c);
+int launch_cull(ho_context* c);
 int build_lbvh(ho_context* c);
 // LBVH over n device boxes (lo xyz, hi xyz); leaf aux bits from d_flags
 // (nullable). Allocates *nodes_out (max(1, n - 1) nodes).

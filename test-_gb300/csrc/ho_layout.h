@@ -107,6 +107,11 @@ constexpr int kStatusRoundGuard = 4;
 // Per-face hull boxes: 6 faces x (lo xyz, hi xyz).
 constexpr int kFaceBoxFloats = 36;
 
+// Per element, what the isosurface exclusion test reads (ho_build.cu,
+// cull_kernel; ho_device.cuh, iso_excluded): K (9, row-major), x0 (3), delta,
+// H, S, one unused, the field's 8 corner values. delta < 0: no certificate.
+constexpr int kCullFloats = 24;
+
 // Largest supported modes per direction (P = 8).
 constexpr int kMaxModes = 9;
 // Pair slots per warp of the round kernel: the per-warp shared memory (element

@@ -125,6 +125,7 @@ extern "C" int ho_intersect_device_noalloc(ho_context* c, int64_t n, const float
   P.fbox = c->d_fbox;
   P.box = c->d_box;
   P.flags = c->d_flags;
+  P.cull = c->d_cull;
   P.rays = rays_dev;
   P.n_rays = n;
   P.cam = CamArgs{};

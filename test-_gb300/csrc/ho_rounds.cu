@@ -116,67 +116,112 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
                                     int32_t* __restrict__ pelem, uint32_t* __restrict__ prank,
                                     uint32_t* __restrict__ ecount, unsigned* __restrict__ ctr) {
   const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= *P.qcount) return;
-  RayState& r = st[item];
-  if (r.done) return;
-  float3 o, d;
-  float iso;
-  bool iso_on;
-  query_ray(P, P.work[item], o, d, iso, iso_on);
+  const int lane = threadIdx.x & 31;
+  bool live = item < *P.qcount && !st[item].done;
+  if (!__any_sync(kFull, live)) return;
   Work w;
-  float2* kb = P.kbuf + static_cast<int64_t>(item) * kCandK;
-  for (int guard = 0; guard < (1 << 20); ++guard) {
-    if (r.cursor >= kCandK) {
-      if (!r.ovf) {
-        r.done = 1;
+  RoundPair p;
+  int elem = -1;
+  if (live) {
+    RayState& r = st[item];
+    float3 o, d;
+    float iso;
+    bool iso_on;
+    query_ray(P, P.work[item], o, d, iso, iso_on);
+    float2* kb = P.kbuf + static_cast<int64_t>(item) * kCandK;
+    const float best_t = r.best.t;
+    int cursor = r.cursor, pass = r.pass, ke = r.ke;
+    float kt = r.kt;
+    bool ovf = r.ovf != 0, done = false;
+    for (int guard = 0; guard < (1 << 20); ++guard) {
+      if (cursor >= kCandK) {
+        if (!ovf) {
+          done = true;
+          break;
+        }
+        float bt[kCandK];
+        int be[kCandK];
+        if (!collect(P, o, d, best_t, kt, ke, bt, be, ovf, w)) {
+          atomicOr(&P.stats->status, kStatusStackOverflow);
+          r.best.flags |= HO_FLAG_INCOMPLETE;
+          done = true;
+          break;
+        }
+        for (int j = 0; j < kCandK; ++j) kb[j] = make_float2(bt[j], __int_as_float(be[j]));
+        cursor = 0;
+        ++pass;
+        ++w.restarts;
+        r.best.flags |= HO_FLAG_OVERFLOW;
+      }
+      const float2 c = kb[cursor];
+      const float ct = c.x;
+      const int ce = __float_as_int(c.y);
+      if (ce == INT_MAX || ct > best_t) {
+        done = true;
         break;
       }
-      float bt[kCandK];
-      int be[kCandK];
-      bool overflow;
-      if (!collect(P, o, d, r.best.t, r.kt, r.ke, bt, be, overflow, w)) {
-        atomicOr(&P.stats->status, kStatusStackOverflow);
-        r.best.flags |= HO_FLAG_INCOMPLETE;
-        r.done = 1;
-        break;
+      const int j = cursor;
+      ++cursor;
+      kt = ct;
+      ke = ce;
+      const float* b = P.box + 6 * static_cast<int64_t>(ce);
+      const float lo[3] = {__ldg(b), __ldg(b + 1), __ldg(b + 2)};
+      const float hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
+      float te, tx;
+      if (!ray_box(o, d, lo, hi, 0.001f, best_t, te, tx)) continue;
+      // a candidate that can hold neither a root nor a face hit ends here,
+      // without a place in a round
+      Pred pr;
+      pr.on = false;
+      if (P.pred && pass == 0 && j < kPredK && item < P.pred_items &&
+          P.cand_e[static_cast<int64_t>(item) * kPredK + j] == ce) {
+        const float* y = P.pred + (static_cast<int64_t>(item) * kPredK + j) * kMlpOut;
+        pr.on = true;
+        pr.xi_in = make_float3(y[0], y[1], y[2]);
+        pr.v = make_float3(y[3], y[4], y[5]);
+        pr.k = __ldg(P.desc + static_cast<int64_t>(ce) * kDescFloats + 45);
+        pr.te = te;
       }
-      for (int j = 0; j < kCandK; ++j) kb[j] = make_float2(bt[j], __int_as_float(be[j]));
-      r.ovf = overflow ? 1 : 0;
-      r.cursor = 0;
-      ++r.pass;
-      ++w.restarts;
-      r.best.flags |= HO_FLAG_OVERFLOW;
-    }
-    const float2 c = kb[r.cursor];
-    const float ct = c.x;
-    const int ce = __float_as_int(c.y);
-    if (ce == INT_MAX || ct > r.best.t) {
-      r.done = 1;
+      const bool scan = iso_on && needs_iso(P, ce, o, d, te, tx, iso, pr);
+      if (!scan && !any_face(P.fbox, ce, o, d, best_t)) {
+        ++w.cand;
+        w.culled += 6;
+        continue;
+      }
+      p.item = static_cast<int32_t>(item);
+      p.j = (pass == 0 ? j : kPairPred) | (scan ? 0 : kPairNoIso);
+      p.te = te;
+      p.tx = tx;
+      elem = ce;
       break;
     }
-    const int j = r.cursor;
-    ++r.cursor;
-    r.kt = ct;
-    r.ke = ce;
-    const float* b = P.box + 6 * static_cast<int64_t>(ce);
-    const float lo[3] = {__ldg(b), __ldg(b + 1), __ldg(b + 2)};
-    const float hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
-    float te, tx;
-    if (!ray_box(o, d, lo, hi, 0.001f, r.best.t, te, tx)) continue;
-    const unsigned k = atomicAdd(ctr, 1u);
-    RoundPair p;
-    p.item = static_cast<int32_t>(item);
-    p.j = r.pass == 0 ? j : -1;
-    p.te = te;
-    p.tx = tx;
-    pairs[k] = p;
-    pelem[k] = ce;
-    prank[k] = atomicAdd(&ecount[ce], 1u);
-    break;
+    r.cursor = cursor;
+    r.pass = pass;
+    r.kt = kt;
+    r.ke = ke;
+    r.ovf = ovf ? 1 : 0;
+    if (done) r.done = 1;
   }
-  if (w.nodes || w.restarts) {
-    atomicAdd(&P.stats->c[ST_NODES], static_cast<unsigned long long>(w.nodes));
-    atomicAdd(&P.stats->c[ST_RESTART], static_cast<unsigned long long>(w.restarts));
+  const unsigned m = __ballot_sync(kFull, elem >= 0);
+  if (m) {
+    const int leader = __ffs(m) - 1;
+    unsigned base = 0;
+    if (lane == leader) base = atomicAdd(ctr, static_cast<unsigned>(__popc(m)));
+    base = __shfl_sync(kFull, base, leader);
+    if (elem >= 0) {
+      const unsigned k = base + __popc(m & ((1u << lane) - 1u));
+      pairs[k] = p;
+      pelem[k] = elem;
+      prank[k] = atomicAdd(&ecount[elem], 1u);
+    }
+  }
+  const unsigned nodes = __reduce_add_sync(kFull, w.nodes), restarts = __reduce_add_sync(kFull, w.restarts),
+                 cand = __reduce_add_sync(kFull, w.cand), culled = __reduce_add_sync(kFull, w.culled);
+  if (lane == 0) {
+    if (nodes) atomicAdd(&P.stats->c[ST_NODES], static_cast<unsigned long long>(nodes));
+    if (restarts) atomicAdd(&P.stats->c[ST_RESTART], static_cast<unsigned long long>(restarts));
+    if (cand) atomicAdd(&P.stats->c[ST_CAND], static_cast<unsigned long long>(cand));
+    if (culled) atomicAdd(&P.stats->c[ST_CULLED], static_cast<unsigned long long>(culled));
   }
 }
 

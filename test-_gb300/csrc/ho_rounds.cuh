@@ -59,9 +59,12 @@ struct RoundCfg {
 // A (ray, candidate) pair of one round, as the gather pass writes it.
 struct RoundPair {
   int32_t item;  // queue item (ray)
-  int32_t j;     // index of the candidate in the ray's list (learned prediction lookup)
+  int32_t j;     // kPairPred bits: index of the candidate in the ray's list (learned prediction lookup,
+                 // kPairPred: none); kPairNoIso: the isosurface search was excluded
   float te, tx;  // segment: the candidate's padded box clipped to [0.001, closest hit]
 };
+
+constexpr int kPairPred = 0xff, kPairNoIso = 0x100;
 
 struct RoundBatch {
   int32_t elem;
@@ -450,10 +453,11 @@ __device__ __noinline__ int admit_pair(WS* Wp, const RoundParams* P, int slot, R
   p.best_t = P->state[rp.item].best.t;
   p.item = rp.item;
   p.elem = elem;
-  int fl = (has_field ? 1 : 0) | (iso_on ? 2 : 0);
-  if (L && rp.j >= 0 && rp.j < kPredK && static_cast<unsigned>(rp.item) < P->pred_items &&
-      P->cand_e[static_cast<int64_t>(rp.item) * kPredK + rp.j] == elem) {
-    const float* y = P->pred + (static_cast<int64_t>(rp.item) * kPredK + rp.j) * kMlpOut;
+  int fl = (has_field ? 1 : 0) | (iso_on && !(rp.j & kPairNoIso) ? 2 : 0);
+  const int pj = rp.j & kPairPred;
+  if (L && pj < kPredK && static_cast<unsigned>(rp.item) < P->pred_items &&
+      P->cand_e[static_cast<int64_t>(rp.item) * kPredK + pj] == elem) {
+    const float* y = P->pred + (static_cast<int64_t>(rp.item) * kPredK + pj) * kMlpOut;
     p.pxi[0] = y[0]; p.pxi[1] = y[1]; p.pxi[2] = y[2];
     p.pv[0] = y[3]; p.pv[1] = y[4]; p.pv[2] = y[5];
     p.pk = __ldg(P->desc + static_cast<int64_t>(elem) * kDescFloats + 45);
@@ -1097,13 +1101,6 @@ __global__ void __launch_bounds__(kTraceBlock) tail_kernel(TraceParams P, RaySta
         const float hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
         float te, tx;
         if (ray_box(o, d, lo, hi, 0.001f, best.t, te, tx)) {
-          const float4* src = reinterpret_cast<const float4*>(P.rec + static_cast<int64_t>(ce) * record_floats(N));
-          __syncwarp();
-          for (int q4 = lane; q4 < record_floats(N) / 4; q4 += 32) slot4[q4] = __ldg(src + q4);
-          __syncwarp();
-          Elem<N, true> el;
-          el.c = CoefRef<true>{slot_addr};
-          el.has_field = (__ldg(P.flags + ce) & 1u) != 0;
           Pred pr;
           pr.on = false;
           if (L && pass == 0 && j < kPredK && item < P.pred_items &&
@@ -1115,7 +1112,22 @@ __global__ void __launch_bounds__(kTraceBlock) tail_kernel(TraceParams P, RaySta
             pr.k = __ldg(P.desc + static_cast<int64_t>(ce) * kDescFloats + 45);
             pr.te = te;
           }
-          visit_warp<N, L>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats, ce, o, d, te, tx, iso, iso_on,
+          kt = ct;
+          ke = ce;
+          const bool scan = iso_on && needs_iso(P, ce, o, d, te, tx, iso, pr);
+          if (!scan && !any_face(P.fbox, ce, o, d, best.t)) {
+            ++wu.cand;
+            wu.culled += 6;
+            continue;
+          }
+          const float4* src = reinterpret_cast<const float4*>(P.rec + static_cast<int64_t>(ce) * record_floats(N));
+          __syncwarp();
+          for (int q4 = lane; q4 < record_floats(N) / 4; q4 += 32) slot4[q4] = __ldg(src + q4);
+          __syncwarp();
+          Elem<N, true> el;
+          el.c = CoefRef<true>{slot_addr};
+          el.has_field = (__ldg(P.flags + ce) & 1u) != 0;
+          visit_warp<N, L>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats, ce, o, d, te, tx, iso, scan,
                            best, w, wu, pr, &r.tie);
         }
         kt = ct;

@@ -163,6 +163,7 @@ static int trace_hexes(ho_context* c, const TraceArgs& a, cudaStream_t s) {
   P.fbox = c->d_fbox;
   P.box = c->d_box;
   P.flags = c->d_flags;
+  P.cull = c->d_cull;
   P.rays = a.rays;
   P.n_rays = a.n_rays;
   P.cam = cam_args(a);

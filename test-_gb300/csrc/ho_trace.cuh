@@ -40,6 +40,7 @@ struct TraceParams {
   const float* __restrict__ fbox;
   const float* __restrict__ box;
   const uint32_t* __restrict__ flags;
+  const float* __restrict__ cull;  // isosurface exclusion certificates
   const float* __restrict__ rays;  // explicit rays or nullptr
   int64_t n_rays;
   CamArgs cam;
@@ -294,6 +295,23 @@ __device__ __forceinline__ HitState miss_state() {
   return b;
 }
 
+// Does a candidate's isosurface search have to run on [te, tx]? (iso on; pr:
+// the network's starts, when it has them.)
+__device__ __forceinline__ bool needs_iso(const TraceParams& P, int elem, float3 o, float3 d, float te, float tx,
+                                          float iso, const Pred& pr) {
+  return (__ldg(P.flags + elem) & 1u) != 0 && !iso_excluded(P.cull, elem, o, d, te, tx, iso, pr.on, pr);
+}
+
+// May any face of the element be hit on [0.001, tmax] (exact culling by the
+// faces' hull boxes)? A candidate that may not, and whose isosurface search is
+// excluded, ends without a solve: nothing of its record is read.
+__device__ __forceinline__ bool any_face(const float* __restrict__ fbox, int elem, float3 o, float3 d, float tmax) {
+  const float* b = fbox + static_cast<int64_t>(elem) * kFaceBoxFloats;
+  for (int f = 0; f < 6; ++f)
+    if (face_may_hit(b, f, o, d, 0.001f, tmax)) return true;
+  return false;
+}
+
 // Pass 2, persistent, one warp per queued query: ordered candidates, each
 // visited with its independent Newton solves spread over the lanes.
 template <int N, bool LEARNED>
@@ -365,14 +383,6 @@ __global__ void __launch_bounds__(kTraceBlock) isect_kernel(TraceParams P) {
         const float hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
         float te, tx;
         if (ray_box(o, d, lo, hi, 0.001f, best.t, te, tx)) {
-          // stage the candidate's record in this warp's shared-memory slot
-          const float4* src = reinterpret_cast<const float4*>(P.rec + static_cast<int64_t>(ce) * record_floats(N));
-          __syncwarp();
-          for (int q4 = lane; q4 < record_floats(N) / 4; q4 += 32) slot4[q4] = __ldg(src + q4);
-          __syncwarp();
-          Elem<N, true> el;
-          el.c = CoefRef<true>{slot_addr};
-          el.has_field = (__ldg(P.flags + ce) & 1u) != 0;
           Pred pr;
           pr.on = false;
           if (LEARNED && pass == 0 && j < kPredK && P.cand_e[static_cast<int64_t>(item) * kPredK + j] == ce) {
@@ -383,8 +393,24 @@ __global__ void __launch_bounds__(kTraceBlock) isect_kernel(TraceParams P) {
             pr.k = __ldg(P.desc + static_cast<int64_t>(ce) * kDescFloats + 45);
             pr.te = te;
           }
+          kt = ct;
+          ke = ce;
+          const bool scan = iso_on && needs_iso(P, ce, o, d, te, tx, iso, pr);
+          if (!scan && !any_face(P.fbox, ce, o, d, best.t)) {
+            ++wu.cand;
+            wu.culled += 6;
+            continue;
+          }
+          // stage the candidate's record in this warp's shared-memory slot
+          const float4* src = reinterpret_cast<const float4*>(P.rec + static_cast<int64_t>(ce) * record_floats(N));
+          __syncwarp();
+          for (int q4 = lane; q4 < record_floats(N) / 4; q4 += 32) slot4[q4] = __ldg(src + q4);
+          __syncwarp();
+          Elem<N, true> el;
+          el.c = CoefRef<true>{slot_addr};
+          el.has_field = (__ldg(P.flags + ce) & 1u) != 0;
           visit_warp<N, LEARNED>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats, ce, o, d, te, tx, iso,
-                                 iso_on, best, w, wu, pr);
+                                 scan, best, w, wu, pr);
         }
         kt = ct;
         ke = ce;

@@ -103,7 +103,7 @@ __global__ void round_init_kernel(RayState* __restrict__ st, const uint8_t* __re
   r.done = 0;
   r.ovf = kovf[i];
   r.its = 0;
-  r.pad = 0;
+  r.seen = 0;
   st[i] = r;
 }
 
@@ -111,10 +111,14 @@ __global__ void round_init_kernel(RayState* __restrict__ st, const uint8_t* __re
 // the ray meets before the closest hit so far (the candidate loop of the
 // reference's traversal, FEM-AABB/raytracer.cu:117-356, in ascending
 // (entry t, element) order). A ray whose list was cut at kCandK walks the
-// tree again for the candidates after the last visited one.
+// tree again for the candidates after the last visited one. limit: visited
+// candidates of a ray before the tail takes it (0: no tail), counted whether
+// they were solved or ended here, so which of the two kernels solves a
+// candidate does not depend on how many ended here (their face Newtons
+// differ in the last bits on a few rays).
 __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, RoundPair* __restrict__ pairs,
                                     int32_t* __restrict__ pelem, uint32_t* __restrict__ prank,
-                                    uint32_t* __restrict__ ecount, unsigned* __restrict__ ctr) {
+                                    uint32_t* __restrict__ ecount, unsigned* __restrict__ ctr, int limit) {
   const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   bool live = item < *P.qcount && !st[item].done;
@@ -130,10 +134,10 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
     query_ray(P, P.work[item], o, d, iso, iso_on);
     float2* kb = P.kbuf + static_cast<int64_t>(item) * kCandK;
     const float best_t = r.best.t;
-    int cursor = r.cursor, pass = r.pass, ke = r.ke;
+    int cursor = r.cursor, pass = r.pass, ke = r.ke, seen = r.seen;
     float kt = r.kt;
     bool ovf = r.ovf != 0, done = false;
-    for (int guard = 0; guard < (1 << 20); ++guard) {
+    for (int guard = 0; guard < (1 << 20) && (limit == 0 || seen < limit); ++guard) {
       if (cursor >= kCandK) {
         if (!ovf) {
           done = true;
@@ -169,6 +173,7 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
       const float hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
       float te, tx;
       if (!ray_box(o, d, lo, hi, 0.001f, best_t, te, tx)) continue;
+      ++seen;
       // a candidate that can hold neither a root nor a face hit ends here,
       // without a place in a round
       Pred pr;
@@ -199,6 +204,7 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
     r.pass = pass;
     r.kt = kt;
     r.ke = ke;
+    r.seen = seen;
     r.ovf = ovf ? 1 : 0;
     if (done) r.done = 1;
   }
@@ -503,14 +509,14 @@ static cudaError_t next_events(ho_context* c, cudaEvent_t* a, cudaEvent_t* b) {
 // launch has a fixed size and reads its counts on the device, so rounds can
 // be enqueued (and captured) without reading anything back.
 static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, bool learned,
-                         int64_t n_cap) {
+                         int64_t n_cap, int limit) {
   RoundBufs& rb = c->rounds;
   const int64_t n_elem = c->n_elem;
   RoundPair* gathered = static_cast<RoundPair*>(rb.pairs);
   const unsigned gi = static_cast<unsigned>((n_cap + 255) / 256);
   RT_TRY(cudaMemsetAsync(rb.ecount, 0, static_cast<size_t>(n_elem) * sizeof(uint32_t), s));
   RT_TRY(cudaMemsetAsync(rb.ctr, 0, kCtrWords * sizeof(unsigned), s));
-  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, gathered, rb.pelem, rb.prank, rb.ecount, rb.ctr);
+  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, gathered, rb.pelem, rb.prank, rb.ecount, rb.ctr, limit);
   {
     const unsigned tiles = static_cast<unsigned>((n_elem + kScanTile - 1) / kScanTile);
     if (tiles > 0) {
@@ -597,7 +603,7 @@ int enqueue_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool lea
   // with the tail, a fixed number of rounds (the tail finishes every ray)
   if (c->tail_after > 0) rounds = std::min(c->round_count, c->tail_after);
   for (int r = 0; r < rounds; ++r) {
-    const int rc = enqueue_round(c, P, R, s, learned, n_cap);
+    const int rc = enqueue_round(c, P, R, s, learned, n_cap, c->tail_after > 0 ? rounds : 0);
     if (rc) return rc;
   }
   if (c->tail_after > 0) {
@@ -627,7 +633,7 @@ int finish_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool lear
     c->rounds_needed = static_cast<int>(rounds);
     if (last == 0) break;
     extra = true;
-    const int rc = enqueue_round(c, P, R, s, learned, n_cap);
+    const int rc = enqueue_round(c, P, R, s, learned, n_cap, 0);
     if (rc) return rc;
   }
   if (extra) {

@@ -84,7 +84,7 @@ struct RayState {
   int done;
   int ovf;      // the current list was cut at kCandK candidates
   int its;      // Newton and face iterations spent on the ray
-  int pad;
+  int seen;     // candidates visited (box met before the closest hit)
 };
 
 struct RoundParams {

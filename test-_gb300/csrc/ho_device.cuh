@@ -46,6 +46,11 @@ __host__ __device__ constexpr unsigned long long eval_flops(int n, int comps) {
   return 3ull * 8 * n + 2ull * comps * (2ull * n * n * n + 3ull * n * n + 4ull * n);
 }
 constexpr unsigned long long kSolveFlops = 60;
+// One evaluation on a face (face_eval): two axes' basis values, and per
+// component 4n^2 + 6n.
+__host__ __device__ constexpr unsigned long long face_eval_flops(int n) {
+  return 2ull * 8 * n + 3ull * (4ull * n * n + 6ull * n);
+}
 
 // ---------------------------------------------------------------------------
 // 1-D Modified-A basis: phi_0 = (1-x)/2, phi_1 = (1+x)/2,
@@ -137,6 +142,7 @@ template <>
 struct CoefRef<false> {
   const float* __restrict__ p;
   __device__ __forceinline__ float4 ld4(int off) const { return __ldg(reinterpret_cast<const float4*>(p + off)); }
+  __device__ __forceinline__ float ld(int off) const { return __ldg(p + off); }
   __device__ __forceinline__ CoefRef at(int off) const { return CoefRef{p + off}; }
 };
 template <>
@@ -145,6 +151,11 @@ struct CoefRef<true> {
   __device__ __forceinline__ float4 ld4(int off) const {
     float4 v;
     asm("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a + 4u * off));
+    return v;
+  }
+  __device__ __forceinline__ float ld(int off) const {
+    float v;
+    asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a + 4u * off));
     return v;
   }
   __device__ __forceinline__ CoefRef at(int off) const { return CoefRef{a + 4u * static_cast<uint32_t>(off)}; }
@@ -779,6 +790,57 @@ __device__ __forceinline__ void setc(float3& v, int a, float s) {
   if (a == 0) v.x = s;
   else if (a == 1) v.y = s;
   else v.z = s;
+}
+
+// Point and the two tangents of face f (face_param's free axes ua < va) at
+// its free coordinates (u, v): out[c] = {x_c, dx_c/du, dx_c/dv, 0}.
+//
+// On a face the fixed coordinate is exactly -1 or 1, where one vertex mode is
+// exactly 1 and every other mode exactly 0, so of the contraction over three
+// axes (eval_comps) only the face's own N x N coefficients contribute, and the
+// Newton needs no derivative across the face. The sums over the free axes run
+// in eval_comps' order, and adding a product with 0 or multiplying by 1 is
+// exact, so the values are eval_comps' to the last bit at 1 / N of its
+// multiply-adds. The face solves are most of the round kernel's steps; their
+// evaluations' cost was 2 (2N^3 + 3N^2) operations a component.
+template <int N, bool SM>
+__device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, float4* __restrict__ out) {
+  constexpr int RS = row_stride(N);
+  int fixed, ua, va;
+  float val;
+  face_param(f, fixed, val, ua, va);
+  const int m = val < 0.f ? 0 : 1;
+  const int sf = fixed == 0 ? 1 : (fixed == 1 ? RS : N * RS);  // strides of the three axes' modes
+  const int su = ua == 0 ? 1 : RS, sv = va == 1 ? RS : N * RS;
+  float pu[N], du[N], pv[N], dv[N];
+  basis_val_der<N>(u, pu, du);
+  basis_val_der<N>(v, pv, dv);
+#pragma unroll 1
+  for (int comp = 0; comp < 3; ++comp) {
+    const CoefRef<SM> cc = c.at(comp * block_floats(N) + m * sf);
+    float x = 0.f, xu = 0.f, xv = 0.f;
+#pragma unroll 1
+    for (int b = 0; b < N; ++b) {
+      float pb = pv[0], db = dv[0];
+#pragma unroll
+      for (int k = 1; k < N; ++k)
+        if (b == k) {
+          pb = pv[k];
+          db = dv[k];
+        }
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int a = 0; a < N; ++a) {
+        const float w = cc.ld(b * sv + a * su);
+        s0 = fmaf(w, pu[a], s0);
+        s1 = fmaf(w, du[a], s1);
+      }
+      x = fmaf(s0, pb, x);
+      xu = fmaf(s1, pb, xu);
+      xv = fmaf(s0, db, xv);
+    }
+    out[comp] = make_float4(x, xu, xv, 0.f);
+  }
 }
 
 // One seed of the ray / curved-face Newton in (u,v,tau): at most 50

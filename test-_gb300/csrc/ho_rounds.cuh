@@ -696,9 +696,34 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
         if (__any_sync(kFull, want_field)) r[3] = tc_finish_comp<N>(taddr, 3, as, ds, at, dt);
       }
       if (act) {
-        if constexpr (!TC) eval_comps<N, true>(el.c, s.xi, want_geom ? 0 : 3, want_field ? 4 : 3, r);
-        w.flops += eval_flops(N, (want_geom ? 3 : 0) + (want_field ? 1 : 0));
-        if (want_geom) {
+        const bool on_face = s.kind == TK_FSEED || s.kind == TK_FLEARN;
+        if constexpr (!TC) {
+          if (on_face) {
+            const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
+            int fixed, ua, va;
+            float val;
+            face_param(f, fixed, val, ua, va);
+            face_eval<N, true>(el.c, f, getc(s.xi, ua), getc(s.xi, va), r);
+          } else {
+            eval_comps<N, true>(el.c, s.xi, want_geom ? 0 : 3, want_field ? 4 : 3, r);
+          }
+        }
+        w.flops += !TC && on_face ? face_eval_flops(N) : eval_flops(N, (want_geom ? 3 : 0) + (want_field ? 1 : 0));
+        if (!TC && on_face) {
+          X = make_float3(r[0].x, r[1].x, r[2].x);
+          // the columns of the two tangents; the third is not used on a face
+          const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
+          int fixed, ua, va;
+          float val;
+          face_param(f, fixed, val, ua, va);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            J[3 * c] = r[c].y;
+            J[3 * c + 1] = ua == 1 ? r[c].y : r[c].z;
+            J[3 * c + 2] = r[c].z;
+          }
+          ++w.geom;
+        } else if (want_geom) {
           X = make_float3(r[0].x, r[1].x, r[2].x);
           J[0] = r[0].y; J[1] = r[0].z; J[2] = r[0].w;
           J[3] = r[1].y; J[4] = r[1].z; J[5] = r[1].w;

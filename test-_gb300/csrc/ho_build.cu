@@ -224,7 +224,7 @@ int launch_setup(ho_context* c) {
 }
 
 // ---------------------------------------------------------------------------
-// Isosurface exclusion certificates (iso_excluded reads them).
+// Element certificates (iso_excluded and face_impossible read them).
 //
 // For an element with map x(xi), let K be the inverse Jacobian of its
 // trilinear part at 0, x0 = x(0) and G(xi) = K (x(xi) - x0), and let beta bound
@@ -238,6 +238,7 @@ int launch_setup(ho_context* c) {
 //    So from any start with |xi| <= S where rho + q (S + rho) <= R (the cold
 //    start 0 is one) the iterates approach xi*: where they stop, they are at
 //    xi*. No sample of a certified element converges anywhere else.
+// The cube reaches at least to 1.5, the clamp of the face Newton's iterates.
 // The field there is its trilinear part, exactly interpolated by the test,
 // plus the higher modes, at most H = sum |c_ijk| V_i V_j V_k over |xi| <= rho.
 // The bounds on the modes and their derivatives over [-r, r], r >= 1, follow
@@ -333,9 +334,9 @@ __global__ void __launch_bounds__(32 * kCullWarps) cull_kernel(const float* __re
     Y = fmaxf(Y, fabsf(mid) + half);
   }
   Y = 1.001f * Y + 0.01f;
-  float delta = -1.f, rho = 0.f, start = 0.f;
+  float delta = -1.f, rho = 0.f, start = 0.f, bound = 0.f;
   for (int attempt = 0; attempt < 3 && ok && delta < 0.f; ++attempt) {
-    const float R = fmaxf(1.f, Y * (attempt == 0 ? 1.2f : (attempt == 1 ? 1.5f : 2.f)));
+    const float R = fmaxf(1.5f, Y * (attempt == 0 ? 1.2f : (attempt == 1 ? 1.5f : 2.f)));
     fill(R);
     float E[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int q = lane; q < S; q += 32) {
@@ -385,6 +386,7 @@ __global__ void __launch_bounds__(32 * kCullWarps) cull_kernel(const float* __re
     rho = Y / (1.f - beta) + 0.01f;
     start = fminf(R, (R - rho) / q - rho);
     if (start >= 0.f) delta = beta * rho + 5e-4f;
+    bound = beta;
   }
   float H = 0.f;
   if (delta >= 0.f) {
@@ -408,7 +410,7 @@ __global__ void __launch_bounds__(32 * kCullWarps) cull_kernel(const float* __re
     o[12] = delta;
     o[13] = H;
     o[14] = start;
-    o[15] = 0.f;
+    o[15] = bound;
     for (int v = 0; v < 8; ++v) o[16 + v] = f[v];
   }
 }

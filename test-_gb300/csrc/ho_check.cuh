@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128) check_kernel(TraceParams P, RayState* __r
       if (failed) {
         fail_list[atomicAdd(n_fail, 1u)] = item;
       } else {
-        if (polished) r.best = h;
+        r.best = h;
         if (r.tie.kind != HO_HIT_MISS) *(tie_end - atomicAdd(n_tie, 1u)) = item;
       }
     }
@@ -171,6 +171,37 @@ __global__ void __launch_bounds__(kTraceBlock) fallback_kernel(TraceParams P, Ra
   if (w.map) atomicAdd(&P.stats->c[ST_MAP], static_cast<unsigned long long>(w.map));
 }
 
+// Without the check: the listed rays' hits are completed (fill_hit).
+template <int N>
+__global__ void __launch_bounds__(128) post_kernel(TraceParams P, RayState* __restrict__ st,
+                                                   const uint32_t* __restrict__ list,
+                                                   const unsigned* __restrict__ n_list) {
+  const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= *n_list) return;
+  const unsigned item = list[k];
+  HitState h = st[item].best;
+  if (!(h.flags & kFlagPost)) return;
+  float3 o, d;
+  float iso;
+  bool iso_on;
+  query_ray(P, P.work[item], o, d, iso, iso_on);
+  const CoefRef<false> c{P.rec + static_cast<int64_t>(h.elem) * record_floats(N)};
+  float xJ[12], ug[4] = {0.f, 0.f, 0.f, 0.f};
+  geom_eval_raw<N, false>(c, h.xi, xJ);
+  if (h.kind == HO_HIT_ISO || (__ldg(P.flags + h.elem) & 1u))
+    field_eval_raw<N, false>(c.at(3 * block_floats(N)), h.xi, ug);
+  const float J[9] = {xJ[1], xJ[2], xJ[3], xJ[5], xJ[6], xJ[7], xJ[9], xJ[10], xJ[11]};
+  fill_hit(h, J, ug[0], d);
+  st[item].best = h;
+}
+
+template <int N>
+cudaError_t launch_post_n(const TraceParams& P, RayState* st, const uint32_t* list, const unsigned* n_list,
+                          int64_t n_cap, cudaStream_t s) {
+  post_kernel<N><<<static_cast<unsigned>((n_cap + 127) / 128), 128, 0, s>>>(P, st, list, n_list);
+  return cudaGetLastError();
+}
+
 // fail_list holds n_cap entries (n_cap >= the listed rays); n_fail and
 // n_tie are zeroed by the caller.
 template <int N>
@@ -218,5 +249,22 @@ extern template cudaError_t launch_residuals_n<8>(const float*, const uint32_t*,
                                                   double*, cudaStream_t);
 extern template cudaError_t launch_residuals_n<9>(const float*, const uint32_t*, int64_t, const float*, const ho_hit*,
                                                   double*, cudaStream_t);
+
+extern template cudaError_t launch_post_n<2>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<4>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<5>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<6>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<7>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<8>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
+extern template cudaError_t launch_post_n<9>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
+                                             cudaStream_t);
 
 }  // namespace ho

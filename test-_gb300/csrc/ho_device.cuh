@@ -843,17 +843,76 @@ __device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, f
   }
 }
 
+// True when no seed of face f can be accepted on the ray's [tmin, tmax], by the
+// element's certificate (cull_kernel). Let z = xi' - xi for a point xi of the
+// cube with position X, a parameter t, and an accepted (xi', t') on the face:
+// G(xi') - G(xi) = e + w (t' - t) + a term of size eps, where e = K (o + t d -
+// X), w = K d and eps covers the acceptance tolerance 1e-4 and rounding, and z
+// differs from it by at most b = beta |z| <= beta / (1 - beta) (|e| + |w| |t' -
+// t| + eps). z's component across the face is known (across), which bounds t'
+// - t when the ray is not nearly parallel to the face; the other two must
+// bring xi' into [-1.001, 1.001]. With xi = 0 this is a slab test in the
+// element's own frame; with the last iterate of a failed seed, e is small and
+// so is what the curvature leaves open.
+static __device__ __noinline__ bool face_impossible(const float* __restrict__ cert, int f, float3 o, float3 d, float3 xi,
+                                             float3 X, float t, float across, float tmin, float tmax) {
+  const float4* c4 = reinterpret_cast<const float4*>(cert);
+  const float4 k0 = __ldg(c4), k1 = __ldg(c4 + 1), k2 = __ldg(c4 + 2), k3 = __ldg(c4 + 3);
+  if (!(k3.x >= 0.f)) return false;
+  const float K[9] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w, k2.x};
+  const float beta = k3.w, bp = beta / (1.f - beta);
+  const float kn = fmaxf(fabsf(K[0]) + fabsf(K[1]) + fabsf(K[2]),
+                         fmaxf(fabsf(K[3]) + fabsf(K[4]) + fabsf(K[5]), fabsf(K[6]) + fabsf(K[7]) + fabsf(K[8])));
+  const float big = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z))) +
+                    fabsf(t) * fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
+  const float eps = kn * (1.05e-4f + 2e-6f * big);
+  const float3 q = make_float3(o.x + t * d.x - X.x, o.y + t * d.y - X.y, o.z + t * d.z - X.z);
+  float e[3], w[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    e[a] = K[3 * a] * q.x + K[3 * a + 1] * q.y + K[3 * a + 2] * q.z;
+    w[a] = K[3 * a] * d.x + K[3 * a + 1] * d.y + K[3 * a + 2] * d.z;
+  }
+  int fixed, ua, va;
+  float val;
+  face_param(f, fixed, val, ua, va);
+  const float en = fmaxf(fabsf(e[0]), fmaxf(fabsf(e[1]), fabsf(e[2])));
+  const float wn = fmaxf(fabsf(w[0]), fmaxf(fabsf(w[1]), fabsf(w[2])));
+  const float ef = (fixed == 0 ? e[0] : (fixed == 1 ? e[1] : e[2])) - across;
+  const float wf = fixed == 0 ? w[0] : (fixed == 1 ? w[1] : w[2]);
+  const float steep = fabsf(wf) - bp * wn;
+  if (!(steep > 1e-3f * wn)) return false;
+  const float s0 = -ef / wf, h = (bp * (en + wn * fabsf(s0) + eps) + eps) / steep;
+  const float tol = 2e-6f * big;
+  const float lo = fmaxf(s0 - h, tmin - t - tol), hi = fminf(s0 + h, tmax - t + tol);
+  if (lo > hi) return true;
+  const float z = bp * (en + wn * fmaxf(fabsf(lo), fabsf(hi)) + eps) + eps;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int a = k == 0 ? ua : va;
+    const float ea = a == 0 ? e[0] : (a == 1 ? e[1] : e[2]), wa = a == 0 ? w[0] : (a == 1 ? w[1] : w[2]);
+    const float p = getc(xi, a) + ea, r0 = wa * lo, r1 = wa * hi;
+    if (p + fmaxf(r0, r1) + z < -1.001f || p + fminf(r0, r1) - z > 1.001f) return true;
+  }
+  return false;
+}
+
+// Iterations after which a first seed is asked whether the face can be hit at
+// all: a seed that converges takes about 7 (its steps are clamped to 0.25),
+// one that sticks at the clamps of u, v or tau runs all its 50.
+constexpr int kSeedPatience = 8;
+
 // One seed of the ray / curved-face Newton in (u,v,tau): at most 50
 // iterations, accept when max|X-Y| < 1e-4 with u,v in [-1.001,1.001] and tau
 // in [tmin,tmax]; step clamp 0.25, divergence break after 5 iterations
 // (high_order.h:213-300).
 template <int N, bool SM>
 __device__ bool face_newton(const Elem<N, SM>& e, float3 o, float3 d, int f, float3 p, float tau, float tmin, float tmax,
-                            float& th, float3& xh, Work& w, int max_it);
+                            float& th, float3& xh, Work& w, int max_it, const float* cert = nullptr, bool* none = nullptr);
 
 template <int N, bool SM>
 __device__ bool face_seed(const Elem<N, SM>& e, float3 o, float3 d, int f, int si, int sj, float tmin, float tmax,
-                          float& th, float3& xh, Work& w) {
+                          float& th, float3& xh, Work& w, const float* cert = nullptr, bool* none = nullptr) {
   int fixed, ua, va;
   float val;
   face_param(f, fixed, val, ua, va);
@@ -866,13 +925,13 @@ __device__ bool face_seed(const Elem<N, SM>& e, float3 o, float3 d, int f, int s
   const float3 df = make_float3(x0.x - o.x, x0.y - o.y, x0.z - o.z);
   float tau = dd > 0.f ? (df.x * d.x + df.y * d.y + df.z * d.z) / dd : 0.f;
   tau = fminf(fmaxf(tau, tmin), tmax);
-  return face_newton<N>(e, o, d, f, p, tau, tmin, tmax, th, xh, w, 50);
+  return face_newton<N>(e, o, d, f, p, tau, tmin, tmax, th, xh, w, 50, cert, none);
 }
 
 // The (u,v,tau) Newton of one seed from a given start point.
 template <int N, bool SM>
 __device__ bool face_newton(const Elem<N, SM>& e, float3 o, float3 d, int f, float3 p, float tau, float tmin, float tmax,
-                            float& th, float3& xh, Work& w, int max_it) {
+                            float& th, float3& xh, Work& w, int max_it, const float* cert, bool* none) {
   int fixed, ua, va;
   float val;
   face_param(f, fixed, val, ua, va);
@@ -884,6 +943,7 @@ __device__ bool face_newton(const Elem<N, SM>& e, float3 o, float3 d, int f, flo
     geom_eval<N>(e, p, X, J, w);
     const float rx = X.x - (o.x + tau * d.x), ry = X.y - (o.y + tau * d.y), rz = X.z - (o.z + tau * d.z);
     const float m = fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz)));
+    bool ended = false;
     if (m < 1e-4f) {
       const float pu = getc(p, ua), pv = getc(p, va);
       if (pu >= -1.001f && pu <= 1.001f && pv >= -1.001f && pv <= 1.001f && tau >= tmin && tau <= tmax) {
@@ -891,9 +951,16 @@ __device__ bool face_newton(const Elem<N, SM>& e, float3 o, float3 d, int f, flo
         xh = p;
         return true;
       }
+      ended = true;
+    } else if (it > 5 && m > prev * 1.5f) {
+      ended = true;
+    }
+    // a first seed that ends without a hit, or takes long: none may have one
+    if (cert && (ended || it == kSeedPatience) && face_impossible(cert, f, o, d, p, X, tau, 0.f, tmin, tmax)) {
+      *none = true;
       return false;
     }
-    if (it > 5 && m > prev * 1.5f) return false;
+    if (ended) return false;
     prev = m;
     const float A[9] = {J[ua], J[va], -d.x, J[3 + ua], J[3 + va], -d.y, J[6 + ua], J[6 + va], -d.z};
     float K[9];
@@ -978,6 +1045,32 @@ struct HitState {
   uint32_t flags;
 };
 
+// Internal flag of a HitState: the face hit's normal (from the Jacobian at xi)
+// and the field value at xi are still to be filled in (fill_hit).
+constexpr uint32_t kFlagPost = 0x80000000u;
+
+// Unit normal of a face hit from the Jacobian's columns (the face's two
+// tangents), against the ray.
+__device__ __forceinline__ float3 face_normal(const float (&J)[9], float3 xi, float3 d) {
+  const float3 dr = make_float3(J[0], J[3], J[6]), ds = make_float3(J[1], J[4], J[7]),
+               dt = make_float3(J[2], J[5], J[8]);
+  float3 n;
+  if (fabsf(xi.x) > 0.9f) n = cross3(ds, dt);
+  else if (fabsf(xi.y) > 0.9f) n = cross3(dr, dt);
+  else n = cross3(dr, ds);
+  n = normalize3(n);
+  if (n.x * d.x + n.y * d.y + n.z * d.z > 0.f) n = make_float3(-n.x, -n.y, -n.z);
+  return n;
+}
+
+// What a hit committed with kFlagPost lacks, from the Jacobian and the field
+// value at its xi.
+__device__ __forceinline__ void fill_hit(HitState& h, const float (&J)[9], float u, float3 d) {
+  if (h.kind == HO_HIT_FACE) h.n = face_normal(J, h.xi, d);
+  h.u = u;
+  h.flags &= ~kFlagPost;
+}
+
 // Two candidates' hits this close in t claim one surface point: a face shared
 // by two elements, an edge of two faces, a root in the overlap of two padded
 // boxes. The reference keeps whichever its visit order and FP32 rounding put
@@ -1056,11 +1149,33 @@ __device__ __forceinline__ bool face_may_hit(const float* __restrict__ fbox, int
   return ray_box(o, d, lo, hi, tmin, tmax, a0, a1);
 }
 
-// Warp version of hit_hex: the (face, seed) Newton solves of the faces that
-// survive the cull are independent, so they are spread over the lanes (at
-// most 6 x 9 = 54, two per lane). For each face the lowest seed index that
-// was accepted answers — the seed the sequential loop would stop at — and
-// faces are then compared in index order as the reference does.
+// The same, with the entry into the hull box.
+__device__ __forceinline__ bool face_entry(const float* __restrict__ fbox, int f, float3 o, float3 d, float tmin,
+                                           float tmax, float& te) {
+  const float* b = fbox + 6 * f;
+  const float lo[3] = {__ldg(b + 0), __ldg(b + 1), __ldg(b + 2)};
+  const float hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
+  float a1;
+  return ray_box(o, d, lo, hi, tmin, tmax, te, a1);
+}
+
+// The same from the element's centre: t at the closest approach to it.
+__device__ __forceinline__ bool face_excluded(const float* __restrict__ cert, int f, float3 o, float3 d, float tmin,
+                                              float tmax) {
+  const float3 x0 = make_float3(__ldg(cert + 9), __ldg(cert + 10), __ldg(cert + 11));
+  const float dd = d.x * d.x + d.y * d.y + d.z * d.z;
+  const float t = ((x0.x - o.x) * d.x + (x0.y - o.y) * d.y + (x0.z - o.z) * d.z) / dd;
+  int fixed, ua, va;
+  float val;
+  face_param(f, fixed, val, ua, va);
+  return face_impossible(cert, f, o, d, make_float3(0.f, 0.f, 0.f), x0, t, val, tmin, tmax);
+}
+
+// How far a face may be entered and still give a hit at or before hi: hi and
+// the rounding of the slab test far from the ray's origin (the hull boxes'
+// own inflation covers the solver's tolerance).
+__device__ __forceinline__ float seed_reach(float hi) { return fminf(hi + 1e-6f * fabsf(hi), FLT_MAX); }
+
 // Where the predicted xi-line enters [-1,1]^3: face, start point, t.
 __device__ __forceinline__ bool predicted_entry(const Pred& pr, float tmin, float tmax, int& face, float3& p,
                                                 float& tau) {
@@ -1093,12 +1208,14 @@ __device__ __forceinline__ bool predicted_entry(const Pred& pr, float tmin, floa
   return true;
 }
 
+// Warp version of hit_hex: the (face, seed) Newton solves of a step are
+// independent, so they are spread over the lanes. For each face the lowest
+// seed index that was accepted answers — the seed the sequential loop would
+// stop at — and faces are then compared in index order as the reference does.
 template <int N, bool L, bool SM>
-__device__ bool hit_hex_warp(const Elem<N, SM>& e, const float* __restrict__ fbox, float3 o, float3 d, float tmin,
+__device__ bool hit_hex_warp(const Elem<N, SM>& e, const float* __restrict__ fbox, const float* __restrict__ cert, float3 o, float3 d, float tmin,
                              float tmax, float& th, float3& xh, int& face, Work& w, Work& wu, const Pred& pr) {
   const int lane = threadIdx.x & 31;
-  unsigned packed = 0;
-  int na = 0;
   // learned: one Newton solve from the predicted element entry; faces whose
   // hull box misses [tmin, t_learned] cannot hold a nearer hit and are skipped
   int lf = -1;
@@ -1116,61 +1233,70 @@ __device__ bool hit_hex_warp(const Elem<N, SM>& e, const float* __restrict__ fbo
       ++wu.rejected;
     }
   }
-  const float cull_hi = lf >= 0 ? lt : tmax;
-  for (int f = 0; f < 6; ++f) {
-    if (f != lf && face_may_hit(fbox, f, o, d, tmin, cull_hi)) {
-      packed |= static_cast<unsigned>(f) << (3 * na);
-      ++na;
-    } else if (f != lf) {
-      ++wu.culled;
-    }
-  }
-  if (na == 0) {
-    if (lf < 0 || !(lt > tmin && lt < tmax)) return false;
-    th = lt;
-    xh = lx;
-    face = lf;
-    return true;
-  }
-  const int T = na * 9;
-  bool ok[2] = {false, false};
-  float tv[2] = {0.f, 0.f};
-  float3 xv[2] = {make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
+  // the seeds as next_seeds (ho_rounds.cuh) orders them, spread over the lanes;
+  // seed 0 of all faces at once, since a step costs the warp the same
+  const bool staged = __ldg(cert + 12) >= 0.f;
+  unsigned todo = lf >= 0 ? 63u & ~(1u << lf) : 63u, tried = 0u, found = 0u;
+  float tv[6];
+  float3 xv[6];
+  for (;;) {
+    float hi = lf >= 0 ? fminf(tmax, lt) : tmax;
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int k = lane + 32 * r;
-    if (k < T) {
-      const int slot = k / 9, sd = k - 9 * slot;
-      const int f = (packed >> (3 * slot)) & 7u;
-      ok[r] = face_seed<N>(e, o, d, f, sd % 3, sd / 3, tmin, tmax, tv[r], xv[r], w);
+    for (int f = 0; f < 6; ++f)
+      if (((found >> f) & 1u) && tv[f] > tmin) hi = fminf(hi, tv[f]);
+    todo &= ~found;
+    for (int f = 0; f < 6; ++f) {
+      if (!((todo >> f) & 1u)) continue;
+      if (!face_may_hit(fbox, f, o, d, tmin, seed_reach(hi)) ||
+          (staged && face_excluded(cert, f, o, d, tmin, seed_reach(hi)))) {
+        ++wu.culled;
+        todo &= ~(1u << f);
+      }
     }
+    if (todo == 0u) break;
+    // fresh: seed 0 (all seeds without a certificate); rest: seeds 1-8
+    const unsigned now = todo;
+    const unsigned rest = now & tried, fresh = now & ~tried;
+    const int per = staged ? 1 : 9, n_fresh = per * __popc(fresh), T = n_fresh + 8 * __popc(rest);
+    unsigned dead = 0u;
+    for (int base = 0; base < T; base += 32) {
+      const int k = base + lane;
+      bool ok = false, none = false;
+      float ts = 0.f;
+      float3 xs = make_float3(0.f, 0.f, 0.f);
+      int f = -1;
+      if (k < T) {
+        unsigned m = k < n_fresh ? fresh : rest;
+        const int slot = k < n_fresh ? k / per : (k - n_fresh) >> 3;
+        for (int q = 0; q < slot; ++q) m &= m - 1u;
+        f = __ffs(m) - 1;
+        const int sd = k < n_fresh ? k - slot * per : 1 + ((k - n_fresh) & 7);
+        ok = face_seed<N>(e, o, d, f, sd % 3, sd / 3, tmin, tmax, ts, xs, w, staged && sd == 0 ? cert : nullptr, &none);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {  // each face's lowest accepted seed
+        if (__any_sync(kFull, none && f == q)) dead |= 1u << q;
+        const unsigned b = __ballot_sync(kFull, ok && f == q);
+        if (b == 0u || ((found >> q) & 1u)) continue;
+        const int src = __ffs(b) - 1;
+        found |= 1u << q;
+        tv[q] = __shfl_sync(kFull, ts, src);
+        xv[q] = shfl3(xs, src);
+      }
+    }
+    todo &= ~(staged ? rest | dead : now);
+    tried |= now;
   }
   bool any = false;
   float best = tmax;
-  int a = 0;  // next surviving slot, in increasing face order
+#pragma unroll
   for (int f = 0; f < 6; ++f) {
-    float tf;
-    float3 xf;
-    if (f == lf) {
-      tf = lt;
-      xf = lx;
-    } else {
-      if (a >= na || static_cast<int>((packed >> (3 * a)) & 7u) != f) continue;
-      const int k0 = lane, k1 = lane + 32;
-      const unsigned b0 = __ballot_sync(kFull, ok[0] && k0 / 9 == a);
-      const unsigned b1 = __ballot_sync(kFull, ok[1] && k1 < T && k1 / 9 == a);
-      ++a;
-      if ((b0 | b1) == 0u) continue;
-      const bool second = b0 == 0u;
-      const int src = second ? __ffs(b1) - 1 : __ffs(b0) - 1;
-      const float tA = __shfl_sync(kFull, tv[0], src), tB = __shfl_sync(kFull, tv[1], src);
-      const float3 xA = shfl3(xv[0], src), xB = shfl3(xv[1], src);
-      tf = second ? tB : tA;
-      xf = second ? xB : xA;
-    }
+    if (f != lf && !((found >> f) & 1u)) continue;
+    const float tf = f == lf ? lt : tv[f];
     if (tf > tmin && tf < best) {
       best = tf;
-      xh = xf;
+      xh = f == lf ? lx : xv[f];
       face = f;
       any = true;
     }
@@ -1181,7 +1307,7 @@ __device__ bool hit_hex_warp(const Elem<N, SM>& e, const float* __restrict__ fbo
 
 // Warp version of visit_candidate: every lane holds the same `best`.
 template <int N, bool L, bool SM>
-__device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox, int eidx, float3 o, float3 d, float te,
+__device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox, const float* __restrict__ cert, int eidx, float3 o, float3 d, float te,
                            float tx, float iso, bool iso_on, HitState& best, Work& w, Work& wu, const Pred& pr,
                            HitState* tie = nullptr) {
   ++wu.cand;
@@ -1196,6 +1322,7 @@ __device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox,
       best.elem = eidx;
       best.face = -1;
       best.kind = HO_HIT_ISO;
+      best.flags &= ~kFlagPost;
       best.xi = xi;
       best.n = n;
       float4 r[4];  // the field at the root, as the round kernel's post evaluation
@@ -1206,7 +1333,7 @@ __device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox,
   }
   int face = -1;
   const long long c0 = clock64();
-  const bool fh = hit_hex_warp<N, L>(e, fbox, o, d, 0.001f, best.t, th, xi, face, w, wu, pr);
+  const bool fh = hit_hex_warp<N, L>(e, fbox, cert, o, d, 0.001f, best.t, th, xi, face, w, wu, pr);
   wu.cyc[3] += clock64() - c0;
   if (fh) {
     if (th > 0.001f && th < best.t) {
@@ -1227,6 +1354,7 @@ __device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox,
       best.elem = eidx;
       best.face = face;
       best.kind = HO_HIT_FACE;
+      best.flags &= ~kFlagPost;
       best.xi = xi;
       best.n = n;
       best.u = e.has_field ? r[3].x : 0.f;

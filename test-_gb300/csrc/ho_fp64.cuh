@@ -286,6 +286,7 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
   const CoefRef<false> c{rec_all + static_cast<int64_t>(h.elem) * record_floats(N)};
   float J[9];
   float3 g = make_float3(0.f, 0.f, 0.f);
+  float u32 = 0.f;
   auto jacobian_at = [&](float3 xi) {
     float xJ[12];
     geom_eval_raw<N, false>(c, xi, xJ);
@@ -296,9 +297,11 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
       float ug[4];
       field_eval_raw<N, false>(c.at(3 * block_floats(N)), xi, ug);
       g = make_float3(ug[1], ug[2], ug[3]);
+      u32 = ug[0];
     }
   };
   jacobian_at(h.xi);
+  if (h.flags & kFlagPost) fill_hit(h, J, u32, d);
   const float dn = fabsf(h.n.x * d.x + h.n.y * d.y + h.n.z * d.z);
   const bool steep = dn >= 0.2f * sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
   double t = h.t, x0 = h.xi.x, x1 = h.xi.y, x2 = h.xi.z, un = u;

@@ -107,9 +107,9 @@ constexpr int kStatusRoundGuard = 4;
 // Per-face hull boxes: 6 faces x (lo xyz, hi xyz).
 constexpr int kFaceBoxFloats = 36;
 
-// Per element, what the isosurface exclusion test reads (ho_build.cu,
-// cull_kernel; ho_device.cuh, iso_excluded): K (9, row-major), x0 (3), delta,
-// H, S, one unused, the field's 8 corner values. delta < 0: no certificate.
+// Per element, what the exclusion tests read (ho_build.cu, cull_kernel;
+// ho_device.cuh, iso_excluded and face_impossible): K (9, row-major), x0 (3),
+// delta, H, S, beta, the field's 8 corner values. delta < 0: no certificate.
 constexpr int kCullFloats = 24;
 
 // Largest supported modes per direction (P = 8).

@@ -401,9 +401,9 @@ int launch_residuals(ho_context* c, int64_t n, const float* rays, const ho_hit* 
   return int(e);
 }
 
-// FP64 check of the rays' hits, plain fallback of the failures.
+// FP64 check of the rays' hits, plain fallback of the failures; without the
+// check, the hits are only completed.
 static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, int64_t n_cap) {
-  if (!c->fp64_check) return 0;
   // the rays with a hit, listed into the (now idle) pair-element buffer, so
   // that the check's threads are all busy
   uint32_t* list = reinterpret_cast<uint32_t*>(c->rounds.pelem);
@@ -414,6 +414,22 @@ static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams&
   ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, R.state, true, list, n_list,
                                                                              P.stats);
   RT_TRY(cudaGetLastError());
+  if (!c->fp64_check) {
+    c->launches += 2;  // ray list, post
+    cudaError_t e;
+    switch (c->N) {
+      case 2: e = launch_post_n<2>(P, R.state, list, n_list, n_cap, s); break;
+      case 3: e = launch_post_n<3>(P, R.state, list, n_list, n_cap, s); break;
+      case 4: e = launch_post_n<4>(P, R.state, list, n_list, n_cap, s); break;
+      case 5: e = launch_post_n<5>(P, R.state, list, n_list, n_cap, s); break;
+      case 6: e = launch_post_n<6>(P, R.state, list, n_list, n_cap, s); break;
+      case 7: e = launch_post_n<7>(P, R.state, list, n_list, n_cap, s); break;
+      case 8: e = launch_post_n<8>(P, R.state, list, n_list, n_cap, s); break;
+      case 9: e = launch_post_n<9>(P, R.state, list, n_list, n_cap, s); break;
+      default: e = cudaErrorInvalidValue; break;
+    }
+    return int(e);
+  }
   c->launches += 4;  // ray list, check, tie rule, fallback
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -456,6 +472,7 @@ static RoundParams round_params(ho_context* c, const TraceParams& P) {
   R.rec = P.rec;
   R.fbox = P.fbox;
   R.flags = P.flags;
+  R.cull = P.cull;
   R.rays = P.rays;
   R.n_rays = P.n_rays;
   R.cam = P.cam;

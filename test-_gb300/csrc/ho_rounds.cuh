@@ -91,6 +91,7 @@ struct RoundParams {
   const float* __restrict__ rec;
   const float* __restrict__ fbox;
   const uint32_t* __restrict__ flags;
+  const float* __restrict__ cull;  // element certificates
   const float* __restrict__ rays;
   int64_t n_rays;
   CamArgs cam;
@@ -119,7 +120,7 @@ struct RoundParams {
 };
 
 // Task word: kind (3 bits) | pair (5 bits) | argument (8 bits).
-enum TaskKind { TK_SAMPLE = 0, TK_REFINE = 1, TK_FSEED = 2, TK_FLEARN = 3, TK_FPOST = 4, TK_IPOST = 5 };
+enum TaskKind { TK_SAMPLE = 0, TK_REFINE = 1, TK_FSEED = 2, TK_FLEARN = 3 };
 __device__ __forceinline__ uint32_t task_word(int kind, int pp, int arg) {
   return (static_cast<uint32_t>(kind) << 13) | (static_cast<uint32_t>(pp) << 8) | static_cast<uint32_t>(arg);
 }
@@ -131,12 +132,12 @@ struct PairSm {
   float te, tx, iso, best_t;
   float pxi[3], pv[3], pk, pte;  // learned prediction (xi at te, d xi/dt per element size)
   int item, elem;
-  int fl;        // bit 0 has field, 1 iso on, 2 prediction available, 3 a warm start was rejected
+  int fl;        // bit 0 has field, 1 iso search, 2 prediction available, 3 a warm start was rejected,
+                 // 4 the element has a certificate
   int pend;      // tasks of the current phase still running
   uint32_t okm;  // samples that converged
   // result under construction
   float ht, hx[3], hg[3];
-  int hface;
   int its;  // Newton and face iterations of this pair
   union {
     struct {  // isosurface samples
@@ -156,6 +157,7 @@ struct PairSm {
       int rit, rstage;
       // face search
       int lf;
+      unsigned ftodo, ftried;  // faces left to search; faces whose seed 0 was queued
       float lt, lx[3];
       int fseed[6];
       float ft[6], fx[6][3];
@@ -197,7 +199,7 @@ struct LaneSolve {
   float3 xi;  // inverse map: xi; face Newton: the face point
   float t;    // inverse map: the sample's t; face Newton: tau
   int it, cap;
-  bool warm, post, inited;
+  bool warm, inited;
   unsigned tried;  // sample: converged samples of the pair it has restarted from
   float prev;  // face Newton: residual of the last iteration
 };
@@ -225,7 +227,6 @@ __device__ __forceinline__ void start_sample_solve(LaneSolve& s, float t, bool w
   s.xi = warm ? xi0 : make_float3(0.f, 0.f, 0.f);
   s.it = 0;
   s.cap = warm ? warm_cap : 50;
-  s.post = false;
   s.tried = 0u;
 }
 
@@ -253,40 +254,30 @@ __device__ __forceinline__ void pair_done(WS& W, int pp, const RoundParams* P) {
 // step, so they are kept out of line: the per-step loop stays small in the
 // instruction cache. Counters come back in the return value.
 
-// Queue the 9 seeds of every face (other than the learned face) whose hull
-// box meets [0.001, cull_hi]; returns the number of faces culled.
-template <int N, class WS>
-__device__ __noinline__ int start_seeds(WS* Wp, int pp, const float* __restrict__ fbox, float cull_hi) {
-  WS& W = *Wp;
-  PairSm& p = W.pr[pp];
-  const float3 o = ld3(p.o), d = ld3(p.d);
-  int n = 0, culled = 0;
-  uint32_t faces = 0;
-  for (int f = 0; f < 6; ++f) {
-    if (f == p.lf) continue;
-    if (face_may_hit(fbox, f, o, d, 0.001f, cull_hi)) {
-      faces |= 1u << f;
-      n += 9;
-    } else {
-      ++culled;
-    }
-  }
-  p.pend = n;
-  if (n == 0) return culled;
-  const unsigned base = atomicAdd(&W.tail, static_cast<unsigned>(n));
-  unsigned k = base;
-  for (int f = 0; f < 6; ++f)
-    if (faces >> f & 1u)
-      for (int sd = 0; sd < 9; ++sd)
-        W.ring[(k++) % RoundCfg<N>::Ring] = static_cast<uint16_t>(task_word(TK_FSEED, pp, 9 * f + sd));
-  return culled;
+// The ray's state after a pair produced a hit. What a full evaluation at the
+// hit gives (a face hit's normal, the field value) is left to the final pass
+// over the rays' answers, which evaluates there anyway (kFlagPost): as tasks of
+// this kernel those evaluations, one per hit, ran on one or two lanes of
+// nearly every step, each several times the cost of a face step.
+__device__ __forceinline__ void commit_hit(const RoundParams& P, const PairSm& p, int kind, int face, float t, float3 xi,
+                                           float3 n) {
+  HitState& b = P.state[p.item].best;
+  note_tie(b, p.best_t, t, &P.state[p.item].tie);  // p.best_t: b.t, read when the pair was admitted
+  b.t = t;
+  b.elem = p.elem;
+  b.face = face;
+  b.kind = kind;
+  b.xi = xi;
+  b.n = n;
+  b.u = 0.f;
+  b.flags |= kFlagPost;
+  if (p.fl & 8) b.flags |= HO_FLAG_FALLBACK;
 }
 
 // Nearest face over the learned face and every face's first accepted seed,
-// in face order. A hit is left in the pair's result fields (the caller
-// starts its post evaluation); no hit finishes the pair.
+// in face order; finishes the pair.
 template <int N, class WS>
-__device__ __noinline__ bool finalize_faces(WS* Wp, int pp, const RoundParams* P) {
+__device__ __noinline__ void finalize_faces(WS* Wp, int pp, const RoundParams* P) {
   WS& W = *Wp;
   PairSm& p = W.pr[pp];
   float best = p.best_t;
@@ -310,37 +301,85 @@ __device__ __noinline__ bool finalize_faces(WS* Wp, int pp, const RoundParams* P
       xh = xf;
     }
   }
-  if (face < 0) {
-    pair_done<N>(W, pp, P);
-    return false;
-  }
-  p.ht = best;
-  st3(p.hx, xh);
-  p.hface = face;
-  return true;
+  if (face >= 0) commit_hit(*P, p, HO_HIT_FACE, face, best, xh, make_float3(0.f, 0.f, 0.f));
+  pair_done<N>(W, pp, P);
 }
 
-__device__ __forceinline__ void start_post(LaneSolve& s, int kind, int pp, float3 xi) {
-  s.task = 0;
-  s.kind = kind;
-  s.pp = pp;
-  s.xi = xi;
-  s.post = true;
-  s.it = 0;
-  s.warm = false;
+// Queue the next seeds of a pair's face search. The answer is the nearest
+// face over every face's first accepted seed, in face order.
+// Without a certificate all 9 seeds of every face whose hull box the ray
+// meets run at once. With one they go from the likeliest outwards: a face
+// that the ray enters (its hull box) behind an accepted hit cannot give a
+// nearer one, a face's later seeds count for nothing once its first seed is
+// accepted, and the certificate excludes most of the faces that the ray
+// passes by (face_excluded, face_impossible). So: seed 0 of the face entered
+// first (unless the learned face already answered); then, of the faces
+// entered before the nearest hit so far, seed 0 of those not tried yet and
+// seeds 1-8 of those whose seed 0 failed without excluding the face. A primary ray mostly ends after its first seed. Coarse elements
+// without certificates keep the seeds together: there the stages' chain of
+// dependent solves took longer than the seeds it saved.
+// Returns the faces culled.
+template <int N, class WS>
+__device__ __noinline__ int next_seeds(WS* Wp, int pp, const float* __restrict__ fbox, const RoundParams* P) {
+  WS& W = *Wp;
+  PairSm& p = W.pr[pp];
+  const float3 o = ld3(p.o), d = ld3(p.d);
+  const bool staged = (p.fl & 16) != 0;
+  float hi = p.best_t;
+  if (p.lf >= 0) hi = fminf(hi, p.lt);
+  unsigned todo = p.ftodo;
+  for (int f = 0; f < 6; ++f)
+    if (p.fseed[f] < 9) {
+      if (p.ft[f] > 0.001f) hi = fminf(hi, p.ft[f]);  // an answer at the ray's start is none
+      todo &= ~(1u << f);
+    }
+  const float reach = seed_reach(hi);
+  const float* cert = P->cull + static_cast<int64_t>(p.elem) * kCullFloats;
+  int culled = 0, nearest = -1;
+  float near_t = FLT_MAX;
+  for (int f = 0; f < 6; ++f) {
+    if (!((todo >> f) & 1u)) continue;
+    float te;
+    if (!face_entry(fbox, f, o, d, 0.001f, reach, te) || (staged && face_excluded(cert, f, o, d, 0.001f, reach))) {
+      ++culled;
+      todo &= ~(1u << f);
+    } else if (te < near_t) {
+      near_t = te;
+      nearest = f;
+    }
+  }
+  if (todo == 0u) {
+    finalize_faces<N>(Wp, pp, P);
+    return culled;
+  }
+  const unsigned now = staged && p.lf < 0 && p.ftried == 0u ? 1u << nearest : todo;
+  const unsigned rest = now & p.ftried;
+  const int per = staged ? 1 : 9, n = per * __popc(now & ~rest) + 8 * __popc(rest);
+  p.pend = n;
+  unsigned k = atomicAdd(&W.tail, static_cast<unsigned>(n));
+  for (int f = 0; f < 6; ++f) {
+    if (!((now >> f) & 1u)) continue;
+    const int s0 = (rest >> f) & 1u ? 1 : 0, s1 = s0 ? 9 : per;
+    for (int sd = s0; sd < s1; ++sd)
+      W.ring[(k++) % RoundCfg<N>::Ring] = static_cast<uint16_t>(task_word(TK_FSEED, pp, 9 * f + sd));
+  }
+  p.ftodo = todo & ~(staged ? rest : now);  // nothing of these faces is left to try
+  p.ftried |= now;
+  return culled;
 }
 
 // Face search of a pair after its isosurface search found nothing (or iso is
 // off): the learned start face first when there is one, else the seeds of
 // the faces whose hull box meets [0.001, closest]. Returns culled faces |
-// 256 when a learned start was rejected | 65536 when the pair needs its face
-// post evaluation now.
+// 256 when a learned start was rejected.
 template <int N, bool L, class WS>
 __device__ __noinline__ int start_faces(WS* Wp, int pp, const float* __restrict__ fbox, const RoundParams* P) {
   WS& W = *Wp;
   PairSm& p = W.pr[pp];
   p.lf = -1;
   for (int f = 0; f < 6; ++f) p.fseed[f] = 9;
+  p.ftodo = 63u;
+  p.ftried = 0u;
   int code = 0;
   if (L && (p.fl & 4)) {
     int f0;
@@ -353,18 +392,15 @@ __device__ __noinline__ int start_faces(WS* Wp, int pp, const float* __restrict_
     }
     code |= 256;
   }
-  code |= start_seeds<N>(Wp, pp, fbox, p.best_t);
-  if (p.pend == 0 && finalize_faces<N>(Wp, pp, P)) code |= 65536;
-  return code;
+  return code | next_seeds<N>(Wp, pp, fbox, P);
 }
 
 template <int N, bool L, class WS>
 __device__ __forceinline__ void face_phase(WS& W, int pp, const float* __restrict__ fbox, const RoundParams* P,
-                                           Work& w, LaneSolve& s) {
+                                           Work& w) {
   const int code = start_faces<N, L>(&W, pp, fbox, P);
   w.culled += code & 255;
   if (code & 256) ++w.rejected;
-  if (code & 65536) start_post(s, TK_FPOST, pp, ld3(W.pr[pp].hx));
 }
 
 // Begin a popped task.
@@ -374,7 +410,7 @@ __device__ __forceinline__ void begin_task(WS& W, uint32_t tw, LaneSolve& s, int
   s.kind = static_cast<int>(tw >> 13);
   s.pp = static_cast<int>((tw >> 8) & 31u);
   s.arg = static_cast<int>(tw & 255u);
-  if (s.pp >= RoundCfg<N>::B || s.kind > TK_IPOST) {  // never queued: drop it
+  if (s.pp >= RoundCfg<N>::B || s.kind > TK_FLEARN) {  // never queued: drop it
     s.task = -1;
     return;
   }
@@ -400,7 +436,6 @@ __device__ __forceinline__ void begin_task(WS& W, uint32_t tw, LaneSolve& s, int
     s.it = 0;
     s.cap = 50;
     s.warm = false;
-    s.post = false;
   } else {  // TK_FLEARN: the predicted entry face and point
     int f0;
     float3 p0;
@@ -412,24 +447,8 @@ __device__ __forceinline__ void begin_task(WS& W, uint32_t tw, LaneSolve& s, int
     s.it = 0;
     s.cap = warm_cap;
     s.warm = true;
-    s.post = false;
     s.inited = true;
   }
-}
-
-// The ray's state after a pair produced a hit.
-__device__ __forceinline__ void commit_hit(const RoundParams& P, const PairSm& p, int kind, int face, float t, float3 xi,
-                                           float3 n, float u) {
-  HitState& b = P.state[p.item].best;
-  note_tie(b, p.best_t, t, &P.state[p.item].tie);  // p.best_t: b.t, read when the pair was admitted
-  b.t = t;
-  b.elem = p.elem;
-  b.face = face;
-  b.kind = kind;
-  b.xi = xi;
-  b.n = n;
-  b.u = u;
-  if (p.fl & 8) b.flags |= HO_FLAG_FALLBACK;
 }
 
 // Fill a free slot with a pair of the batch and queue its first tasks.
@@ -464,6 +483,7 @@ __device__ __noinline__ int admit_pair(WS* Wp, const RoundParams* P, int slot, R
     p.pte = rp.te;
     fl |= 4;
   }
+  if (__ldg(P->cull + static_cast<int64_t>(elem) * kCullFloats + 12) >= 0.f) fl |= 16;
   p.fl = fl;
   p.okm = 0u;
   p.its = 0;
@@ -568,7 +588,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
     s.t = 0.f;
     s.it = 0;
     s.cap = 0;
-    s.warm = s.post = s.inited = false;
+    s.warm = s.inited = false;
     s.tried = 0u;
     s.prev = FLT_MAX;
     // every task ends within a bounded number of steps; the guard is far above
@@ -606,7 +626,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
               const int code = admit_pair<N, L>(&W, &P, slot, P.pairs[bt.first + adm + lane], bt.elem, has_field, fbox);
               ++w.cand;
               w.culled += code & 255;
-              if (code & 256) ++w.rejected;  // a face post at admission cannot happen: no face was searched
+              if (code & 256) ++w.rejected;
             } else {
               atomicOr(&P.stats->status, kStatusRoundGuard);
             }
@@ -662,9 +682,8 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
       float u = 0.f;
       float3 gr = make_float3(0.f, 0.f, 0.f);
       // inverse-map iteration of an isosurface solve: the field comes with it
-      const bool ahead = (s.kind == TK_SAMPLE || s.kind == TK_REFINE) && !s.post;
-      const bool want_geom = act && s.kind != TK_IPOST;
-      const bool want_field = act && ((s.post && (s.kind != TK_FPOST || has_field)) || ahead);
+      const bool on_face = s.kind == TK_FSEED || s.kind == TK_FLEARN;
+      const bool want_field = act && !on_face;
       float4 r[4];
       if constexpr (TC) {
         // every thread's point as a row of the step's MMAs; idle lanes give a
@@ -689,14 +708,13 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
         }
         tc_fence_after();
         const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-        if (__any_sync(kFull, want_geom)) {
+        if (__any_sync(kFull, act)) {
 #pragma unroll 1
           for (int comp = 0; comp < 3; ++comp) r[comp] = tc_finish_comp<N>(taddr, comp, as, ds, at, dt);
         }
         if (__any_sync(kFull, want_field)) r[3] = tc_finish_comp<N>(taddr, 3, as, ds, at, dt);
       }
       if (act) {
-        const bool on_face = s.kind == TK_FSEED || s.kind == TK_FLEARN;
         if constexpr (!TC) {
           if (on_face) {
             const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
@@ -705,10 +723,10 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
             face_param(f, fixed, val, ua, va);
             face_eval<N, true>(el.c, f, getc(s.xi, ua), getc(s.xi, va), r);
           } else {
-            eval_comps<N, true>(el.c, s.xi, want_geom ? 0 : 3, want_field ? 4 : 3, r);
+            eval_comps<N, true>(el.c, s.xi, 0, 4, r);
           }
         }
-        w.flops += !TC && on_face ? face_eval_flops(N) : eval_flops(N, (want_geom ? 3 : 0) + (want_field ? 1 : 0));
+        w.flops += !TC && on_face ? face_eval_flops(N) : eval_flops(N, on_face ? 3 : 4);
         if (!TC && on_face) {
           X = make_float3(r[0].x, r[1].x, r[2].x);
           // the columns of the two tangents; the third is not used on a face
@@ -722,16 +740,13 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
             J[3 * c + 1] = ua == 1 ? r[c].y : r[c].z;
             J[3 * c + 2] = r[c].z;
           }
-          ++w.geom;
-        } else if (want_geom) {
+        } else {
           X = make_float3(r[0].x, r[1].x, r[2].x);
           J[0] = r[0].y; J[1] = r[0].z; J[2] = r[0].w;
           J[3] = r[1].y; J[4] = r[1].z; J[5] = r[1].w;
           J[6] = r[2].y; J[7] = r[2].z; J[8] = r[2].w;
-          ++w.geom;
-        } else {
-          for (int q = 0; q < 9; ++q) J[q] = 0.f;
         }
+        ++w.geom;
         if (want_field) {
           u = r[3].x;
           gr = make_float3(r[3].y, r[3].z, r[3].w);
@@ -745,42 +760,31 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
       float3 sg = make_float3(0.f, 0.f, 0.f);
       if (act) {
         PairSm& p = W.pr[s.pp];
-        if (s.kind == TK_SAMPLE || s.kind == TK_REFINE) {
+        if (!on_face) {
           float K[9];
           invert3(J, K);
-          if (!s.post) {
-            ++w.newton;
-            w.flops += kSolveFlops;
-            const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
-                        rz = X.z - (p.o[2] + s.t * p.d[2]);
-            const float d0 = K[0] * rx + K[1] * ry + K[2] * rz;
-            const float d1 = K[3] * rx + K[4] * ry + K[5] * rz;
-            const float d2 = K[6] * rx + K[7] * ry + K[8] * rz;
-            s.xi.x -= d0;
-            s.xi.y -= d1;
-            s.xi.z -= d2;
-            ++s.it;
-            if (fabsf(d0) < 1e-5f && fabsf(d1) < 1e-5f && fabsf(d2) < 1e-5f) {
-              if (ahead) {  // value and gradient at the converged point, first order
-                sg = make_float3(K[0] * gr.x + K[3] * gr.y + K[6] * gr.z, K[1] * gr.x + K[4] * gr.y + K[7] * gr.z,
-                                 K[2] * gr.x + K[5] * gr.y + K[8] * gr.z);
-                sf = (u - (gr.x * d0 + gr.y * d1 + gr.z * d2)) - p.iso;
-                sdf = sg.x * p.d[0] + sg.y * p.d[1] + sg.z * p.d[2];
-                end = 1;
-              } else {
-                s.post = true;
-              }
-            } else if (!(fabsf(d0) + fabsf(d1) + fabsf(d2) < FLT_MAX)) {
-              end = 2;
-            } else if (s.it >= s.cap) {
-              end = 2;
-            }
-          } else {
+          ++w.newton;
+          w.flops += kSolveFlops;
+          const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
+                      rz = X.z - (p.o[2] + s.t * p.d[2]);
+          const float d0 = K[0] * rx + K[1] * ry + K[2] * rz;
+          const float d1 = K[3] * rx + K[4] * ry + K[5] * rz;
+          const float d2 = K[6] * rx + K[7] * ry + K[8] * rz;
+          s.xi.x -= d0;
+          s.xi.y -= d1;
+          s.xi.z -= d2;
+          ++s.it;
+          if (fabsf(d0) < 1e-5f && fabsf(d1) < 1e-5f && fabsf(d2) < 1e-5f) {
+            // value and gradient at the converged point, first order
             sg = make_float3(K[0] * gr.x + K[3] * gr.y + K[6] * gr.z, K[1] * gr.x + K[4] * gr.y + K[7] * gr.z,
                              K[2] * gr.x + K[5] * gr.y + K[8] * gr.z);
-            sf = u - p.iso;
+            sf = (u - (gr.x * d0 + gr.y * d1 + gr.z * d2)) - p.iso;
             sdf = sg.x * p.d[0] + sg.y * p.d[1] + sg.z * p.d[2];
             end = 1;
+          } else if (!(fabsf(d0) + fabsf(d1) + fabsf(d2) < FLT_MAX)) {
+            end = 2;
+          } else if (s.it >= s.cap) {
+            end = 2;
           }
           if (s.warm && end != 0) {
             if (end == 1) {
@@ -818,11 +822,10 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
                 s.cap = 50;
               }
               s.it = 0;
-              s.post = false;
-              end = 0;
+                        end = 0;
             }
           }
-        } else if (s.kind == TK_FSEED || s.kind == TK_FLEARN) {
+        } else {
           const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
           int fixed, ua, va;
           float val;
@@ -837,6 +840,10 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
           }
           ++w.face;
           w.flops += kSolveFlops;
+          const bool first = s.kind == TK_FSEED && (p.fl & 16) != 0 && s.arg == 9 * f;
+          const float3 xi0 = s.xi;
+          const float t0 = s.t;
+          const bool late = s.it == kSeedPatience;
           const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
                       rz = X.z - (p.o[2] + s.t * p.d[2]);
           const float m = fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz)));
@@ -865,12 +872,17 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
             setc(s.xi, fixed, val);
             if (++s.it >= s.cap) end = 2;
           }
+          // a first seed that ends without a hit, or takes long: none may have one
+          if (first && (end == 2 || (end == 0 && late)) &&
+              face_impossible(P.cull + static_cast<int64_t>(p.elem) * kCullFloats, f, ld3(p.o), ld3(p.d), xi0, X, t0, 0.f,
+                              tmin, tmax)) {
+            atomicAnd(&p.ftodo, ~(1u << f));
+            end = 2;
+          }
           if (end != 0 && s.kind == TK_FLEARN) {
             if (end == 1) ++w.accepted;
             else ++w.rejected;
           }
-        } else {
-          end = 1;  // post evaluations finish in one step
         }
         if (end != 0) atomicAdd(&p.its, s.it);
       }
@@ -940,13 +952,13 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
               s.pp = pp;
               start_sample_solve(s, p.mt, warm_pair, lerp3(ld3(p.lsx), ld3(p.rxi), 0.5f), P.warm_cap);
             } else {
-              face_phase<N, L>(W, pp, fbox, &P, w, s);
+              face_phase<N, L>(W, pp, fbox, &P, w);
             }
           }
         } else if (s.kind == TK_REFINE) {
           if (p.rstage == 0) {  // midpoint solve ended
             if (end == 2) {
-              face_phase<N, L>(W, pp, fbox, &P, w, s);  // the isosurface search failed
+              face_phase<N, L>(W, pp, fbox, &P, w);  // the isosurface search failed
             } else {
               p.msf = sf;
               p.msdf = sdf;
@@ -1003,45 +1015,23 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
                 start_sample_solve(s, p.mt, warm_pair, lerp3(ld3(p.lsx), ld3(p.rxi), 0.5f), P.warm_cap);
               }
             }
-            if (found) {  // the field value at the root's xi, then the hit
-              s.task = 0;
-              s.kind = TK_IPOST;
-              s.xi = ld3(p.hx);
-              s.post = true;
-              s.it = 0;
-              s.warm = false;
+            if (found) {
+              if (p.ht > 0.001f && p.ht < p.best_t) {
+                float3 n = normalize3(ld3(p.hg));
+                if (n.x * p.d[0] + n.y * p.d[1] + n.z * p.d[2] > 0.f) n = make_float3(-n.x, -n.y, -n.z);
+                commit_hit(P, p, HO_HIT_ISO, -1, p.ht, ld3(p.hx), n);
+              }
+              pair_done<N>(W, pp, &P);
             }
           }
-        } else if (s.kind == TK_FSEED) {
-          if (atomicSub(&p.pend, 1) == 1 && finalize_faces<N>(&W, pp, &P)) start_post(s, TK_FPOST, pp, ld3(p.hx));
-        } else if (s.kind == TK_FLEARN) {
-          if (end == 1) {
+        } else {
+          if (s.kind == TK_FLEARN && end == 1) {
             p.lf = s.arg;
+            p.ftodo &= ~(1u << s.arg);
             p.lt = s.t;
             st3(p.lx, s.xi);
           }
-          w.culled += start_seeds<N>(&W, pp, fbox, end == 1 ? s.t : p.best_t);
-          if (p.pend == 0 && finalize_faces<N>(&W, pp, &P)) start_post(s, TK_FPOST, pp, ld3(p.hx));
-        } else if (s.kind == TK_FPOST) {
-          // normal from the Jacobian columns (the face's two tangents)
-          const float3 dr = make_float3(J[0], J[3], J[6]), ds = make_float3(J[1], J[4], J[7]),
-                       dt = make_float3(J[2], J[5], J[8]);
-          const float3 xi = s.xi;
-          float3 n;
-          if (fabsf(xi.x) > 0.9f) n = cross3(ds, dt);
-          else if (fabsf(xi.y) > 0.9f) n = cross3(dr, dt);
-          else n = cross3(dr, ds);
-          n = normalize3(n);
-          if (n.x * p.d[0] + n.y * p.d[1] + n.z * p.d[2] > 0.f) n = make_float3(-n.x, -n.y, -n.z);
-          commit_hit(P, p, HO_HIT_FACE, p.hface, p.ht, xi, n, has_field ? u : 0.f);
-          pair_done<N>(W, pp, &P);
-        } else if (s.kind == TK_IPOST) {
-          if (p.ht > 0.001f && p.ht < p.best_t) {
-            float3 n = normalize3(ld3(p.hg));
-            if (n.x * p.d[0] + n.y * p.d[1] + n.z * p.d[2] > 0.f) n = make_float3(-n.x, -n.y, -n.z);
-            commit_hit(P, p, HO_HIT_ISO, -1, p.ht, s.xi, n, u);
-          }
-          pair_done<N>(W, pp, &P);
+          if (atomicSub(&p.pend, 1) == 1) w.culled += next_seeds<N>(&W, pp, fbox, &P);
         }
       }
       __syncwarp();
@@ -1152,7 +1142,8 @@ __global__ void __launch_bounds__(kTraceBlock) tail_kernel(TraceParams P, RaySta
           Elem<N, true> el;
           el.c = CoefRef<true>{slot_addr};
           el.has_field = (__ldg(P.flags + ce) & 1u) != 0;
-          visit_warp<N, L>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats, ce, o, d, te, tx, iso, scan,
+          visit_warp<N, L>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats,
+                           P.cull + static_cast<int64_t>(ce) * kCullFloats, ce, o, d, te, tx, iso, scan,
                            best, w, wu, pr, &r.tie);
         }
         kt = ct;

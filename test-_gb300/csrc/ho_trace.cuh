@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(kTraceBlock) isect_kernel(TraceParams P) {
           Elem<N, true> el;
           el.c = CoefRef<true>{slot_addr};
           el.has_field = (__ldg(P.flags + ce) & 1u) != 0;
-          visit_warp<N, LEARNED>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats, ce, o, d, te, tx, iso,
+          visit_warp<N, LEARNED>(el, P.fbox + static_cast<int64_t>(ce) * kFaceBoxFloats,
+                                 P.cull + static_cast<int64_t>(ce) * kCullFloats, ce, o, d, te, tx, iso,
                                  scan, best, w, wu, pr);
         }
         kt = ct;

@@ -238,11 +238,11 @@ void ho_destroy(ho_context* c) {
     cudaFree(c->d_qctr);
     cudaFree(c->rounds.state);
     cudaFree(c->rounds.pairs);
-    cudaFree(c->rounds.pelem);
+    cudaFree(c->rounds.pkey);
     cudaFree(c->rounds.prank);
     cudaFree(c->rounds.batches);
-    cudaFree(c->rounds.ecount);
-    cudaFree(c->rounds.eoff);
+    cudaFree(c->rounds.kcount);
+    cudaFree(c->rounds.koff);
     cudaFree(c->rounds.tile_sums);
     cudaFree(c->rounds.ctr);
     cudaFree(c->rounds.fail);

@@ -123,17 +123,17 @@ struct RoundBufs {
   size_t state_cap = 0;
   void* pairs = nullptr;     // gathered + element-sorted pairs
   size_t pairs_cap = 0;
-  int32_t* pelem = nullptr;
-  size_t pelem_cap = 0;
+  int32_t* pkey = nullptr;   // 2 * element + (isosurface search)
+  size_t pkey_cap = 0;
   uint32_t* prank = nullptr;
   size_t prank_cap = 0;
   void* batches = nullptr;
   size_t batches_cap = 0;
-  uint32_t* ecount = nullptr;  // per element
-  size_t ecount_cap = 0;
-  uint32_t* eoff = nullptr;
-  size_t eoff_cap = 0;
-  uint32_t* tile_sums = nullptr;  // per 4096 elements, for the offsets' scan
+  uint32_t* kcount = nullptr;  // per key
+  size_t kcount_cap = 0;
+  uint32_t* koff = nullptr;
+  size_t koff_cap = 0;
+  uint32_t* tile_sums = nullptr;  // per 4096 keys, for the offsets' scan
   size_t tile_sums_cap = 0;
   unsigned* ctr = nullptr;   // pairs, batches, next batch, failed FP64 checks
   size_t ctr_cap = 0;

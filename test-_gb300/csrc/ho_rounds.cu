@@ -117,8 +117,8 @@ __global__ void round_init_kernel(RayState* __restrict__ st, const uint8_t* __re
 // candidate does not depend on how many ended here (their face Newtons
 // differ in the last bits on a few rays).
 __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, RoundPair* __restrict__ pairs,
-                                    int32_t* __restrict__ pelem, uint32_t* __restrict__ prank,
-                                    uint32_t* __restrict__ ecount, unsigned* __restrict__ ctr, int limit) {
+                                    int32_t* __restrict__ pkey, uint32_t* __restrict__ prank,
+                                    uint32_t* __restrict__ kcount, unsigned* __restrict__ ctr, int limit) {
   const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   bool live = item < *P.qcount && !st[item].done;
@@ -216,9 +216,11 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
     base = __shfl_sync(kFull, base, leader);
     if (elem >= 0) {
       const unsigned k = base + __popc(m & ((1u << lane) - 1u));
+      // element-sorted with the pairs that search for an isosurface apart
+      const int key = 2 * elem + (p.j & kPairNoIso ? 0 : 1);
       pairs[k] = p;
-      pelem[k] = elem;
-      prank[k] = atomicAdd(&ecount[elem], 1u);
+      pkey[k] = key;
+      prank[k] = atomicAdd(&kcount[key], 1u);
     }
   }
   const unsigned nodes = __reduce_add_sync(kFull, w.nodes), restarts = __reduce_add_sync(kFull, w.restarts),
@@ -253,8 +255,8 @@ __global__ void ray_list_kernel(const unsigned* __restrict__ qcount, const RaySt
 }
 
 // Also tallies the round (non-empty rounds and pairs) into the work counters.
-__global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const int32_t* __restrict__ pelem,
-                                     const uint32_t* __restrict__ prank, const uint32_t* __restrict__ eoff,
+__global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const int32_t* __restrict__ pkey,
+                                     const uint32_t* __restrict__ prank, const uint32_t* __restrict__ koff,
                                      const unsigned* __restrict__ ctr, RoundPair* __restrict__ sorted,
                                      DevStats* stats) {
   const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -264,29 +266,37 @@ __global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const 
     atomicAdd(&stats->c[ST_PAIRS], static_cast<unsigned long long>(n_pairs));
   }
   if (k >= n_pairs) return;
-  sorted[eoff[pelem[k]] + prank[k]] = pairs[k];
+  sorted[koff[pkey[k]] + prank[k]] = pairs[k];
 }
 
 // Ctr layout: [0] pairs of the round, [3] failed FP64 checks, [4..5] the
 // tail's list count and cursor, [6..7] the check's list count and tie count,
-// and per order n (2..9) the batch count, region start, write cursor and take
-// cursor.
-constexpr int kCtrOrderNb = 16, kCtrOrderOff = 26, kCtrOrderCur = 36, kCtrOrderNext = 46, kCtrWords = 64;
+// and per order n (2..9) the batch count, region start, write cursor of the
+// face batches, take cursor, and count and write cursor of the isosurface
+// batches, which come first in the region.
+constexpr int kCtrOrderNb = 16, kCtrOrderOff = 26, kCtrOrderCur = 36, kCtrOrderNext = 46, kCtrIsoNb = 56,
+              kCtrIsoCur = 66, kCtrWords = 80;
 
 __device__ __forceinline__ int batch_size(int chunk, int order, bool tc) {
   return chunk > 0 ? chunk : round_batch_default(order, tc);
 }
 
-// Batches per order: each element's pairs in batches of its order's size.
-__global__ void round_batch_count_kernel(const uint32_t* __restrict__ ecount, const uint8_t* __restrict__ order,
+// Batches per order: a key's pairs (key 2 e: element e's pairs without an
+// isosurface search, 2 e + 1: with one) in batches of its element's order's
+// size. A warp step costs what its most expensive lane does, an isosurface
+// sample several times a face step, so the two kinds share no batch; the
+// isosurface batches, the longer ones, come first.
+__global__ void round_batch_count_kernel(const uint32_t* __restrict__ kcount, const uint8_t* __restrict__ order,
                                          int64_t n_elem, int chunk, bool tc, unsigned* __restrict__ ctr) {
-  const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= n_elem) return;
-  const int c = static_cast<int>(ecount[e]);
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= 2 * n_elem) return;
+  const int c = static_cast<int>(kcount[k]);
   if (c == 0) return;
-  const int n = order[e];
+  const int n = order[k >> 1];
   const int B = batch_size(chunk, n, tc);
-  atomicAdd(&ctr[kCtrOrderNb + n], static_cast<unsigned>((c + B - 1) / B));
+  const unsigned nb = static_cast<unsigned>((c + B - 1) / B);
+  atomicAdd(&ctr[kCtrOrderNb + n], nb);
+  if (k & 1) atomicAdd(&ctr[kCtrIsoNb + n], nb);
 }
 
 // Region start of each order's batches (orders in increasing n).
@@ -294,28 +304,30 @@ __global__ void round_order_offsets_kernel(unsigned* __restrict__ ctr) {
   unsigned run = 0;
   for (int n = 0; n < 10; ++n) {
     ctr[kCtrOrderOff + n] = run;
-    ctr[kCtrOrderCur + n] = 0;
+    ctr[kCtrOrderCur + n] = ctr[kCtrIsoNb + n];
+    ctr[kCtrIsoCur + n] = 0;
     ctr[kCtrOrderNext + n] = 0;
     run += ctr[kCtrOrderNb + n];
   }
 }
 
-// Each element's pairs in batches, written into its order's region.
-__global__ void round_batch_kernel(const uint32_t* __restrict__ ecount, const uint32_t* __restrict__ eoff,
+// Each key's pairs in batches, written into its order's region.
+__global__ void round_batch_kernel(const uint32_t* __restrict__ kcount, const uint32_t* __restrict__ koff,
                                    const uint8_t* __restrict__ order, int64_t n_elem, int chunk, bool tc,
                                    RoundBatch* __restrict__ batches, unsigned* __restrict__ ctr) {
-  const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= n_elem) return;
-  const int c = static_cast<int>(ecount[e]);
+  const int64_t key = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (key >= 2 * n_elem) return;
+  const int c = static_cast<int>(kcount[key]);
   if (c == 0) return;
-  const int n = order[e];
+  const int n = order[key >> 1];
   const int B = batch_size(chunk, n, tc);
   const int nb = (c + B - 1) / B;
-  const unsigned base = ctr[kCtrOrderOff + n] + atomicAdd(&ctr[kCtrOrderCur + n], static_cast<unsigned>(nb));
+  const unsigned base = ctr[kCtrOrderOff + n] + atomicAdd(&ctr[(key & 1 ? kCtrIsoCur : kCtrOrderCur) + n],
+                                                          static_cast<unsigned>(nb));
   for (int k = 0; k < nb; ++k) {
     RoundBatch bt;
-    bt.elem = static_cast<int32_t>(e);
-    bt.first = static_cast<int32_t>(eoff[e]) + k * B;
+    bt.elem = static_cast<int32_t>(key >> 1);
+    bt.first = static_cast<int32_t>(koff[key]) + k * B;
     bt.count = min(B, c - k * B);
     bt.pad = 0;
     batches[base + k] = bt;
@@ -372,12 +384,12 @@ int prepare_rounds(ho_context* c, int64_t n_cap) {
   RoundBufs& rb = c->rounds;
   RT_TRY(grow(rb.state, rb.state_cap, n, sizeof(RayState)));
   RT_TRY(grow(rb.pairs, rb.pairs_cap, 2 * n, sizeof(RoundPair)));
-  RT_TRY(grow(rb.pelem, rb.pelem_cap, n, sizeof(int32_t)));
+  RT_TRY(grow(rb.pkey, rb.pkey_cap, n, sizeof(int32_t)));
   RT_TRY(grow(rb.prank, rb.prank_cap, n, sizeof(uint32_t)));
   RT_TRY(grow(rb.batches, rb.batches_cap, n, sizeof(RoundBatch)));
-  RT_TRY(grow(rb.ecount, rb.ecount_cap, static_cast<size_t>(n_elem), sizeof(uint32_t)));
-  RT_TRY(grow(rb.eoff, rb.eoff_cap, static_cast<size_t>(n_elem), sizeof(uint32_t)));
-  RT_TRY(grow(rb.tile_sums, rb.tile_sums_cap, static_cast<size_t>((n_elem + kScanTile - 1) / kScanTile),
+  RT_TRY(grow(rb.kcount, rb.kcount_cap, static_cast<size_t>(2 * n_elem), sizeof(uint32_t)));
+  RT_TRY(grow(rb.koff, rb.koff_cap, static_cast<size_t>(2 * n_elem), sizeof(uint32_t)));
+  RT_TRY(grow(rb.tile_sums, rb.tile_sums_cap, static_cast<size_t>((2 * n_elem + kScanTile - 1) / kScanTile),
               sizeof(uint32_t)));
   RT_TRY(grow(rb.ctr, rb.ctr_cap, kCtrWords, sizeof(unsigned)));
   RT_TRY(grow(rb.fail, rb.fail_cap, n, sizeof(uint32_t)));
@@ -404,9 +416,9 @@ int launch_residuals(ho_context* c, int64_t n, const float* rays, const ho_hit* 
 // FP64 check of the rays' hits, plain fallback of the failures; without the
 // check, the hits are only completed.
 static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, int64_t n_cap) {
-  // the rays with a hit, listed into the (now idle) pair-element buffer, so
+  // the rays with a hit, listed into the (now idle) pair-key buffer, so
   // that the check's threads are all busy
-  uint32_t* list = reinterpret_cast<uint32_t*>(c->rounds.pelem);
+  uint32_t* list = reinterpret_cast<uint32_t*>(c->rounds.pkey);
   unsigned* n_list = c->rounds.ctr + 6;
   unsigned* n_tie = c->rounds.ctr + 7;
   RT_TRY(cudaMemsetAsync(c->rounds.ctr + 3, 0, sizeof(unsigned), s));
@@ -531,22 +543,23 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   const int64_t n_elem = c->n_elem;
   RoundPair* gathered = static_cast<RoundPair*>(rb.pairs);
   const unsigned gi = static_cast<unsigned>((n_cap + 255) / 256);
-  RT_TRY(cudaMemsetAsync(rb.ecount, 0, static_cast<size_t>(n_elem) * sizeof(uint32_t), s));
+  const int64_t n_keys = 2 * n_elem;
+  RT_TRY(cudaMemsetAsync(rb.kcount, 0, static_cast<size_t>(n_keys) * sizeof(uint32_t), s));
   RT_TRY(cudaMemsetAsync(rb.ctr, 0, kCtrWords * sizeof(unsigned), s));
-  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, gathered, rb.pelem, rb.prank, rb.ecount, rb.ctr, limit);
+  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, gathered, rb.pkey, rb.prank, rb.kcount, rb.ctr, limit);
   {
-    const unsigned tiles = static_cast<unsigned>((n_elem + kScanTile - 1) / kScanTile);
+    const unsigned tiles = static_cast<unsigned>((n_keys + kScanTile - 1) / kScanTile);
     if (tiles > 0) {
-      tile_sum_kernel<<<tiles, 1024, 0, s>>>(rb.ecount, n_elem, rb.tile_sums);
-      tile_scan_kernel<<<tiles, 1024, 0, s>>>(rb.ecount, n_elem, rb.tile_sums, rb.eoff);
+      tile_sum_kernel<<<tiles, 1024, 0, s>>>(rb.kcount, n_keys, rb.tile_sums);
+      tile_scan_kernel<<<tiles, 1024, 0, s>>>(rb.kcount, n_keys, rb.tile_sums, rb.koff);
     }
   }
-  round_scatter_kernel<<<gi, 256, 0, s>>>(gathered, rb.pelem, rb.prank, rb.eoff, rb.ctr,
+  round_scatter_kernel<<<gi, 256, 0, s>>>(gathered, rb.pkey, rb.prank, rb.koff, rb.ctr,
                                           const_cast<RoundPair*>(R.pairs), P.stats);
-  const unsigned ge = static_cast<unsigned>((n_elem + 255) / 256);
-  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.ecount, c->d_cord, n_elem, c->round_chunk, c->use_tc, rb.ctr);
+  const unsigned ge = static_cast<unsigned>((n_keys + 255) / 256);
+  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, n_elem, c->round_chunk, c->use_tc, rb.ctr);
   round_order_offsets_kernel<<<1, 1, 0, s>>>(rb.ctr);
-  round_batch_kernel<<<ge, 256, 0, s>>>(rb.ecount, rb.eoff, c->d_cord, n_elem, c->round_chunk, c->use_tc,
+  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, n_elem, c->round_chunk, c->use_tc,
                                         const_cast<RoundBatch*>(R.batches), rb.ctr);
   RT_TRY(cudaGetLastError());
   c->launches += 7 + __builtin_popcount(c->orders);

@@ -277,8 +277,13 @@ __global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const 
 constexpr int kCtrOrderNb = 16, kCtrOrderOff = 26, kCtrOrderCur = 36, kCtrOrderNext = 46, kCtrIsoNb = 56,
               kCtrIsoCur = 66, kCtrWords = 80;
 
-__device__ __forceinline__ int batch_size(int chunk, int order, bool tc) {
-  return chunk > 0 ? chunk : round_batch_default(order, tc);
+// Pairs per batch of a key (HO_OPT_ROUND_CHUNK, else the slots).
+__device__ __forceinline__ int batch_size(int chunk, int order, bool tc, bool faces) {
+  return chunk > 0 ? chunk : (faces ? face_slots(order) : round_batch_default(order, tc));
+}
+// Does a key's batch take the face layout?
+__device__ __forceinline__ bool face_batch(int64_t key, bool tc, const float* __restrict__ cull) {
+  return !tc && !(key & 1) && __ldg(cull + (key >> 1) * kCullFloats + 12) >= 0.f;
 }
 
 // Batches per order: a key's pairs (key 2 e: element e's pairs without an
@@ -287,13 +292,14 @@ __device__ __forceinline__ int batch_size(int chunk, int order, bool tc) {
 // sample several times a face step, so the two kinds share no batch; the
 // isosurface batches, the longer ones, come first.
 __global__ void round_batch_count_kernel(const uint32_t* __restrict__ kcount, const uint8_t* __restrict__ order,
-                                         int64_t n_elem, int chunk, bool tc, unsigned* __restrict__ ctr) {
+                                         const float* __restrict__ cull, int64_t n_elem, int chunk, bool tc,
+                                         unsigned* __restrict__ ctr) {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= 2 * n_elem) return;
   const int c = static_cast<int>(kcount[k]);
   if (c == 0) return;
   const int n = order[k >> 1];
-  const int B = batch_size(chunk, n, tc);
+  const int B = batch_size(chunk, n, tc, face_batch(k, tc, cull));
   const unsigned nb = static_cast<unsigned>((c + B - 1) / B);
   atomicAdd(&ctr[kCtrOrderNb + n], nb);
   if (k & 1) atomicAdd(&ctr[kCtrIsoNb + n], nb);
@@ -313,14 +319,15 @@ __global__ void round_order_offsets_kernel(unsigned* __restrict__ ctr) {
 
 // Each key's pairs in batches, written into its order's region.
 __global__ void round_batch_kernel(const uint32_t* __restrict__ kcount, const uint32_t* __restrict__ koff,
-                                   const uint8_t* __restrict__ order, int64_t n_elem, int chunk, bool tc,
-                                   RoundBatch* __restrict__ batches, unsigned* __restrict__ ctr) {
+                                   const uint8_t* __restrict__ order, const float* __restrict__ cull, int64_t n_elem,
+                                   int chunk, bool tc, RoundBatch* __restrict__ batches, unsigned* __restrict__ ctr) {
   const int64_t key = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (key >= 2 * n_elem) return;
   const int c = static_cast<int>(kcount[key]);
   if (c == 0) return;
   const int n = order[key >> 1];
-  const int B = batch_size(chunk, n, tc);
+  const bool faces = face_batch(key, tc, cull);
+  const int B = batch_size(chunk, n, tc, faces);
   const int nb = (c + B - 1) / B;
   const unsigned base = ctr[kCtrOrderOff + n] + atomicAdd(&ctr[(key & 1 ? kCtrIsoCur : kCtrOrderCur) + n],
                                                           static_cast<unsigned>(nb));
@@ -329,7 +336,7 @@ __global__ void round_batch_kernel(const uint32_t* __restrict__ kcount, const ui
     bt.elem = static_cast<int32_t>(key >> 1);
     bt.first = static_cast<int32_t>(koff[key]) + k * B;
     bt.count = min(B, c - k * B);
-    bt.pad = 0;
+    bt.faces = faces ? 1 : 0;
     batches[base + k] = bt;
   }
 }

@@ -34,6 +34,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "ho_device.cuh"
 #include "ho_host.h"
 #include "ho_learn.h"
@@ -70,7 +72,7 @@ struct RoundBatch {
   int32_t elem;
   int32_t first;  // into the element-sorted pairs
   int32_t count;
-  int32_t pad;
+  int32_t faces;  // 1: no pair searches for an isosurface and the element has a certificate
 };
 
 // Per queue item state kept across rounds.
@@ -149,32 +151,44 @@ struct PairSm {
       __half sg[kSamples][3];
     };
     struct {
-      // refinement
-      float rlt, rrt, mt, ct;
-      float lsf, lsx[3], lsg[3];
-      float rxi[3];
-      float msf, msdf, msx[3], msg[3];
-      int rit, rstage;
       // face search
       int lf;
       unsigned ftodo, ftried;  // faces left to search; faces whose seed 0 was queued
       float lt, lx[3];
       int fseed[6];
       float ft[6], fx[6][3];
+      // refinement (not in a face batch's slots, which end here)
+      float rlt, rrt, mt, ct;
+      float lsf, lsx[3], lsg[3];
+      float rxi[3];
+      float msf, msdf, msx[3], msg[3];
+      int rit, rstage;
     };
   };
 };
+// Slots of a batch without isosurface searches on a certified element end
+// before the sample store and the refinement's state, so more of them fit: 32
+// instead of 20 up to 7 modes, a pair for every lane (such a pair mostly has
+// one solve at a time).
+constexpr int kFacePairBytes = (static_cast<int>(offsetof(PairSm, rlt)) + 7) / 8 * 8;
+__host__ __device__ constexpr int face_slots(int n) {
+  return round_slots(n) * static_cast<int>(sizeof(PairSm)) / kFacePairBytes < 32
+             ? round_slots(n) * static_cast<int>(sizeof(PairSm)) / kFacePairBytes
+             : 32;
+}
 
 // Rec = false: the tensor-core form keeps the element's coefficients once per
 // CTA as its MMA operand instead.
 template <int N, bool Rec = true>
 struct WarpSm {
   float rec[Rec ? record_floats(N) : 4];
-  PairSm pr[RoundCfg<N>::B];
+  alignas(16) unsigned char store[RoundCfg<N>::B * sizeof(PairSm)];
   uint16_t ring[RoundCfg<N>::Ring];
   unsigned head, tail;
   unsigned freem;     // free pair slots
   unsigned admitted;  // pairs of the batch admitted so far
+  int stride, slots;  // the batch's slots in the store
+  __device__ __forceinline__ PairSm& pair(int pp) { return *reinterpret_cast<PairSm*>(store + pp * stride); }
 };
 
 template <int N>
@@ -245,7 +259,7 @@ __device__ __forceinline__ Pred pair_pred(const PairSm& p) {
 // A pair is finished: its iterations go to its ray and its slot is free.
 template <int N, class WS>
 __device__ __forceinline__ void pair_done(WS& W, int pp, const RoundParams* P) {
-  const PairSm& p = W.pr[pp];
+  const PairSm& p = W.pair(pp);
   atomicAdd(&P->state[p.item].its, p.its);
   atomicOr(&W.freem, 1u << pp);
 }
@@ -279,7 +293,7 @@ __device__ __forceinline__ void commit_hit(const RoundParams& P, const PairSm& p
 template <int N, class WS>
 __device__ __noinline__ void finalize_faces(WS* Wp, int pp, const RoundParams* P) {
   WS& W = *Wp;
-  PairSm& p = W.pr[pp];
+  PairSm& p = W.pair(pp);
   float best = p.best_t;
   int face = -1;
   float3 xh = make_float3(0.f, 0.f, 0.f);
@@ -322,7 +336,7 @@ __device__ __noinline__ void finalize_faces(WS* Wp, int pp, const RoundParams* P
 template <int N, class WS>
 __device__ __noinline__ int next_seeds(WS* Wp, int pp, const float* __restrict__ fbox, const RoundParams* P) {
   WS& W = *Wp;
-  PairSm& p = W.pr[pp];
+  PairSm& p = W.pair(pp);
   const float3 o = ld3(p.o), d = ld3(p.d);
   const bool staged = (p.fl & 16) != 0;
   float hi = p.best_t;
@@ -352,8 +366,11 @@ __device__ __noinline__ int next_seeds(WS* Wp, int pp, const float* __restrict__
     finalize_faces<N>(Wp, pp, P);
     return culled;
   }
-  const unsigned now = staged && p.lf < 0 && p.ftried == 0u ? 1u << nearest : todo;
-  const unsigned rest = now & p.ftried;
+  unsigned now = staged && p.lf < 0 && p.ftried == 0u ? 1u << nearest : todo;
+  // (one face's later seeds at a time: the ring has room for them)
+  unsigned rest = now & p.ftried;
+  now &= ~(rest & (rest - 1u));
+  rest = now & p.ftried;
   const int per = staged ? 1 : 9, n = per * __popc(now & ~rest) + 8 * __popc(rest);
   p.pend = n;
   unsigned k = atomicAdd(&W.tail, static_cast<unsigned>(n));
@@ -375,7 +392,7 @@ __device__ __noinline__ int next_seeds(WS* Wp, int pp, const float* __restrict__
 template <int N, bool L, class WS>
 __device__ __noinline__ int start_faces(WS* Wp, int pp, const float* __restrict__ fbox, const RoundParams* P) {
   WS& W = *Wp;
-  PairSm& p = W.pr[pp];
+  PairSm& p = W.pair(pp);
   p.lf = -1;
   for (int f = 0; f < 6; ++f) p.fseed[f] = 9;
   p.ftodo = 63u;
@@ -410,13 +427,13 @@ __device__ __forceinline__ void begin_task(WS& W, uint32_t tw, LaneSolve& s, int
   s.kind = static_cast<int>(tw >> 13);
   s.pp = static_cast<int>((tw >> 8) & 31u);
   s.arg = static_cast<int>(tw & 255u);
-  if (s.pp >= RoundCfg<N>::B || s.kind > TK_FLEARN) {  // never queued: drop it
+  if (s.pp >= W.slots || s.kind > TK_FLEARN) {  // never queued: drop it
     s.task = -1;
     return;
   }
   s.inited = false;
   s.prev = FLT_MAX;
-  const PairSm& p = W.pr[s.pp];
+  const PairSm& p = W.pair(s.pp);
   if (s.kind == TK_SAMPLE) {
     const float t = p.te + (p.tx - p.te) * (float(s.arg) / 16.0f);
     const bool warm = L && (p.fl & 4);
@@ -458,7 +475,7 @@ __device__ __noinline__ int admit_pair(WS* Wp, const RoundParams* P, int slot, R
                                        bool has_field, const float* __restrict__ fbox) {
   constexpr int R = RoundCfg<N>::Ring;
   WS& W = *Wp;
-  PairSm& p = W.pr[slot];
+  PairSm& p = W.pair(slot);
   const int64_t q = P->work[rp.item];
   float3 o, d;
   float iso;
@@ -514,7 +531,7 @@ constexpr size_t round_tc_off() {
 template <int N, bool L, bool TC>
 __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
   constexpr int B = RoundCfg<N>::B, R = RoundCfg<N>::Ring;
-  constexpr unsigned kAllSlots = B >= 32 ? 0xffffffffu : ((1u << B) - 1u);
+  static_assert(face_slots(N) * 13 <= R && B * 54 <= R, "the ring holds every task that a batch's pairs can queue");
   constexpr size_t kWarpBytes = (sizeof(WarpSm<N, !TC>) + 15) / 16 * 16;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   extern __shared__ __align__(128) unsigned char round_smem[];
@@ -570,7 +587,9 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
     if (lane == 0) {
       W.head = 0;
       W.tail = 0;
-      W.freem = kAllSlots;
+      W.slots = bt.faces ? face_slots(N) : B;
+      W.stride = bt.faces ? kFacePairBytes : static_cast<int>(sizeof(PairSm));
+      W.freem = W.slots >= 32 ? 0xffffffffu : (1u << W.slots) - 1u;
       W.admitted = 0;
     }
     if constexpr (TC) {
@@ -621,7 +640,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
             unsigned m = fm;  // the lane-th free slot: drop the lowest `lane` set bits
             for (int k = 0; k < lane; ++k) m &= m - 1u;
             const int slot = __ffs(m) - 1;
-            if (slot >= 0 && slot < B) {
+            if (slot >= 0 && slot < W.slots) {
               atomicAnd(&W.freem, ~(1u << slot));
               const int code = admit_pair<N, L>(&W, &P, slot, P.pairs[bt.first + adm + lane], bt.elem, has_field, fbox);
               ++w.cand;
@@ -759,7 +778,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
       float sf = 0.f, sdf = 0.f;
       float3 sg = make_float3(0.f, 0.f, 0.f);
       if (act) {
-        PairSm& p = W.pr[s.pp];
+        PairSm& p = W.pair(s.pp);
         if (!on_face) {
           float K[9];
           invert3(J, K);
@@ -891,9 +910,9 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
       __syncwarp();
       // face seeds: the lowest accepted seed index of each face wins
       const bool seed_ok = act && end == 1 && s.kind == TK_FSEED;
-      if (seed_ok) atomicMin(&W.pr[s.pp].fseed[s.arg / 9], s.arg % 9);
+      if (seed_ok) atomicMin(&W.pair(s.pp).fseed[s.arg / 9], s.arg % 9);
       if (act && end != 0 && s.kind == TK_SAMPLE) {  // store the sample
-        PairSm& p = W.pr[s.pp];
+        PairSm& p = W.pair(s.pp);
         const int i = s.arg;
         if (end == 1) {
           atomicOr(&p.okm, 1u << i);
@@ -906,7 +925,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
       }
       __syncwarp();
       if (seed_ok) {
-        PairSm& p = W.pr[s.pp];
+        PairSm& p = W.pair(s.pp);
         const int f = s.arg / 9;
         if (p.fseed[f] == s.arg % 9) {
           p.ft[f] = s.t;
@@ -916,7 +935,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
       __syncwarp();
       // -- finished solves: phase transitions
       if (act && end != 0) {
-        PairSm& p = W.pr[s.pp];
+        PairSm& p = W.pair(s.pp);
         const int pp = s.pp;
         const bool warm_pair = L && (p.fl & 4);
         s.task = -1;

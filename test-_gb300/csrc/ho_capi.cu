@@ -247,6 +247,14 @@ void ho_destroy(ho_context* c) {
     cudaFree(c->rounds.ctr);
     cudaFree(c->rounds.fail);
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
+    for (int n = 0; n <= ho::kMaxModes; ++n) {
+      if (c->order_streams[n]) {
+        cudaStreamSynchronize(c->order_streams[n]);
+        cudaStreamDestroy(c->order_streams[n]);
+      }
+      if (c->order_done[n]) cudaEventDestroy(c->order_done[n]);
+    }
+    if (c->order_fork) cudaEventDestroy(c->order_fork);
     for (cudaEvent_t ev : c->round_events) cudaEventDestroy(ev);
     cudaFree(c->d_pred);
     cudaFree(c->d_cand);

@@ -216,6 +216,10 @@ struct ho_context {
   size_t work_cap = 0;
   unsigned* d_qctr = nullptr;     // [0] queue length, [1] next item
   ho::RoundBufs rounds;
+  // one stream per element order of a mixed-order scene (the orders' round
+  // kernels run side by side), forked from and joined to the call's stream
+  cudaStream_t order_streams[ho::kMaxModes + 1] = {};
+  cudaEvent_t order_fork = nullptr, order_done[ho::kMaxModes + 1] = {};
   // batched / learned engine options (ho_set_option)
   int round_chunk = 0;       // pairs per element batch (0: the kernel's pair slots)
   int warm_cap = 4;          // round kernel: iterations of a warm-started solve before its cold restart

@@ -400,6 +400,13 @@ int prepare_rounds(ho_context* c, int64_t n_cap) {
               sizeof(uint32_t)));
   RT_TRY(grow(rb.ctr, rb.ctr_cap, kCtrWords, sizeof(unsigned)));
   RT_TRY(grow(rb.fail, rb.fail_cap, n, sizeof(uint32_t)));
+  if (__builtin_popcount(c->orders) > 1) {  // streams and events of the orders' launches
+    if (!c->order_fork) RT_TRY(cudaEventCreateWithFlags(&c->order_fork, cudaEventDisableTiming));
+    for (int m = kMinModes; m <= kMaxModes; ++m) {
+      if (!c->order_streams[m]) RT_TRY(cudaStreamCreateWithFlags(&c->order_streams[m], cudaStreamNonBlocking));
+      if (!c->order_done[m]) RT_TRY(cudaEventCreateWithFlags(&c->order_done[m], cudaEventDisableTiming));
+    }
+  }
   return 0;
 }
 
@@ -564,36 +571,48 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   round_scatter_kernel<<<gi, 256, 0, s>>>(gathered, rb.pkey, rb.prank, rb.koff, rb.ctr,
                                           const_cast<RoundPair*>(R.pairs), P.stats);
   const unsigned ge = static_cast<unsigned>((n_keys + 255) / 256);
-  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, n_elem, c->round_chunk, c->use_tc, rb.ctr);
+  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, rb.ctr);
   round_order_offsets_kernel<<<1, 1, 0, s>>>(rb.ctr);
-  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, n_elem, c->round_chunk, c->use_tc,
+  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc,
                                         const_cast<RoundBatch*>(R.batches), rb.ctr);
   RT_TRY(cudaGetLastError());
   c->launches += 7 + __builtin_popcount(c->orders);
-  // one launch per element order present in the scene
+  // One launch per element order present in the scene. Each ends with a few
+  // warps on its longest pairs; on streams of their own (in a captured call,
+  // branches of the graph) one order's blocks take the room that another's
+  // leave, where one after the other each would wait for the last pair before.
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   if (c->time_rounds) {
     RT_TRY(next_events(c, &t0, &t1));
     RT_TRY(record_event(t0, s));
   }
+  const bool fork = __builtin_popcount(c->orders) > 1;
+  if (fork) RT_TRY(cudaEventRecord(c->order_fork, s));
   cudaError_t e = cudaSuccess;
-  for (int n = kMinModes; n <= kMaxModes && e == cudaSuccess; ++n) {
+  bool first = true;
+  for (int n = kMaxModes; n >= kMinModes && e == cudaSuccess; --n) {
     if (!((c->orders >> n) & 1u)) continue;
     RoundParams Rn = R;
     Rn.batch_base = rb.ctr + kCtrOrderOff + n;
     Rn.n_batches = rb.ctr + kCtrOrderNb + n;
     Rn.next_batch = rb.ctr + kCtrOrderNext + n;
+    // the first (largest) order stays on the call's stream
+    cudaStream_t so = first ? s : c->order_streams[n];
+    if (!first) RT_TRY(cudaStreamWaitEvent(so, c->order_fork, 0));
     switch (n) {
-      case 2: e = launch_round_n<2>(Rn, s, learned, c->use_tc); break;
-      case 3: e = launch_round_n<3>(Rn, s, learned, c->use_tc); break;
-      case 4: e = launch_round_n<4>(Rn, s, learned, c->use_tc); break;
-      case 5: e = launch_round_n<5>(Rn, s, learned, c->use_tc); break;
-      case 6: e = launch_round_n<6>(Rn, s, learned, c->use_tc); break;
-      case 7: e = launch_round_n<7>(Rn, s, learned, c->use_tc); break;
-      case 8: e = launch_round_n<8>(Rn, s, learned, c->use_tc); break;
-      case 9: e = launch_round_n<9>(Rn, s, learned, c->use_tc); break;
+      case 2: e = launch_round_n<2>(Rn, so, learned, c->use_tc); break;
+      case 3: e = launch_round_n<3>(Rn, so, learned, c->use_tc); break;
+      case 4: e = launch_round_n<4>(Rn, so, learned, c->use_tc); break;
+      case 5: e = launch_round_n<5>(Rn, so, learned, c->use_tc); break;
+      case 6: e = launch_round_n<6>(Rn, so, learned, c->use_tc); break;
+      case 7: e = launch_round_n<7>(Rn, so, learned, c->use_tc); break;
+      case 8: e = launch_round_n<8>(Rn, so, learned, c->use_tc); break;
+      case 9: e = launch_round_n<9>(Rn, so, learned, c->use_tc); break;
       default: e = cudaErrorInvalidValue; break;
     }
+    if (!first && e == cudaSuccess) e = cudaEventRecord(c->order_done[n], so);
+    if (!first && e == cudaSuccess) e = cudaStreamWaitEvent(s, c->order_done[n], 0);
+    first = false;
   }
   RT_TRY(e);
   if (t1) RT_TRY(record_event(t1, s));

@@ -793,7 +793,8 @@ __device__ __forceinline__ void setc(float3& v, int a, float s) {
 }
 
 // Point and the two tangents of face f (face_param's free axes ua < va) at
-// its free coordinates (u, v): out[c] = {x_c, dx_c/du, dx_c/dv, 0}.
+// its free coordinates (u, v), components 0 to comps - 1 (x, y, z, the field):
+// out[c] = {x_c, dx_c/du, dx_c/dv, 0}.
 //
 // On a face the fixed coordinate is exactly -1 or 1, where one vertex mode is
 // exactly 1 and every other mode exactly 0, so of the contraction over three
@@ -804,7 +805,7 @@ __device__ __forceinline__ void setc(float3& v, int a, float s) {
 // multiply-adds. The face solves are most of the round kernel's steps; their
 // evaluations' cost was 2 (2N^3 + 3N^2) operations a component.
 template <int N, bool SM>
-__device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, float4* __restrict__ out) {
+__device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, int comps, float4* __restrict__ out) {
   constexpr int RS = row_stride(N);
   int fixed, ua, va;
   float val;
@@ -816,7 +817,7 @@ __device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, f
   basis_val_der<N>(u, pu, du);
   basis_val_der<N>(v, pv, dv);
 #pragma unroll 1
-  for (int comp = 0; comp < 3; ++comp) {
+  for (int comp = 0; comp < comps; ++comp) {
     const CoefRef<SM> cc = c.at(comp * block_floats(N) + m * sf);
     float x = 0.f, xu = 0.f, xv = 0.f;
 #pragma unroll 1
@@ -1061,6 +1062,14 @@ __device__ __forceinline__ float3 face_normal(const float (&J)[9], float3 xi, fl
   n = normalize3(n);
   if (n.x * d.x + n.y * d.y + n.z * d.z > 0.f) n = make_float3(-n.x, -n.y, -n.z);
   return n;
+}
+
+// Does face_normal take a hit on face f from the face's own two tangents?
+__device__ __forceinline__ bool normal_on_face(int f, float3 xi) {
+  int fixed, ua, va;
+  float val;
+  face_param(f, fixed, val, ua, va);
+  return fixed == 0 || (!(fabsf(xi.x) > 0.9f) && (fixed == 1 || !(fabsf(xi.y) > 0.9f)));
 }
 
 // What a hit committed with kFlagPost lacks, from the Jacobian and the field

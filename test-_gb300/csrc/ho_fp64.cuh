@@ -170,6 +170,70 @@ __device__ double value64(const float* __restrict__ blk, const float (&ah)[N], c
   return static_cast<double>(v.hi) + static_cast<double>(v.lo);
 }
 
+// value64 at a point on a face (the fixed axis' coordinate is exactly -1 or 1):
+// there the basis values across the face are exactly 1 for one vertex mode m
+// and exactly 0 for the others, products and sums with those are exact, and
+// what is left is the sum over the face's N x N coefficients with the other
+// two axes' values, operation by operation the one that value64 makes (a, b
+// and their strides: the inner and the outer of those axes). The same double-
+// single number at 1 / N of the work; nearly all hits are on faces.
+template <int N>
+__device__ double face_value64(const float* __restrict__ blk, bool inner_i, int sa, int sb, const Ds (&pa)[N],
+                               const Ds (&pb)[N]) {
+  Ds v = {0.f, 0.f};
+#pragma unroll 1
+  for (int b = 0; b < N; ++b) {
+    Ds q = {0.f, 0.f};
+    const float* row = blk + b * sb;
+    if (inner_i) {  // the sum over i: exact products, the running sum in two floats
+      float sh = 0.f, sl = 0.f;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const float c = __ldg(row + i * sa);
+        const float p = __fmul_rn(c, pa[i].hi);
+        const float ep = __fmaf_rn(c, pa[i].hi, -p);
+        float s, es;
+        two_sum(sh, p, s, es);
+        sh = s;
+        sl = __fadd_rn(sl, __fadd_rn(__fadd_rn(es, ep), __fmul_rn(c, pa[i].lo)));
+      }
+      q = ds_norm(sh, sl);
+    } else {  // the sum over j
+#pragma unroll
+      for (int j = 0; j < N; ++j) q = ds_add(q, ds_mul({__ldg(row + j * sa), 0.f}, pa[j]));
+    }
+    Ds pk = pb[0];  // pb[b] by selection: the array stays in registers
+#pragma unroll
+    for (int kk = 1; kk < N; ++kk)
+      if (kk == b) pk = pb[kk];
+    v = ds_add(v, ds_mul(q, pk));
+  }
+  return static_cast<double>(v.hi) + static_cast<double>(v.lo);
+}
+
+// fp64_residual_vec for a point on face f.
+template <int N>
+__device__ __noinline__ void fp64_face_residual(const float* __restrict__ rec_all, int elem, int f, float3 o, float3 d,
+                                                double t, double x0, double x1, double x2, bool want_field,
+                                                double* __restrict__ r, double& u) {
+  constexpr int RS = row_stride(N);
+  const float* rec = rec_all + static_cast<int64_t>(elem) * record_floats(N);
+  int fixed, ua, va;
+  float val;
+  face_param(f, fixed, val, ua, va);
+  const int m = val < 0.f ? 0 : 1;
+  rec += m * (fixed == 0 ? 1 : (fixed == 1 ? RS : N * RS));
+  const bool inner_i = ua == 0;
+  const int sa = inner_i ? 1 : RS, sb = va == 1 ? RS : N * RS;
+  Ds pa[N], pb[N];
+  basis_val_ds<N>(ds_of(inner_i ? x0 : x1), pa);
+  basis_val_ds<N>(ds_of(va == 1 ? x1 : x2), pb);
+  r[0] = face_value64<N>(rec, inner_i, sa, sb, pa, pb) - (static_cast<double>(o.x) + t * d.x);
+  r[1] = face_value64<N>(rec + block_floats(N), inner_i, sa, sb, pa, pb) - (static_cast<double>(o.y) + t * d.y);
+  r[2] = face_value64<N>(rec + 2 * block_floats(N), inner_i, sa, sb, pa, pb) - (static_cast<double>(o.z) + t * d.z);
+  u = want_field ? face_value64<N>(rec + 3 * block_floats(N), inner_i, sa, sb, pa, pb) : 0.0;
+}
+
 // The FP64 residual vector r = x(xi) - (o + t d) of a point in element elem,
 // and the field value u(xi) (0 when unused).
 template <int N>
@@ -274,8 +338,20 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
   if (h.kind == HO_HIT_MISS) return true;
   const bool iso_hit = h.kind != HO_HIT_FACE;
   const bool has_field = iso_hit || (__ldg(eflags + h.elem) & 1u) != 0;
+  // a face hit's fixed coordinate is exactly -1 or 1, and the polish keeps it
+  bool on_face = false;
+  if (!iso_hit) {
+    int fixed, ua, va;
+    float val;
+    face_param(h.face, fixed, val, ua, va);
+    on_face = getc(h.xi, fixed) == val;
+  }
+  const auto residual = [&](double t, double x0, double x1, double x2, double (&r)[3], double& u) {
+    if (on_face) fp64_face_residual<N>(rec_all, h.elem, h.face, o, d, t, x0, x1, x2, has_field, r, u);
+    else fp64_residual_vec<N>(rec_all, h.elem, o, d, t, x0, x1, x2, has_field, r, u);
+  };
   double r[3], u;
-  fp64_residual_vec<N>(rec_all, h.elem, o, d, h.t, h.xi.x, h.xi.y, h.xi.z, has_field, r, u);
+  residual(h.t, h.xi.x, h.xi.y, h.xi.z, r, u);
   const double rpos = fmax(fabs(r[0]), fmax(fabs(r[1]), fabs(r[2])));
   if (!iso_hit) {
     if (rpos > kCheckFaceTol) return false;
@@ -288,6 +364,24 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
   float3 g = make_float3(0.f, 0.f, 0.f);
   float u32 = 0.f;
   auto jacobian_at = [&](float3 xi) {
+    if (on_face) {  // the two tangents and the field's derivatives along them: all that a face hit's steps use
+      int fixed, ua, va;
+      float val;
+      face_param(h.face, fixed, val, ua, va);
+      float4 fr[4];
+      face_eval<N, false>(c, h.face, getc(xi, ua), getc(xi, va), has_field ? 4 : 3, fr);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        J[3 * k] = ua == 0 ? fr[k].y : 0.f;
+        J[3 * k + 1] = ua == 1 ? fr[k].y : (va == 1 ? fr[k].z : 0.f);
+        J[3 * k + 2] = va == 2 ? fr[k].z : 0.f;
+      }
+      if (has_field) {
+        g = make_float3(ua == 0 ? fr[3].y : 0.f, ua == 1 ? fr[3].y : (va == 1 ? fr[3].z : 0.f), va == 2 ? fr[3].z : 0.f);
+        u32 = fr[3].x;
+      }
+      return;
+    }
     float xJ[12];
     geom_eval_raw<N, false>(c, xi, xJ);
     J[0] = xJ[1]; J[1] = xJ[2]; J[2] = xJ[3];
@@ -301,7 +395,16 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
     }
   };
   jacobian_at(h.xi);
-  if (h.flags & kFlagPost) fill_hit(h, J, u32, d);
+  if (h.flags & kFlagPost) {
+    if (on_face && !normal_on_face(h.face, h.xi)) {  // near another face's edge the normal takes the third column
+      float xJ[12];
+      geom_eval_raw<N, false>(c, h.xi, xJ);
+      const float Jn[9] = {xJ[1], xJ[2], xJ[3], xJ[5], xJ[6], xJ[7], xJ[9], xJ[10], xJ[11]};
+      fill_hit(h, Jn, u32, d);
+    } else {
+      fill_hit(h, J, u32, d);
+    }
+  }
   const float dn = fabsf(h.n.x * d.x + h.n.y * d.y + h.n.z * d.z);
   const bool steep = dn >= 0.2f * sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
   double t = h.t, x0 = h.xi.x, x1 = h.xi.y, x2 = h.xi.z, un = u;
@@ -322,7 +425,7 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
     if (step + 1 == kPolishSteps || (mx <= done && fabs(dt) <= done)) break;
     if (mx > 1e-3)
       jacobian_at(make_float3(static_cast<float>(x0), static_cast<float>(x1), static_cast<float>(x2)));
-    fp64_residual_vec<N>(rec_all, h.elem, o, d, t, x0, x1, x2, has_field, r, u);
+    residual(t, x0, x1, x2, r, u);
     un = u;
   }
   if (h.kind == HO_HIT_FACE) {

@@ -116,9 +116,13 @@ __global__ void round_init_kernel(RayState* __restrict__ st, const uint8_t* __re
 // they were solved or ended here, so which of the two kernels solves a
 // candidate does not depend on how many ended here (their face Newtons
 // differ in the last bits on a few rays).
+// settle: before the tail, rays go on past the candidates that end here and
+// stop before the first that has to be solved (no pairs are written), so the
+// tail's list holds only rays with something left to solve.
 __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, RoundPair* __restrict__ pairs,
                                     int32_t* __restrict__ pkey, uint32_t* __restrict__ prank,
-                                    uint32_t* __restrict__ kcount, unsigned* __restrict__ ctr, int limit) {
+                                    uint32_t* __restrict__ kcount, unsigned* __restrict__ ctr, int limit,
+                                    bool settle) {
   const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   bool live = item < *P.qcount && !st[item].done;
@@ -164,7 +168,8 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
         done = true;
         break;
       }
-      const int j = cursor;
+      const int j = cursor, e0 = ke;
+      const float k0 = kt;
       ++cursor;
       kt = ct;
       ke = ce;
@@ -192,6 +197,12 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
         ++w.cand;
         w.culled += 6;
         continue;
+      }
+      if (settle) {
+        cursor = j;
+        kt = k0;
+        ke = e0;
+        break;
       }
       p.item = static_cast<int32_t>(item);
       p.j = (pass == 0 ? j : kPairPred) | (scan ? 0 : kPairNoIso);
@@ -560,7 +571,8 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   const int64_t n_keys = 2 * n_elem;
   RT_TRY(cudaMemsetAsync(rb.kcount, 0, static_cast<size_t>(n_keys) * sizeof(uint32_t), s));
   RT_TRY(cudaMemsetAsync(rb.ctr, 0, kCtrWords * sizeof(unsigned), s));
-  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, gathered, rb.pkey, rb.prank, rb.kcount, rb.ctr, limit);
+  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, gathered, rb.pkey, rb.prank, rb.kcount, rb.ctr, limit,
+                                      false);
   {
     const unsigned tiles = static_cast<unsigned>((n_keys + kScanTile - 1) / kScanTile);
     if (tiles > 0) {
@@ -627,6 +639,8 @@ static int enqueue_tail(ho_context* c, const TraceParams& P, const RoundParams& 
   unsigned* n_list = rb.ctr + 4;
   unsigned* next = rb.ctr + 5;
   RT_TRY(cudaMemsetAsync(rb.ctr + 4, 0, 2 * sizeof(unsigned), s));
+  round_gather_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(
+      P, R.state, static_cast<RoundPair*>(rb.pairs), rb.pkey, rb.prank, rb.kcount, rb.ctr, 0, true);
   ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, R.state, false, rb.fail,
                                                                              n_list, P.stats);
   RT_TRY(cudaGetLastError());
@@ -644,7 +658,7 @@ static int enqueue_tail(ho_context* c, const TraceParams& P, const RoundParams& 
   }
   RT_TRY(e);
   RT_TRY(cudaMemsetAsync(rb.ctr, 0, sizeof(unsigned), s));
-  c->launches += 2;
+  c->launches += 3;
   return 0;
 }
 

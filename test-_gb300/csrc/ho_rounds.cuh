@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
             int fixed, ua, va;
             float val;
             face_param(f, fixed, val, ua, va);
-            face_eval<N, true>(el.c, f, getc(s.xi, ua), getc(s.xi, va), r);
+            face_eval<N, true>(el.c, f, getc(s.xi, ua), getc(s.xi, va), 3, r);
           } else {
             eval_comps<N, true>(el.c, s.xi, 0, 4, r);
           }

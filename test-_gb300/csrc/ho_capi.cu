@@ -226,6 +226,8 @@ void ho_destroy(ho_context* c) {
     cudaFree(c->d_stats);
     cudaFree(c->d_hits);
     cudaFree(c->d_phits);
+    cudaFree(c->d_pheavy);
+    if (c->pheavy_done) cudaEventDestroy(c->pheavy_done);
     if (c->prim_events[0]) cudaEventDestroy(c->prim_events[0]);
     if (c->prim_events[1]) cudaEventDestroy(c->prim_events[1]);
     if (c->call_done) cudaEventDestroy(c->call_done);

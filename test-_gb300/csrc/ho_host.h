@@ -77,6 +77,8 @@ int element_order(const HostScene& hs, int64_t e);
 // pack_records at N = order[e]).
 void pack_compact(const HostScene& hs, std::vector<float>& rec, std::vector<int64_t>& off, std::vector<uint8_t>& order);
 
+// Inverse of a dense n x n matrix (row-major, FP64); false when singular.
+bool invert_dense(std::vector<double> a, int n, std::vector<double>& inv);
 // 1-D change of basis Modified-A -> Bernstein on [a,b] for n modes:
 // phi_i(x) = sum_k M[i*n+k] * B_k((x-a)/(b-a)).
 void modal_to_bernstein(int n, double a, double b, std::vector<double>& M);
@@ -175,6 +177,8 @@ struct ho_context {
   // prisms, quads and curved triangles (ho_prim.cu)
   int64_t n_prims = 0;
   void* d_prims = nullptr;        // n_prims PrimRec, kind-major
+  void* d_pcull = nullptr;        // n_prims PrimCull
+  float* d_pstart = nullptr;      // per prism: the points of its solver's 7 starts (21 floats)
   float* d_pgeom = nullptr;
   float* d_pfield = nullptr;
   float* d_pbox = nullptr;        // n_prims * 6
@@ -182,6 +186,9 @@ struct ho_context {
   int64_t n_pnodes = 0;
   int pbvh_depth = 0;
   int64_t prim_counts[3] = {0, 0, 0};
+  void* d_pheavy = nullptr;       // queries that the primitive pass hands to its warp-per-query kernel
+  size_t pheavy_cap = 0;          // its bytes
+  cudaEvent_t pheavy_done = nullptr;  // that kernel's last launch
   ho_hit* d_phits = nullptr;      // hits of calls that asked for none (the primitive pass needs them)
   size_t phits_cap = 0;
   cudaEvent_t prim_events[2] = {nullptr, nullptr};  // HO_OPT_TIME_ROUNDS: around the primitive pass
@@ -296,7 +303,10 @@ void prims_free(ho_context* c);
 // replaced by a nearer primitive hit. fresh: the hexahedra were not traced
 // (a scene without them); every query is written.
 // stats: device counters for the traversal status (nullptr: the context's).
-int launch_prims(ho_context* c, const TraceArgs& a, ho_hit* hits, bool fresh, DevStats* stats, cudaStream_t s);
+// may_allocate: grow the context's list of queries for the second kernel (one
+// that may not runs every query to its end on one thread).
+int launch_prims(ho_context* c, const TraceArgs& a, ho_hit* hits, bool fresh, DevStats* stats, cudaStream_t s,
+                 bool may_allocate = true);
 // The FP64 check's residuals for caller-given hits (ho_rounds.cu).
 int launch_residuals(ho_context* c, int64_t n, const float* rays, const ho_hit* hits, double* out, cudaStream_t s);
 }  // namespace ho

@@ -155,7 +155,7 @@ extern "C" int ho_intersect_device_noalloc(ho_context* c, int64_t n, const float
     a.n_iso = 1;
     a.iso[0] = iso;
     a.iso_on_mask = P.iso_on_mask;
-    e = static_cast<cudaError_t>(launch_prims(c, a, out_dev, true, P.stats, s));
+    e = static_cast<cudaError_t>(launch_prims(c, a, out_dev, true, P.stats, s, false));
     if (e != cudaSuccess) {
       c->err = std::string("primitive kernel: ") + cudaGetErrorString(e);
       return HO_ERR_CUDA;
@@ -184,7 +184,7 @@ extern "C" int ho_intersect_device_noalloc(ho_context* c, int64_t n, const float
     a.n_iso = 1;
     a.iso[0] = iso;
     a.iso_on_mask = P.iso_on_mask;
-    e = static_cast<cudaError_t>(launch_prims(c, a, out_dev, false, P.stats, s));
+    e = static_cast<cudaError_t>(launch_prims(c, a, out_dev, false, P.stats, s, false));
   }
   if (e != cudaSuccess) {
     c->err = std::string("trace kernels: ") + cudaGetErrorString(e);

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -58,9 +59,135 @@ __global__ void prim_setup_kernel(PrimRec* __restrict__ recs, const float* __res
   }
 }
 
+// Interpolation on [-1.05, 1.05] at n points and the change to the Bernstein
+// basis of degree n - 1 there: a polynomial lies between its Bernstein
+// coefficients' extremes. amp: the change's infinity norm, for the rounding.
+struct PrimMats {
+  float node[kPrimMaxModes + 1][kPrimMaxModes];
+  float inv[kPrimMaxModes + 1][kPrimMaxModes * kPrimMaxModes];
+  float amp[kPrimMaxModes + 1];
+};
+
+// One block per primitive, once per scene: the oriented bounds over r, s (, t)
+// in [-1.05, 1.05], the widest range that a hit or a quad's containment test
+// accepts (a linear triangle clamps its point into the triangle: its
+// vertices), along the rows of the inverse Jacobian at the centre.
+__global__ void __launch_bounds__(64) prim_cull_kernel(const PrimRec* __restrict__ recs, const float* __restrict__ pool,
+                                                       const PrimMats* __restrict__ mats, PrimCull* __restrict__ cull,
+                                                       float* __restrict__ start) {
+  constexpr int kMost = kPrimMaxModes * kPrimMaxModes * kPrimMaxModes;
+  __shared__ float pt[2][3][kMost];
+  __shared__ float red[64];
+  const PrimRec& p = recs[blockIdx.x];
+  const bool curved = pr_curved(p);
+  if (p.kind == kPrimPrism && threadIdx.x < 7) {  // the points of the prism solver's starts
+    const float3 X = pr_point(p, pool, pr_prism_start(threadIdx.x));
+    float* x = start + 21 * static_cast<int64_t>(blockIdx.x) + 3 * threadIdx.x;
+    x[0] = X.x;
+    x[1] = X.y;
+    x[2] = X.z;
+  }
+  int dim[3] = {1, 1, 1};
+  if (p.kind == kPrimTri) {
+    dim[0] = 3;
+  } else {
+    for (int a = 0; a < (p.kind == kPrimPrism ? 3 : 2); ++a) dim[a] = curved ? max(2, static_cast<int>(pmode(p.gm, a))) : 2;
+  }
+  const int n = dim[0] * dim[1] * dim[2];
+  float amp = 1.f;
+  int cur = 0;
+  if (p.kind == kPrimTri) {
+    if (threadIdx.x < 3)
+      for (int a = 0; a < 3; ++a) pt[0][a][threadIdx.x] = p.v[3 * threadIdx.x + a];
+    __syncthreads();
+  } else {
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+      const int i = q % dim[0], j = (q / dim[0]) % dim[1], k = q / (dim[0] * dim[1]);
+      const float3 X = pr_point(p, pool, make_float3(mats->node[dim[0]][i], mats->node[dim[1]][j],
+                                                     p.kind == kPrimPrism ? mats->node[dim[2]][k] : 0.f));
+      pt[0][0][q] = X.x;
+      pt[0][1][q] = X.y;
+      pt[0][2][q] = X.z;
+    }
+    __syncthreads();
+    int stride = 1;
+    for (int ax = 0; ax < (p.kind == kPrimPrism ? 3 : 2); ++ax) {
+      const float* M = mats->inv[dim[ax]];
+      amp *= mats->amp[dim[ax]];
+      for (int q = threadIdx.x; q < n; q += blockDim.x) {
+        const int at = (q / stride) % dim[ax], base = q - at * stride;
+        for (int a = 0; a < 3; ++a) {
+          float v = 0.f;
+          for (int r = 0; r < dim[ax]; ++r) v += M[at * kPrimMaxModes + r] * pt[cur][a][base + r * stride];
+          pt[cur ^ 1][a][q] = v;
+        }
+      }
+      stride *= dim[ax];
+      cur ^= 1;
+      __syncthreads();
+    }
+  }
+  // directions: rows of the inverse of the tangents at the centre (a surface's
+  // third tangent: its normal)
+  float3 t[3];
+  if (p.kind == kPrimTri) {
+    t[0] = pr_sub(pr_vert(p, 1), pr_vert(p, 0));
+    t[1] = pr_sub(pr_vert(p, 2), pr_vert(p, 0));
+  } else {
+    float3 X;
+    pr_geom(p, pool, make_float3(0.f, 0.f, 0.f), X, t);
+  }
+  if (p.kind != kPrimPrism) t[2] = pr_cross(t[0], t[1]);
+  const float3 c[3] = {pr_cross(t[1], t[2]), pr_cross(t[2], t[0]), pr_cross(t[0], t[1])};
+  const float det = pr_dot(t[0], c[0]);
+  const float inv = 1.0f / det;
+  PrimCull out;
+  float size = 0.f;
+  bool ok = !(p.kind == kPrimTri && curved) && fabsf(det) > 1e-30f && fabsf(inv) < 1e30f;
+  const auto block_max = [&](float x) {
+    red[threadIdx.x] = x == x ? x : FLT_MAX;  // a NaN counts as infinite
+    __syncthreads();
+    for (int h = 32; h > 0; h >>= 1) {
+      if (threadIdx.x < h) red[threadIdx.x] = fmaxf(red[threadIdx.x], red[threadIdx.x + h]);
+      __syncthreads();
+    }
+    const float r = red[0];
+    __syncthreads();
+    return r;
+  };
+  for (int a = 0; a < 3; ++a) {
+    float m = 0.f;
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+      const float v = fabsf(pt[cur][a][q]);
+      m = v <= FLT_MAX ? fmaxf(m, v) : FLT_MAX;
+    }
+    size = fmaxf(size, block_max(m));
+  }
+  ok = ok && size < 1e15f;
+  for (int k = 0; k < 3; ++k) {
+    const float mv[3] = {c[k].x * inv, c[k].y * inv, c[k].z * inv};
+    const float m1 = fabsf(mv[0]) + fabsf(mv[1]) + fabsf(mv[2]);
+    float lo = FLT_MAX, hi = -FLT_MAX;
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+      const float v = mv[0] * pt[cur][0][q] + mv[1] * pt[cur][1][q] + mv[2] * pt[cur][2][q];
+      lo = fminf(lo, v);
+      hi = fmaxf(hi, v);
+    }
+    const float slack = m1 * size * 1e-6f * (2.f + amp);
+    out.lo[k] = -block_max(-lo) - slack;
+    out.hi[k] = block_max(hi) + slack;
+    for (int a = 0; a < 3; ++a) out.m[3 * k + a] = mv[a];
+    ok = ok && m1 < 1e20f && fabsf(out.lo[k]) < 1e25f && fabsf(out.hi[k]) < 1e25f;
+  }
+  out.size = ok ? size : -1.f;
+  if (threadIdx.x == 0) cull[blockIdx.x] = out;
+}
+
 struct PrimParams {
   const BNode* __restrict__ nodes;
   const PrimRec* __restrict__ prims;
+  const PrimCull* __restrict__ cull;
+  const float* __restrict__ start;  // per prism: the points of its solver's 7 starts
   const float* __restrict__ geom;
   const float* __restrict__ field;
   const float* __restrict__ rays;
@@ -75,43 +202,114 @@ struct PrimParams {
   int64_t n_queries;
   bool fresh;
   DevStats* stats;
+  struct PrimHeavy* heavy;  // queries handed to the warp-per-query kernel (nullptr: none are)
+  unsigned heavy_cap;       // the most that fit
+  unsigned* heavy_ctr;      // their count (it may pass heavy_cap), and the next to take
 };
 
-// One query's primitive pass: the candidates in (box entry, index) order on
-// [0.001, closest hit so far], then the hit record and the pixel.
-__device__ __forceinline__ void prim_query(const PrimParams& P, int64_t q, PrimWork& pw, unsigned& cand, Work& w) {
+// A primitive whose bounds the ray misses is no candidate, nor a prism whose
+// starts all end at once.
+struct PrimKeep {
+  const PrimParams& P;
   float3 o, d;
-  float iso;
-  bool iso_on;
-  query_ray_from(P.rays, P.n_rays, P.cam, P.iso, P.iso_mask, P.views, P.n_views, q, o, d, iso, iso_on);
-  ho_hit h;
-  if (P.fresh) {
-    h.t = FLT_MAX;
-    h.elem = -1;
-    h.face = -1;
-    h.kind = HO_HIT_MISS;
-    for (int a = 0; a < 3; ++a) h.xi[a] = h.n[a] = 0.f;
-    h.u = 0.f;
-    h.flags = 0;
-    h.iters = 0;
-  } else {
-    h = P.hits[q];
+  float tmax;
+  __device__ __forceinline__ bool operator()(int e) const {
+    if (!pr_may_hit(P.cull[e], o, d, 0.001f, tmax, kPrimTol)) return false;
+    const PrimRec& p = P.prims[e];
+    return p.kind != kPrimPrism || pr_prism_begins(p, P.start + 21 * static_cast<int64_t>(e), o, d, 0.001f, tmax);
   }
-  float best = h.kind != HO_HIT_MISS ? h.t : FLT_MAX;
-  int win = -1;
-  float3 xw = make_float3(0.f, 0.f, 0.f);
+};
+
+// A query's answer so far and where its candidate walk stands.
+struct PrimState {
+  float best;  // closest hit so far
+  int win;     // its primitive (-1: none of this pass)
+  float3 x;
+  float kt;  // last visited key (entry, index)
+  int ke;
+};
+// A query handed to the warp-per-query kernel.
+struct PrimHeavy {
+  int32_t q;
+  uint32_t iters;
+  PrimState s;
+};
+// Iterations after which a query is handed over. A quad's or a triangle's
+// start search takes 1,000 to 4,000 iterations when it finds nothing; on one
+// thread a ray that passes several such surfaces ran for hundreds of
+// milliseconds after the others had ended.
+constexpr uint32_t kPrimBudget = 256;
+// Most queries handed over in a call (40 bytes each); the others run to their
+// end where they are.
+constexpr int64_t kPrimHeavyMost = int64_t(1) << 22;
+
+__device__ __forceinline__ ho_hit prim_base(const PrimParams& P, int64_t q) {
+  if (!P.fresh) return P.hits[q];
+  ho_hit h;
+  h.t = FLT_MAX;
+  h.elem = -1;
+  h.face = -1;
+  h.kind = HO_HIT_MISS;
+  for (int a = 0; a < 3; ++a) h.xi[a] = h.n[a] = 0.f;
+  h.u = 0.f;
+  h.flags = 0;
+  h.iters = 0;
+  return h;
+}
+
+// The hit record and the pixel of a finished query.
+__device__ __forceinline__ void prim_finish(const PrimParams& P, int64_t q, float3 d, ho_hit h, const PrimState& s,
+                                            uint32_t iters, bool incomplete) {
+  if (s.win >= 0) {
+    const PrimRec& p = P.prims[s.win];
+    const float3 n = pr_normal(p, P.geom, s.x, d);
+    h.t = s.best;
+    h.elem = p.local;
+    h.face = -1;
+    h.kind = static_cast<int16_t>(HO_HIT_PRISM + p.kind);
+    h.xi[0] = s.x.x;
+    h.xi[1] = s.x.y;
+    h.xi[2] = s.x.z;
+    h.n[0] = n.x;
+    h.n[1] = n.y;
+    h.n[2] = n.z;
+    h.u = pr_field(p, P.field, s.x);
+    h.flags = 0;
+  }
+  h.iters += iters;
+  if (incomplete) h.flags |= HO_FLAG_INCOMPLETE;
+  if (P.hits && (P.fresh || s.win >= 0 || incomplete)) P.hits[q] = h;
+  if (P.rgb && P.rays == nullptr && (P.fresh || s.win >= 0)) {
+    HitState v;
+    v.t = h.t;
+    v.elem = h.elem;
+    v.face = h.face;
+    v.kind = h.kind;
+    v.n = make_float3(h.n[0], h.n[1], h.n[2]);
+    shade(v, d, P.rgb + 3 * q);
+  }
+}
+
+// The candidates of a query in (box entry, index) order on [0.001, closest hit
+// so far], from where its walk stands. One thread's form (W = false) hands
+// over after kPrimBudget iterations when it may (returns false, with the place
+// in the list); a warp's form
+// (all lanes with the same arguments; wu: the work that all lanes repeat) runs
+// to the end.
+template <bool W>
+__device__ __forceinline__ bool prim_walk(const PrimParams& P, float3 o, float3 d, PrimState& s, PrimWork& pw,
+                                          PrimWork& wu, unsigned& cand, Work& w, bool& incomplete,
+                                          unsigned* place = nullptr) {
   const uint32_t iters0 = pw.iters;
-  float kt = -FLT_MAX;
-  int ke = -1;
-  bool incomplete = false;
+  bool asked = false;
   for (;;) {
     float bt[kPrimCandK];
     int be[kPrimCandK];
     bool overflow;
-    if (!collect_in<kPrimCandK>(P.nodes, o, d, best, kt, ke, bt, be, overflow, w)) {
-      atomicOr(&P.stats->status, kStatusStackOverflow);
+    if (!collect_in<kPrimCandK>(P.nodes, o, d, s.best, s.kt, s.ke, bt, be, overflow, w, PrimKeep{P, o, d, s.best})) {
+      if (!W || (threadIdx.x & 31) == 0) atomicOr(&P.stats->status, kStatusStackOverflow);
       incomplete = true;
-      break;
+      return true;
     }
     bool done = false;
 #pragma unroll 1
@@ -124,61 +322,71 @@ __device__ __forceinline__ void prim_query(const PrimParams& P, int64_t q, PrimW
           ct = bt[m];
           ce = be[m];
         }
-      if (ce == INT_MAX || ct > best) {
+      if (ce == INT_MAX || ct > s.best) {
         done = true;
         break;
       }
+      if (!W && P.heavy && !asked && pw.iters - iters0 > kPrimBudget) {
+        asked = true;
+        *place = atomicAdd(P.heavy_ctr, 1u);
+        if (*place < P.heavy_cap) return false;
+      }
       const PrimRec& p = P.prims[ce];  // read in place: the solvers take it by reference
+      const PrimCull& c = P.cull[ce];
+      const float* start = P.start + 21 * static_cast<int64_t>(ce);
       float te, tx, th;
       float3 xh;
       ++cand;
-      if (pr_slab(o, d, p.lo, p.hi, 0.001f, best, te, tx) && pr_hit(p, P.geom, o, d, 0.001f, best, th, xh, pw) &&
-          th > 0.001f && th < best) {
-        best = th;
-        win = ce;
-        xw = xh;
+      if (pr_slab(o, d, p.lo, p.hi, 0.001f, s.best, te, tx)) {
+        bool hit;
+        if (W)
+          hit = p.kind == kPrimPrism ? pr_hit_prism_warp(p, c, start, P.geom, o, d, 0.001f, s.best, th, xh, pw)
+                                     : pr_hit_surface_warp(p, c, P.geom, o, d, 0.001f, s.best, th, xh, pw, wu);
+        else
+          hit = p.kind == kPrimPrism ? pr_hit_prism(p, c, start, P.geom, o, d, 0.001f, s.best, th, xh, pw)
+                                     : pr_hit_surface(p, c, P.geom, o, d, 0.001f, s.best, th, xh, pw);
+        if (hit && th > 0.001f && th < s.best) {
+          s.best = th;
+          s.win = ce;
+          s.x = xh;
+        }
       }
-      kt = ct;
-      ke = ce;
+      s.kt = ct;
+      s.ke = ce;
     }
-    if (done || !overflow) break;
-  }
-  if (win >= 0) {
-    const PrimRec& p = P.prims[win];
-    const float3 n = pr_normal(p, P.geom, xw, d);
-    h.t = best;
-    h.elem = p.local;
-    h.face = -1;
-    h.kind = static_cast<int16_t>(HO_HIT_PRISM + p.kind);
-    h.xi[0] = xw.x;
-    h.xi[1] = xw.y;
-    h.xi[2] = xw.z;
-    h.n[0] = n.x;
-    h.n[1] = n.y;
-    h.n[2] = n.z;
-    h.u = pr_field(p, P.field, xw);
-    h.flags = 0;
-  }
-  h.iters += pw.iters - iters0;
-  if (incomplete) h.flags |= HO_FLAG_INCOMPLETE;
-  if (P.hits && (P.fresh || win >= 0 || incomplete)) P.hits[q] = h;
-  if (P.rgb && P.rays == nullptr && (P.fresh || win >= 0)) {
-    HitState s;
-    s.t = h.t;
-    s.elem = h.elem;
-    s.face = h.face;
-    s.kind = h.kind;
-    s.n = make_float3(h.n[0], h.n[1], h.n[2]);
-    shade(s, d, P.rgb + 3 * q);
+    if (done || !overflow) return true;
   }
 }
 
 __global__ void __launch_bounds__(kPrimThreads, HO_PRIM_MIN_BLOCKS) prim_trace_kernel(PrimParams P) {
-  PrimWork pw;
+  PrimWork pw, wu;
   unsigned cand = 0;
   Work w;
   const int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (q < P.n_queries) prim_query(P, q, pw, cand, w);
+  if (q < P.n_queries) {
+    float3 o, d;
+    float iso;
+    bool iso_on;
+    query_ray_from(P.rays, P.n_rays, P.cam, P.iso, P.iso_mask, P.views, P.n_views, q, o, d, iso, iso_on);
+    const ho_hit h = prim_base(P, q);
+    PrimState s;
+    s.best = h.kind != HO_HIT_MISS ? h.t : FLT_MAX;
+    s.win = -1;
+    s.x = make_float3(0.f, 0.f, 0.f);
+    s.kt = -FLT_MAX;
+    s.ke = -1;
+    bool incomplete = false;
+    unsigned place = 0;
+    if (prim_walk<false>(P, o, d, s, pw, wu, cand, w, incomplete, &place)) {
+      prim_finish(P, q, d, h, s, pw.iters, incomplete);
+    } else {
+      PrimHeavy v;
+      v.q = static_cast<int32_t>(q);
+      v.iters = pw.iters;
+      v.s = s;
+      P.heavy[place] = v;
+    }
+  }
   // counters: summed over the warp when all its lanes are here together
   // (the last block's tail warp is partial), else added one by one
   const unsigned long long v[4] = {cand, pw.iters, pw.flops, w.nodes};
@@ -192,6 +400,46 @@ __global__ void __launch_bounds__(kPrimThreads, HO_PRIM_MIN_BLOCKS) prim_trace_k
       if ((threadIdx.x & 31) != 0) x = 0;
     }
     if (x) atomicAdd(&P.stats->c[ST_PRIM_CAND + k], x);
+  }
+}
+
+// The handed-over queries, a warp each: the starts of a candidate's search run
+// on the lanes (the answer is the one that the loops would find). What bounds
+// it is the evaluation's chain of dependent FP32 operations; what it replaces
+// was bound by the longest query: a picture of 4,138 curved triangles ran
+// 454 ms on one thread a query.
+__global__ void __launch_bounds__(kPrimThreads) prim_heavy_kernel(PrimParams P) {
+  const int lane = threadIdx.x & 31;
+  const unsigned n = min(*P.heavy_ctr, P.heavy_cap);
+  PrimWork pw, wu;  // each lane's own, and what all lanes repeat
+  unsigned cand = 0;
+  Work w;
+  for (;;) {
+    unsigned k = 0;
+    if (lane == 0) k = atomicAdd(P.heavy_ctr + 1, 1u);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= n) break;
+    const PrimHeavy v = P.heavy[k];
+    float3 o, d;
+    float iso;
+    bool iso_on;
+    query_ray_from(P.rays, P.n_rays, P.cam, P.iso, P.iso_mask, P.views, P.n_views, v.q, o, d, iso, iso_on);
+    PrimState s = v.s;
+    bool incomplete = false;
+    const uint32_t lane0 = pw.iters, all0 = wu.iters;
+    prim_walk<true>(P, o, d, s, pw, wu, cand, w, incomplete);
+    const uint32_t its = __reduce_add_sync(0xffffffffu, pw.iters - lane0) + wu.iters - all0;
+    if (lane == 0) prim_finish(P, v.q, d, prim_base(P, v.q), s, v.iters + its, incomplete);
+    __syncwarp();
+  }
+  const unsigned long long v[4] = {lane == 0 ? cand : 0u, pw.iters + (lane == 0 ? wu.iters : 0u),
+                                   pw.flops + (lane == 0 ? wu.flops : 0ull), lane == 0 ? w.nodes : 0u};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    unsigned long long x = v[k];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    if (lane == 0 && x) atomicAdd(&P.stats->c[ST_PRIM_CAND + k], x);
   }
 }
 
@@ -224,11 +472,14 @@ void pack_prims(const HostPrims& hp, std::vector<PrimRec>& recs, int64_t counts[
 
 void prims_free(ho_context* c) {
   cudaFree(c->d_prims);
+  cudaFree(c->d_pcull);
+  cudaFree(c->d_pstart);
   cudaFree(c->d_pgeom);
   cudaFree(c->d_pfield);
   cudaFree(c->d_pbox);
   cudaFree(c->d_pnodes);
-  c->d_prims = nullptr;
+  c->d_prims = c->d_pcull = nullptr;
+  c->d_pstart = nullptr;
   c->d_pgeom = c->d_pfield = c->d_pbox = nullptr;
   c->d_pnodes = nullptr;
   c->n_prims = c->n_pnodes = 0;
@@ -257,19 +508,63 @@ int prims_build(ho_context* c) {
   prim_setup_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(static_cast<PrimRec*>(c->d_prims),
                                                                            c->d_pgeom, n, c->d_pbox);
   PR_TRY(cudaGetLastError());
+  {
+    PrimMats M;
+    std::memset(&M, 0, sizeof(M));
+    std::vector<double> B, V;
+    for (int m = 2; m <= kPrimMaxModes; ++m) {
+      // Bernstein polynomials at Chebyshev-Lobatto points, inverted
+      std::vector<double> x(m);
+      B.assign(static_cast<size_t>(m) * m, 0.0);
+      for (int r = 0; r < m; ++r) {
+        x[r] = 0.5 - 0.5 * std::cos(M_PI * r / (m - 1));
+        M.node[m][r] = static_cast<float>(-1.05 + 2.1 * x[r]);
+        double binom = 1.0;
+        for (int k = 0; k < m; ++k) {
+          if (k > 0) binom = binom * (m - k) / k;
+          B[r * m + k] = binom * std::pow(x[r], k) * std::pow(1.0 - x[r], m - 1 - k);
+        }
+      }
+      invert_dense(B, m, V);
+      for (int k = 0; k < m; ++k) {
+        double row = 0.0;
+        for (int r = 0; r < m; ++r) {
+          M.inv[m][k * kPrimMaxModes + r] = static_cast<float>(V[k * m + r]);
+          row += std::fabs(V[k * m + r]);
+        }
+        M.amp[m] = std::max(M.amp[m], static_cast<float>(row));
+      }
+    }
+    PrimMats* dm = nullptr;
+    PR_TRY(cudaMalloc(&c->d_pcull, n * sizeof(PrimCull)));
+    PR_TRY(cudaMalloc(&c->d_pstart, std::max<int64_t>(c->prim_counts[0], 1) * 21 * sizeof(float)));
+    PR_TRY(cudaMalloc(&dm, sizeof(PrimMats)));
+    cudaError_t e = cudaMemcpyAsync(dm, &M, sizeof(M), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) {
+      prim_cull_kernel<<<static_cast<unsigned>(n), 64, 0, s>>>(static_cast<const PrimRec*>(c->d_prims), c->d_pgeom, dm,
+                                                               static_cast<PrimCull*>(c->d_pcull), c->d_pstart);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaFree(dm);
+    PR_TRY(e);
+  }
   float bounds[6];
   const int rc = build_tree(c->d_pbox, nullptr, n, s, &c->d_pnodes, &c->n_pnodes, &c->pbvh_depth, bounds);
   if (rc) return rc;
   c->n_prims = n;
-  c->device_bytes += n * static_cast<int64_t>(sizeof(PrimRec) + 24 + sizeof(BNode)) +
+  c->device_bytes += n * static_cast<int64_t>(sizeof(PrimRec) + sizeof(PrimCull) + 24 + sizeof(BNode)) +
                      static_cast<int64_t>((ng + nf) * sizeof(float));
   return 0;
 }
 
-int launch_prims(ho_context* c, const TraceArgs& a, ho_hit* hits, bool fresh, DevStats* stats, cudaStream_t s) {
+int launch_prims(ho_context* c, const TraceArgs& a, ho_hit* hits, bool fresh, DevStats* stats, cudaStream_t s,
+                 bool may_allocate) {
   PrimParams P;
   P.nodes = c->d_pnodes;
   P.prims = static_cast<const PrimRec*>(c->d_prims);
+  P.cull = static_cast<const PrimCull*>(c->d_pcull);
+  P.start = c->d_pstart;
   P.geom = c->d_pgeom;
   P.field = c->d_pfield;
   P.rays = a.rays;
@@ -287,7 +582,50 @@ int launch_prims(ho_context* c, const TraceArgs& a, ho_hit* hits, bool fresh, De
   P.stats = stats ? stats : c->d_stats;
   if (P.n_queries == 0) return 0;
   const int64_t blocks = (P.n_queries + kPrimThreads - 1) / kPrimThreads;
+  P.heavy = nullptr;
+  P.heavy_cap = 0;
+  P.heavy_ctr = nullptr;
+  // The list is the context's. A call that the caller is capturing does not
+  // use it (the graph would keep its address), nor one for which there is no
+  // memory: their queries all run on one thread each. Calls on other streams
+  // wait for the list's last reader.
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  PR_TRY(cudaStreamIsCapturing(s, &cs));
+  if (may_allocate && cs == cudaStreamCaptureStatusNone) {
+    const int64_t places = std::min(P.n_queries, kPrimHeavyMost);
+    const size_t want = 16 + static_cast<size_t>(places) * sizeof(PrimHeavy);
+    if (!c->pheavy_done) PR_TRY(cudaEventCreateWithFlags(&c->pheavy_done, cudaEventDisableTiming));
+    if (want > c->pheavy_cap) {
+      cudaFree(c->d_pheavy);
+      c->d_pheavy = nullptr;
+      c->pheavy_cap = 0;
+      if (cudaMalloc(&c->d_pheavy, want) == cudaSuccess) {
+        c->pheavy_cap = want;
+      } else {
+        cudaGetLastError();
+        c->d_pheavy = nullptr;
+      }
+    }
+    if (c->d_pheavy) {
+      P.heavy_ctr = static_cast<unsigned*>(c->d_pheavy);
+      P.heavy = reinterpret_cast<PrimHeavy*>(static_cast<char*>(c->d_pheavy) + 16);
+      P.heavy_cap = static_cast<unsigned>(places);
+      PR_TRY(cudaStreamWaitEvent(s, c->pheavy_done, 0));
+      PR_TRY(cudaMemsetAsync(P.heavy_ctr, 0, 2 * sizeof(unsigned), s));
+    }
+  }
   prim_trace_kernel<<<static_cast<unsigned>(blocks), kPrimThreads, 0, s>>>(P);
+  PR_TRY(cudaGetLastError());
+  if (P.heavy) {
+    int dev = 0, sms = 0;
+    PR_TRY(cudaGetDevice(&dev));
+    PR_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t most = (P.n_queries * 32 + kPrimThreads - 1) / kPrimThreads;
+    prim_heavy_kernel<<<static_cast<unsigned>(std::min<int64_t>(most, sms * 8)), kPrimThreads, 0, s>>>(P);
+    PR_TRY(cudaGetLastError());
+    PR_TRY(cudaEventRecord(c->pheavy_done, s));
+    ++c->launches;
+  }
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -126,7 +126,7 @@ std::vector<double> gll_nodes(int n) {
   return x;
 }
 
-static bool invert_dense(std::vector<double> a, int n, std::vector<double>& inv) {
+bool invert_dense(std::vector<double> a, int n, std::vector<double>& inv) {
   inv.assign(static_cast<size_t>(n) * n, 0.0);
   for (int i = 0; i < n; ++i) inv[i * n + i] = 1.0;
   for (int c = 0; c < n; ++c) {

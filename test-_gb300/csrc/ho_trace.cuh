@@ -97,9 +97,14 @@ __device__ __forceinline__ void load_child(const BNode* __restrict__ nodes, int 
 // Collect the K smallest candidate keys > (kt, ke) with entry <= tmax from
 // the tree `nodes`. Returns false on traversal-stack overflow (status set by
 // the caller).
-template <int K>
+// keep(e): whether leaf e is a candidate at all (a leaf that the caller can
+// prove has no hit is left out, so a walk's K places go to the others).
+struct KeepAll {
+  __device__ __forceinline__ bool operator()(int) const { return true; }
+};
+template <int K, class Keep = KeepAll>
 static __device__ bool collect_in(const BNode* __restrict__ nodes, float3 o, float3 d, float tmax, float kt, int ke,
-                                  float (&bt)[K], int (&be)[K], bool& overflow, Work& w) {
+                                  float (&bt)[K], int (&be)[K], bool& overflow, Work& w, Keep keep = Keep()) {
 #pragma unroll
   for (int j = 0; j < K; ++j) {
     bt[j] = FLT_MAX;
@@ -132,6 +137,7 @@ static __device__ bool collect_in(const BNode* __restrict__ nodes, float3 o, flo
       if (id[c] < 0) {
         const int e = ~id[c];
         if (!key_less(kt, ke, a0, e)) continue;  // already visited
+        if (!keep(e)) continue;
         if (!key_less(a0, e, bt[K - 1], be[K - 1])) {
           overflow = true;
           continue;

@@ -234,6 +234,82 @@ __device__ __noinline__ void pr_modal_geom(const PrimRec& p, const float* __rest
   }
 }
 
+// pr_modal_geom at M modes in every direction, the usual case, with all loops
+// unrolled: the same operations in the same order (nothing is contracted), but
+// the basis values stay in registers, the recurrences' constants are folded
+// and independent terms overlap. The solvers are chains of these evaluations,
+// and the general form above keeps its basis values in indexed local arrays.
+template <int Kind, int M>
+__device__ __noinline__ void pr_modal_geom_m(const float* __restrict__ c, float3 x, float3& X, float3* __restrict__ tan) {
+  constexpr int tri = M * (M + 1) / 2;
+  constexpr int blk = Kind == kPrimPrism ? tri * M : (Kind == kPrimQuad ? M * M : tri);
+  float v[3] = {0.f, 0.f, 0.f}, dr[3] = {0.f, 0.f, 0.f}, ds[3] = {0.f, 0.f, 0.f}, dt[3] = {0.f, 0.f, 0.f};
+  float ar[M], dar[M], bs[M], dbs[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    ar[i] = pr_a(i, x.x);
+    dar[i] = pr_a_d(i, x.x);
+    if (Kind != kPrimTri) {
+      bs[i] = pr_a(i, x.y);
+      dbs[i] = pr_a_d(i, x.y);
+    }
+  }
+  int idx = 0;
+  if (Kind == kPrimPrism) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      float bt[M], dbt[M];
+#pragma unroll
+      for (int k = 0; k < M - i; ++k) {
+        bt[k] = pr_b(i, k, x.z);
+        dbt[k] = pr_b_d(i, k, x.z);
+      }
+#pragma unroll
+      for (int j = 0; j < M; ++j)
+#pragma unroll
+        for (int k = 0; k < M - i; ++k, ++idx)
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            const float cf = __ldg(c + a * blk + idx);
+            v[a] += cf * ar[i] * bs[j] * bt[k];
+            dr[a] += cf * dar[i] * bs[j] * bt[k];
+            ds[a] += cf * ar[i] * dbs[j] * bt[k];
+            dt[a] += cf * ar[i] * bs[j] * dbt[k];
+          }
+    }
+  } else if (Kind == kPrimQuad) {
+#pragma unroll
+    for (int j = 0; j < M; ++j)
+#pragma unroll
+      for (int i = 0; i < M; ++i, ++idx)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float cf = __ldg(c + a * blk + idx);
+          v[a] += cf * ar[i] * bs[j];
+          dr[a] += cf * dar[i] * bs[j];
+          ds[a] += cf * ar[i] * dbs[j];
+        }
+  } else {
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+#pragma unroll
+      for (int j = 0; j < M - i; ++j, ++idx) {
+        const float bj = pr_b(i, j, x.y), dbj = pr_b_d(i, j, x.y);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float cf = __ldg(c + a * blk + idx);
+          v[a] += cf * ar[i] * bj;
+          dr[a] += cf * dar[i] * bj;
+          ds[a] += cf * ar[i] * dbj;
+        }
+      }
+  }
+  X = make_float3(v[0], v[1], v[2]);
+  tan[0] = make_float3(dr[0], dr[1], dr[2]);
+  tan[1] = make_float3(ds[0], ds[1], ds[2]);
+  tan[2] = make_float3(dt[0], dt[1], dt[2]);
+}
+
 // Clamped barycentric (u, v) of a triangle's (r, s) (TriElement.cu:17-31).
 __device__ inline void pr_bary(float r, float s, float& u, float& v) {
   u = fminf(fmaxf(0.5f * (r + 1.0f), 0.0f), 1.0f);
@@ -296,10 +372,30 @@ __device__ __noinline__ void pr_linear_geom(const PrimRec& p, float3 x, float3& 
   }
 }
 
+// Modes whose evaluation is unrolled (pr_modal_geom_m).
+constexpr unsigned kPrimUnrolled = 5;
 __device__ inline void pr_geom(const PrimRec& p, const float* __restrict__ pool, float3 x, float3& X, float3* tan) {
   if (!pr_curved(p)) {
     pr_linear_geom(p, x, X, tan);
     return;
+  }
+  const unsigned m = pmode(p.gm, 0);
+  if (tan && m >= 2 && m <= kPrimUnrolled && p.gm == (m | m << 8 | (p.kind == kPrimPrism ? m << 16 : 0u))) {
+    const float* c = pool + p.goff;
+    switch (4 * p.kind + static_cast<int>(m) - 2) {
+      case 0: pr_modal_geom_m<kPrimPrism, 2>(c, x, X, tan); return;
+      case 1: pr_modal_geom_m<kPrimPrism, 3>(c, x, X, tan); return;
+      case 2: pr_modal_geom_m<kPrimPrism, 4>(c, x, X, tan); return;
+      case 3: pr_modal_geom_m<kPrimPrism, 5>(c, x, X, tan); return;
+      case 4: pr_modal_geom_m<kPrimQuad, 2>(c, x, X, tan); return;
+      case 5: pr_modal_geom_m<kPrimQuad, 3>(c, x, X, tan); return;
+      case 6: pr_modal_geom_m<kPrimQuad, 4>(c, x, X, tan); return;
+      case 7: pr_modal_geom_m<kPrimQuad, 5>(c, x, X, tan); return;
+      case 8: pr_modal_geom_m<kPrimTri, 2>(c, x, X, tan); return;
+      case 9: pr_modal_geom_m<kPrimTri, 3>(c, x, X, tan); return;
+      case 10: pr_modal_geom_m<kPrimTri, 4>(c, x, X, tan); return;
+      default: pr_modal_geom_m<kPrimTri, 5>(c, x, X, tan); return;
+    }
   }
   pr_modal_geom(p, pool, x, X, tan);
 }

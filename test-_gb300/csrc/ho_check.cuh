@@ -57,6 +57,20 @@ cudaError_t launch_residuals_n(const float* rec, const uint32_t* flags, int64_t 
   return cudaGetLastError();
 }
 
+// The k-th listed ray: the front list, then, from the next warp on, the list
+// that grows from the back.
+__device__ __forceinline__ bool listed_item(unsigned k, const uint32_t* list, unsigned n_list, const uint32_t* list_end,
+                                            unsigned n_back, unsigned& item) {
+  if (k < n_list) {
+    item = list[k];
+    return true;
+  }
+  const unsigned first = (n_list + 31u) & ~31u;
+  if (k < first || k - first >= n_back) return false;
+  item = *(list_end - (k - first));
+  return true;
+}
+
 // One thread per listed ray (the queued rays with a hit): FP64 check and
 // polish; failures are listed from the front of fail_list, rays that passed
 // with a tie partner from its back (tie_end downwards: a listed ray goes to
@@ -65,12 +79,13 @@ template <int N>
 __global__ void __launch_bounds__(128) check_kernel(TraceParams P, RayState* __restrict__ st,
                                                     const uint32_t* __restrict__ list,
                                                     const unsigned* __restrict__ n_list,
+                                                    const uint32_t* __restrict__ list_end,
+                                                    const unsigned* __restrict__ n_back,
                                                     uint32_t* __restrict__ fail_list, unsigned* __restrict__ n_fail,
                                                     uint32_t* __restrict__ tie_end, unsigned* __restrict__ n_tie) {
-  const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned item;
   bool checked = false, failed = false, polished = false;
-  if (k < *n_list) {
-    const unsigned item = list[k];
+  if (listed_item(blockIdx.x * blockDim.x + threadIdx.x, list, *n_list, list_end, *n_back, item)) {
     RayState& r = st[item];
     if (r.best.kind != HO_HIT_MISS) {
       float3 o, d;
@@ -175,10 +190,11 @@ __global__ void __launch_bounds__(kTraceBlock) fallback_kernel(TraceParams P, Ra
 template <int N>
 __global__ void __launch_bounds__(128) post_kernel(TraceParams P, RayState* __restrict__ st,
                                                    const uint32_t* __restrict__ list,
-                                                   const unsigned* __restrict__ n_list) {
-  const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= *n_list) return;
-  const unsigned item = list[k];
+                                                   const unsigned* __restrict__ n_list,
+                                                   const uint32_t* __restrict__ list_end,
+                                                   const unsigned* __restrict__ n_back) {
+  unsigned item;
+  if (!listed_item(blockIdx.x * blockDim.x + threadIdx.x, list, *n_list, list_end, *n_back, item)) return;
   HitState h = st[item].best;
   if (!(h.flags & kFlagPost)) return;
   float3 o, d;
@@ -197,8 +213,8 @@ __global__ void __launch_bounds__(128) post_kernel(TraceParams P, RayState* __re
 
 template <int N>
 cudaError_t launch_post_n(const TraceParams& P, RayState* st, const uint32_t* list, const unsigned* n_list,
-                          int64_t n_cap, cudaStream_t s) {
-  post_kernel<N><<<static_cast<unsigned>((n_cap + 127) / 128), 128, 0, s>>>(P, st, list, n_list);
+                          const uint32_t* list_end, const unsigned* n_back, int64_t n_cap, cudaStream_t s) {
+  post_kernel<N><<<static_cast<unsigned>((n_cap + 32 + 127) / 128), 128, 0, s>>>(P, st, list, n_list, list_end, n_back);
   return cudaGetLastError();
 }
 
@@ -206,32 +222,40 @@ cudaError_t launch_post_n(const TraceParams& P, RayState* st, const uint32_t* li
 // n_tie are zeroed by the caller.
 template <int N>
 cudaError_t launch_check_n(const TraceParams& P, RayState* st, const uint32_t* list, const unsigned* n_list,
-                           uint32_t* fail_list, unsigned* n_fail, unsigned* n_tie, int64_t n_cap, int sms,
+                           const uint32_t* list_end, const unsigned* n_back, uint32_t* fail_list, unsigned* n_fail, unsigned* n_tie, int64_t n_cap, int sms,
                            cudaStream_t s) {
   uint32_t* tie_end = fail_list + (n_cap - 1);
-  check_kernel<N><<<static_cast<unsigned>((n_cap + 127) / 128), 128, 0, s>>>(P, st, list, n_list, fail_list, n_fail,
-                                                                              tie_end, n_tie);
+  check_kernel<N><<<static_cast<unsigned>((n_cap + 32 + 127) / 128), 128, 0, s>>>(
+      P, st, list, n_list, list_end, n_back, fail_list, n_fail, tie_end, n_tie);
   tie_kernel<N><<<sms * 2, 128, 0, s>>>(P, st, tie_end, n_tie);
   fallback_kernel<N><<<sms * 2, kTraceBlock, 0, s>>>(P, st, fail_list, n_fail);
   return cudaGetLastError();
 }
 
 extern template cudaError_t launch_check_n<2>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<4>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<5>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<6>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<7>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<8>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 extern template cudaError_t launch_check_n<9>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              uint32_t*, unsigned*, unsigned*, int64_t, int, cudaStream_t);
+                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
+                                              int64_t, int, cudaStream_t);
 
 extern template cudaError_t launch_residuals_n<2>(const float*, const uint32_t*, int64_t, const float*, const ho_hit*,
                                                   double*, cudaStream_t);
@@ -250,21 +274,21 @@ extern template cudaError_t launch_residuals_n<8>(const float*, const uint32_t*,
 extern template cudaError_t launch_residuals_n<9>(const float*, const uint32_t*, int64_t, const float*, const ho_hit*,
                                                   double*, cudaStream_t);
 
-extern template cudaError_t launch_post_n<2>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<4>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<5>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<6>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<7>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<8>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
-extern template cudaError_t launch_post_n<9>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, int64_t,
-                                             cudaStream_t);
+extern template cudaError_t launch_post_n<2>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<4>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<5>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<6>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<7>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<8>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<9>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
+                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
 
 }  // namespace ho

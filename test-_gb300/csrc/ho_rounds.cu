@@ -247,12 +247,31 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
 // Queued rays listed by a predicate (warp-aggregated appends): hits = false,
 // the rays still in flight after the main rounds (for the tail kernel; the
 // count goes to the work counters too); hits = true, the rays with a hit
-// (for the FP64 check).
+// (for the FP64 check): from the front of the list those that its shorter path
+// answers, face hits away from the face's edges, from the back the others, so
+// that a warp of the check mostly runs one path (a 1920 x 1080 picture of 3
+// isovalues, 1.54 M hits: check 4.2 -> 1.9 ms, tie pass 0.51 -> 0.43 ms).
 __global__ void ray_list_kernel(const unsigned* __restrict__ qcount, const RayState* __restrict__ st, bool hits,
-                                uint32_t* __restrict__ list, unsigned* __restrict__ n_list, DevStats* stats) {
+                                uint32_t* __restrict__ list, unsigned* __restrict__ n_list,
+                                uint32_t* __restrict__ list_end, unsigned* __restrict__ n_back, DevStats* stats) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool live = false;
-  if (i < *qcount) live = hits ? st[i].best.kind != HO_HIT_MISS : !st[i].done;
+  bool live = false, back = false;
+  if (i < *qcount) {
+    live = hits ? st[i].best.kind != HO_HIT_MISS : !st[i].done;
+    if (hits && live) {
+      const HitState& b = st[i].best;
+      back = b.kind != HO_HIT_FACE || !normal_on_face(b.face, b.xi);
+      live = !back;
+    }
+  }
+  const unsigned mb = __ballot_sync(kFull, back);
+  if (mb) {
+    const int lane = threadIdx.x & 31, leader = __ffs(mb) - 1;
+    unsigned base = 0;
+    if (lane == leader) base = atomicAdd(n_back, static_cast<unsigned>(__popc(mb)));
+    base = __shfl_sync(kFull, base, leader);
+    if (back) *(list_end - (base + __popc(mb & ((1u << lane) - 1u)))) = i;
+  }
   const unsigned m = __ballot_sync(kFull, live);
   if (!m) return;
   const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
@@ -281,7 +300,8 @@ __global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const 
 }
 
 // Ctr layout: [0] pairs of the round, [3] failed FP64 checks, [4..5] the
-// tail's list count and cursor, [6..7] the check's list count and tie count,
+// tail's list count and cursor, [6..8] the check's front count, tie count and
+// back count,
 // and per order n (2..9) the batch count, region start, write cursor of the
 // face batches, take cursor, and count and write cursor of the isosurface
 // batches, which come first in the region.
@@ -446,23 +466,25 @@ static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams&
   uint32_t* list = reinterpret_cast<uint32_t*>(c->rounds.pkey);
   unsigned* n_list = c->rounds.ctr + 6;
   unsigned* n_tie = c->rounds.ctr + 7;
+  unsigned* n_back = c->rounds.ctr + 8;
+  uint32_t* list_end = list + (n_cap - 1);
   RT_TRY(cudaMemsetAsync(c->rounds.ctr + 3, 0, sizeof(unsigned), s));
-  RT_TRY(cudaMemsetAsync(n_list, 0, 2 * sizeof(unsigned), s));
+  RT_TRY(cudaMemsetAsync(n_list, 0, 3 * sizeof(unsigned), s));
   ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, R.state, true, list, n_list,
-                                                                             P.stats);
+                                                                             list_end, n_back, P.stats);
   RT_TRY(cudaGetLastError());
   if (!c->fp64_check) {
     c->launches += 2;  // ray list, post
     cudaError_t e;
     switch (c->N) {
-      case 2: e = launch_post_n<2>(P, R.state, list, n_list, n_cap, s); break;
-      case 3: e = launch_post_n<3>(P, R.state, list, n_list, n_cap, s); break;
-      case 4: e = launch_post_n<4>(P, R.state, list, n_list, n_cap, s); break;
-      case 5: e = launch_post_n<5>(P, R.state, list, n_list, n_cap, s); break;
-      case 6: e = launch_post_n<6>(P, R.state, list, n_list, n_cap, s); break;
-      case 7: e = launch_post_n<7>(P, R.state, list, n_list, n_cap, s); break;
-      case 8: e = launch_post_n<8>(P, R.state, list, n_list, n_cap, s); break;
-      case 9: e = launch_post_n<9>(P, R.state, list, n_list, n_cap, s); break;
+      case 2: e = launch_post_n<2>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 3: e = launch_post_n<3>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 4: e = launch_post_n<4>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 5: e = launch_post_n<5>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 6: e = launch_post_n<6>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 7: e = launch_post_n<7>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 8: e = launch_post_n<8>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 9: e = launch_post_n<9>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
       default: e = cudaErrorInvalidValue; break;
     }
     return int(e);
@@ -474,28 +496,28 @@ static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams&
   cudaError_t e;
   switch (c->N) {
     case 2:
-      e = launch_check_n<2>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<2>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 3:
-      e = launch_check_n<3>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<3>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 4:
-      e = launch_check_n<4>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<4>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 5:
-      e = launch_check_n<5>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<5>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 6:
-      e = launch_check_n<6>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<6>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 7:
-      e = launch_check_n<7>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<7>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 8:
-      e = launch_check_n<8>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<8>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     case 9:
-      e = launch_check_n<9>(P, R.state, list, n_list, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
+      e = launch_check_n<9>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
       break;
     default: e = cudaErrorInvalidValue; break;
   }
@@ -642,7 +664,7 @@ static int enqueue_tail(ho_context* c, const TraceParams& P, const RoundParams& 
   round_gather_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(
       P, R.state, static_cast<RoundPair*>(rb.pairs), rb.pkey, rb.prank, rb.kcount, rb.ctr, 0, true);
   ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, R.state, false, rb.fail,
-                                                                             n_list, P.stats);
+                                                                             n_list, nullptr, nullptr, P.stats);
   RT_TRY(cudaGetLastError());
   cudaError_t e;
   switch (c->N) {

@@ -437,13 +437,27 @@ struct Sample {
 // Jacobian once more at the converged point (sample_along with AH = false);
 // the round kernel and the warp-per-ray kernel both use this form, with the
 // same arithmetic, so they give the same answers.
-template <int N, bool SM>
+// U: all 32 lanes call it with the same arguments, so each evaluates one
+// component (the lane's number modulo 4) and takes the others by shuffles
+// (the tail of 12 views of mixed orders 13.3 -> 10.8 ms).
+template <int N, bool SM, bool U = false>
 __device__ __forceinline__ bool sample_ahead(const Elem<N, SM>& e, float3 o, float3 d, float t, float iso, Sample& s,
                                              Work& w, float3 xi0, int max_it) {
   float3 xi = xi0;
   for (int it = 1;; ++it) {
     float4 r[4];
-    eval_comps<N, SM>(e.c, xi, 0, 4, r);
+    if constexpr (U) {
+      const int comp = threadIdx.x & 3;
+      float4 own[4];
+      eval_comps<N, SM>(e.c, xi, comp, comp + 1, own);
+      const float4 v = own[comp];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        r[k] = make_float4(__shfl_sync(0xffffffffu, v.x, k), __shfl_sync(0xffffffffu, v.y, k),
+                           __shfl_sync(0xffffffffu, v.z, k), __shfl_sync(0xffffffffu, v.w, k));
+    } else {
+      eval_comps<N, SM>(e.c, xi, 0, 4, r);
+    }
     w.flops += eval_flops(N, 4);
     ++w.geom;
     ++w.field;
@@ -475,10 +489,10 @@ __device__ __forceinline__ bool sample_ahead(const Elem<N, SM>& e, float3 o, flo
   }
 }
 
-template <int N, bool SM, bool AH = false>
+template <int N, bool SM, bool AH = false, bool U = false>
 __device__ __forceinline__ bool sample_along(const Elem<N, SM>& e, float3 o, float3 d, float t, float iso, Sample& s,
                                              Work& w, float3 xi0 = make_float3(0.f, 0.f, 0.f), int max_it = 50) {
-  if constexpr (AH) return sample_ahead<N, SM>(e, o, d, t, iso, s, w, xi0, max_it);
+  if constexpr (AH) return sample_ahead<N, SM, U>(e, o, d, t, iso, s, w, xi0, max_it);
   const float3 p = make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
   if (!inverse_map<N>(e, p, s.xi, w, xi0, max_it)) return false;
   float u;
@@ -499,17 +513,17 @@ __device__ __forceinline__ bool sample_along(const Elem<N, SM>& e, float3 o, flo
 // if that does not converge the plain cold-start solve answers (the fallback
 // the learned guess never replaces).
 constexpr int kWarmCap = 4;
-template <int N, bool SM, bool AH = false>
+template <int N, bool SM, bool AH = false, bool U = false>
 __device__ __forceinline__ bool sample_warm(const Elem<N, SM>& e, float3 o, float3 d, float t, float iso, Sample& s,
                                             Work& w, bool warm, float3 xi0) {
   if (warm) {
-    if (sample_along<N, SM, AH>(e, o, d, t, iso, s, w, xi0, kWarmCap)) {
+    if (sample_along<N, SM, AH, U>(e, o, d, t, iso, s, w, xi0, kWarmCap)) {
       ++w.accepted;
       return true;
     }
     ++w.rejected;
   }
-  return sample_along<N, SM, AH>(e, o, d, t, iso, s, w);
+  return sample_along<N, SM, AH, U>(e, o, d, t, iso, s, w);
 }
 
 __device__ __forceinline__ float3 lerp3(float3 a, float3 b, float u) {
@@ -519,21 +533,21 @@ __device__ __forceinline__ float3 lerp3(float3 a, float3 b, float u) {
 // At most 20 safeguarded Newton/bisection steps on a bracket [lt, rt] whose
 // left sample is ls; done when |f| < 1e-5, else the midpoint with the left
 // sample's xi and gradient (RayIsosurface.cu:121-177).
-template <int N, bool SM, bool AH = false>
+template <int N, bool SM, bool AH = false, bool U = false>
 __device__ __forceinline__ bool refine_bracket(const Elem<N, SM>& e, float3 o, float3 d, float iso, float lt, float rt,
                                                Sample ls, float& th, float3& xh, float3& gh, Work& w,
                                                bool warm = false, float3 rxi = make_float3(0.f, 0.f, 0.f)) {
   for (int it = 0; it < 20; ++it) {
     const float mt = 0.5f * (lt + rt);
     Sample ms;
-    if (!sample_warm<N, SM, AH>(e, o, d, mt, iso, ms, w, warm, lerp3(ls.xi, rxi, 0.5f))) return false;
+    if (!sample_warm<N, SM, AH, U>(e, o, d, mt, iso, ms, w, warm, lerp3(ls.xi, rxi, 0.5f))) return false;
     float ct = mt;
     if (fabsf(ms.df) > 1e-8f) {
       const float nt = mt - ms.f / ms.df;
       if (nt > lt && nt < rt) ct = nt;
     }
     Sample cs;
-    if (!sample_warm<N, SM, AH>(e, o, d, ct, iso, cs, w, warm, ms.xi)) {
+    if (!sample_warm<N, SM, AH, U>(e, o, d, ct, iso, cs, w, warm, ms.xi)) {
       ct = mt;  // keep the failed solve's xi, as the reference does
       cs.f = ms.f;
       cs.g = ms.g;
@@ -673,7 +687,7 @@ __device__ bool find_iso_warp(const Elem<N, SM>& e, float3 o, float3 d, float t0
   ls.g = shfl3(s.g, li);
   const float3 rxi = shfl3(s.xi, ri);
   const long long c1 = clock64();
-  const bool found = refine_bracket<N, SM, true>(e, o, d, iso, lt, rt, ls, th, xh, gh, wu, L && pr.on, rxi);
+  const bool found = refine_bracket<N, SM, true, true>(e, o, d, iso, lt, rt, ls, th, xh, gh, wu, L && pr.on, rxi);
   wu.cyc[2] += clock64() - c1;
   return found;
 }
@@ -793,7 +807,7 @@ __device__ __forceinline__ void setc(float3& v, int a, float s) {
 }
 
 // Point and the two tangents of face f (face_param's free axes ua < va) at
-// its free coordinates (u, v), components 0 to comps - 1 (x, y, z, the field):
+// its free coordinates (u, v), components [c0, c1) (0-2: x, y, z, 3: the field):
 // out[c] = {x_c, dx_c/du, dx_c/dv, 0}.
 //
 // On a face the fixed coordinate is exactly -1 or 1, where one vertex mode is
@@ -805,7 +819,8 @@ __device__ __forceinline__ void setc(float3& v, int a, float s) {
 // multiply-adds. The face solves are most of the round kernel's steps; their
 // evaluations' cost was 2 (2N^3 + 3N^2) operations a component.
 template <int N, bool SM>
-__device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, int comps, float4* __restrict__ out) {
+__device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, int c0, int c1,
+                                       float4* __restrict__ out) {
   constexpr int RS = row_stride(N);
   int fixed, ua, va;
   float val;
@@ -817,7 +832,7 @@ __device__ __noinline__ void face_eval(CoefRef<SM> c, int f, float u, float v, i
   basis_val_der<N>(u, pu, du);
   basis_val_der<N>(v, pv, dv);
 #pragma unroll 1
-  for (int comp = 0; comp < comps; ++comp) {
+  for (int comp = c0; comp < c1; ++comp) {
     const CoefRef<SM> cc = c.at(comp * block_floats(N) + m * sf);
     float x = 0.f, xu = 0.f, xv = 0.f;
 #pragma unroll 1

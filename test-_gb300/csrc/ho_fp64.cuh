@@ -369,7 +369,7 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
       float val;
       face_param(h.face, fixed, val, ua, va);
       float4 fr[4];
-      face_eval<N, false>(c, h.face, getc(xi, ua), getc(xi, va), has_field ? 4 : 3, fr);
+      face_eval<N, false>(c, h.face, getc(xi, ua), getc(xi, va), 0, has_field ? 4 : 3, fr);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         J[3 * k] = ua == 0 ? fr[k].y : 0.f;

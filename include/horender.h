@@ -375,10 +375,14 @@ int ho_set_mode(ho_context* ctx, int mode);
  *                     in t is weighed against it by the FP64 tie rule
  *                     (HO_FLAG_TIE, ho_stats.fp64_ties). 0: off (the
  *                     solvers' own answers).
- * HO_OPT_ROUND_CHUNK  pairs per element batch of the round kernel (1..4096;
- *                     default: the kernel's pair slots, 20 per warp up to 7
- *                     modes per direction, 12 at 8, 8 at 9, times 4 warps in
- *                     the tensor-core form); ho_autotune picks it.
+ * HO_OPT_ROUND_CHUNK  pairs per element batch of the round kernel (1..4096).
+ *                     Unset: at most the kernel's pair slots (20 per warp up
+ *                     to 7 modes per direction, 12 at 8, 8 at 9, times 4 warps
+ *                     in the tensor-core form: the value that ho_get_option
+ *                     gives; 32 for face searches on elements with a
+ *                     convergence certificate), fewer while a round has too
+ *                     few pairs to give 16 warps of every SM a batch;
+ *                     ho_autotune picks a fixed one.
  * HO_OPT_TENSOR      0 (default): the FP32 CUDA-core round kernel for every
  *                     order; 1: elements of up to 8 modes per direction are
  *                     intersected by the tensor-core round kernel (tcgen05

@@ -308,9 +308,21 @@ __global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const 
 constexpr int kCtrOrderNb = 16, kCtrOrderOff = 26, kCtrOrderCur = 36, kCtrOrderNext = 46, kCtrIsoNb = 56,
               kCtrIsoCur = 66, kCtrWords = 80;
 
-// Pairs per batch of a key (HO_OPT_ROUND_CHUNK, else the slots).
-__device__ __forceinline__ int batch_size(int chunk, int order, bool tc, bool faces) {
-  return chunk > 0 ? chunk : (faces ? face_slots(order) : round_batch_default(order, tc));
+// Batches per SM that a round's pairs are spread over, before batches grow.
+constexpr unsigned kSpreadPerSm = 16;
+// Pairs per batch of a key: HO_OPT_ROUND_CHUNK, else the slots, or fewer while
+// the round has less than `spread` full batches (16 warps an SM). A warp's lanes
+// are fed by a batch's pairs, so a full batch keeps them busiest; but a round
+// that cannot fill the device lasts as long as its longest batch, and a batch of
+// one or two pairs, with the warp to itself, is several times shorter. Calls
+// before (full batches only) and after: 1,024 rays 1.81 -> 1.18 ms, a 320 x 180
+// picture 3.5 -> 2.5 ms, four path bounces 14.4 -> 12.7 ms; 4 or more batches a
+// resident warp change nothing (1920 x 1080: 15.3 ms either way); 64 an SM:
+// 2.6 ms and 13.0 ms for the second and third.
+__device__ __forceinline__ int batch_size(int chunk, int order, bool tc, bool faces, unsigned pairs, unsigned spread) {
+  if (chunk > 0) return chunk;
+  const int most = faces ? face_slots(order) : round_batch_default(order, tc);
+  return tc ? most : max(1, min(most, static_cast<int>((pairs + spread - 1) / spread)));
 }
 // Does a key's batch take the face layout?
 __device__ __forceinline__ bool face_batch(int64_t key, bool tc, const float* __restrict__ cull) {
@@ -324,13 +336,13 @@ __device__ __forceinline__ bool face_batch(int64_t key, bool tc, const float* __
 // isosurface batches, the longer ones, come first.
 __global__ void round_batch_count_kernel(const uint32_t* __restrict__ kcount, const uint8_t* __restrict__ order,
                                          const float* __restrict__ cull, int64_t n_elem, int chunk, bool tc,
-                                         unsigned* __restrict__ ctr) {
+                                         unsigned spread, unsigned* __restrict__ ctr) {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= 2 * n_elem) return;
   const int c = static_cast<int>(kcount[k]);
   if (c == 0) return;
   const int n = order[k >> 1];
-  const int B = batch_size(chunk, n, tc, face_batch(k, tc, cull));
+  const int B = batch_size(chunk, n, tc, face_batch(k, tc, cull), ctr[0], spread);
   const unsigned nb = static_cast<unsigned>((c + B - 1) / B);
   atomicAdd(&ctr[kCtrOrderNb + n], nb);
   if (k & 1) atomicAdd(&ctr[kCtrIsoNb + n], nb);
@@ -351,14 +363,15 @@ __global__ void round_order_offsets_kernel(unsigned* __restrict__ ctr) {
 // Each key's pairs in batches, written into its order's region.
 __global__ void round_batch_kernel(const uint32_t* __restrict__ kcount, const uint32_t* __restrict__ koff,
                                    const uint8_t* __restrict__ order, const float* __restrict__ cull, int64_t n_elem,
-                                   int chunk, bool tc, RoundBatch* __restrict__ batches, unsigned* __restrict__ ctr) {
+                                   int chunk, bool tc, unsigned spread, RoundBatch* __restrict__ batches,
+                                   unsigned* __restrict__ ctr) {
   const int64_t key = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (key >= 2 * n_elem) return;
   const int c = static_cast<int>(kcount[key]);
   if (c == 0) return;
   const int n = order[key >> 1];
   const bool faces = face_batch(key, tc, cull);
-  const int B = batch_size(chunk, n, tc, faces);
+  const int B = batch_size(chunk, n, tc, faces, ctr[0], spread);
   const int nb = (c + B - 1) / B;
   const unsigned base = ctr[kCtrOrderOff + n] + atomicAdd(&ctr[(key & 1 ? kCtrIsoCur : kCtrOrderCur) + n],
                                                           static_cast<unsigned>(nb));
@@ -605,9 +618,13 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   round_scatter_kernel<<<gi, 256, 0, s>>>(gathered, rb.pkey, rb.prank, rb.koff, rb.ctr,
                                           const_cast<RoundPair*>(R.pairs), P.stats);
   const unsigned ge = static_cast<unsigned>((n_keys + 255) / 256);
-  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, rb.ctr);
+  int dev = 0, sms = 0;
+  RT_TRY(cudaGetDevice(&dev));
+  RT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const unsigned spread = kSpreadPerSm * static_cast<unsigned>(sms);
+  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread, rb.ctr);
   round_order_offsets_kernel<<<1, 1, 0, s>>>(rb.ctr);
-  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc,
+  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread,
                                         const_cast<RoundBatch*>(R.batches), rb.ctr);
   RT_TRY(cudaGetLastError());
   c->launches += 7 + __builtin_popcount(c->orders);

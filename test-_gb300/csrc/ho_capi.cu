@@ -234,6 +234,7 @@ void ho_destroy(ho_context* c) {
     cudaFree(c->d_rgb);
     cudaFree(c->d_rays);
     cudaFree(c->d_views);
+    cudaFree(c->d_batch);
     cudaFree(c->d_work);
     cudaFree(c->d_kbuf);
     cudaFree(c->d_kovf);
@@ -1123,14 +1124,14 @@ int upload_params(ho_context* c, const float* flat) {
   return HO_OK;
 }
 
-int download_params(ho_context* c, float* flat, bool grads) {
+int download_params(ho_context* c, float* flat) {
   std::vector<std::vector<float>> W(4), b(4);
   for (int l = 0; l < 4; ++l) {
     W[l].resize(static_cast<size_t>(kLayerInPad[l]) * kLayerOut[l]);
     b[l].resize(kLayerOut[l]);
-    CK(cudaMemcpyAsync(W[l].data(), grads ? c->mlp.gW[l] : c->mlp.W[l], W[l].size() * sizeof(float),
+    CK(cudaMemcpyAsync(W[l].data(), c->mlp.W[l], W[l].size() * sizeof(float),
                        cudaMemcpyDeviceToHost, c->stream), "read parameters");
-    CK(cudaMemcpyAsync(b[l].data(), grads ? c->mlp.gb[l] : c->mlp.b[l], b[l].size() * sizeof(float),
+    CK(cudaMemcpyAsync(b[l].data(), c->mlp.b[l], b[l].size() * sizeof(float),
                        cudaMemcpyDeviceToHost, c->stream), "read parameters");
   }
   CK(cudaStreamSynchronize(c->stream), "sync");
@@ -1178,7 +1179,7 @@ int ho_mlp_set_params(ho_context* c, const float* params) {
 int ho_mlp_get_params(ho_context* c, float* params) {
   if (!c || !params) return HO_ERR_ARG;
   if (!c->mlp.ready) return fail(c, HO_ERR_STATE, "no network");
-  return download_params(c, params, false);
+  return download_params(c, params);
 }
 
 int ho_mlp_forward(ho_context* c, const float* X, int64_t n, float* Y) {
@@ -1206,30 +1207,22 @@ int ho_mlp_grad(ho_context* c, const float* X, const float* T, const uint8_t* va
                 float* grads) {
   if (!c || !X || !T || !valid || n <= 0 || !loss || !grads) return HO_ERR_ARG;
   if (!c->mlp.ready) return fail(c, HO_ERR_STATE, "no network");
-  std::vector<uint16_t> xb;
-  to_bf16_rows(X, n, xb);
-  void* dx = nullptr;
-  float *dt = nullptr, *dl = nullptr;
-  uint8_t* dv = nullptr;
-  CK(cudaMalloc(&dx, xb.size() * 2), "cudaMalloc");
-  CK(cudaMalloc(&dt, static_cast<size_t>(n) * ho::kMlpOut * sizeof(float)), "cudaMalloc");
-  CK(cudaMalloc(&dv, n), "cudaMalloc");
-  CK(cudaMalloc(&dl, sizeof(float)), "cudaMalloc");
-  CK(cudaMemcpyAsync(dx, xb.data(), xb.size() * 2, cudaMemcpyHostToDevice, c->stream), "upload");
-  CK(cudaMemcpyAsync(dt, T, static_cast<size_t>(n) * ho::kMlpOut * sizeof(float), cudaMemcpyHostToDevice, c->stream),
-     "upload");
+  const size_t nx = static_cast<size_t>(n) * ho::kMlpIn, nt = static_cast<size_t>(n) * ho::kMlpOut;
+  int rc = ensure_buf(c, c->d_batch, c->batch_cap, (nx + nt) * sizeof(float) + n, "cudaMalloc(batch)");
+  if (rc) return rc;
+  float *dx = reinterpret_cast<float*>(c->d_batch), *dt = dx + nx;
+  uint8_t* dv = reinterpret_cast<uint8_t*>(dt + nt);
+  CK(cudaMemcpyAsync(dx, X, nx * sizeof(float), cudaMemcpyHostToDevice, c->stream), "upload");
+  CK(cudaMemcpyAsync(dt, T, nt * sizeof(float), cudaMemcpyHostToDevice, c->stream), "upload");
   CK(cudaMemcpyAsync(dv, valid, n, cudaMemcpyHostToDevice, c->stream), "upload");
   int nv = 0;
   for (int i = 0; i < n; ++i) nv += valid[i] ? 1 : 0;
-  const int rc = c->mlp.forward_backward(n, dx, dt, dv, nv, dl, c->stream);
+  rc = c->mlp.forward_backward(n, dx, nullptr, dt, dv, nv, c->stream);
   if (rc) return cuda_fail(c, rc, "network backward");
-  CK(cudaMemcpyAsync(loss, dl, sizeof(float), cudaMemcpyDeviceToHost, c->stream), "read");
-  const int r2 = download_params(c, grads, true);
-  cudaFree(dx);
-  cudaFree(dt);
-  cudaFree(dv);
-  cudaFree(dl);
-  return r2;
+  CK(cudaMemcpyAsync(grads, c->mlp.grads, ho::kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream), "read");
+  CK(cudaMemcpyAsync(loss, c->mlp.grads + ho::kMlpParams, sizeof(float), cudaMemcpyDeviceToHost, c->stream), "read");
+  CK(cudaStreamSynchronize(c->stream), "sync");
+  return HO_OK;
 }
 
 int ho_learn_samples(ho_context* c, int64_t n, uint64_t seed, float* X, float* T, uint8_t* valid) {
@@ -1293,7 +1286,7 @@ int ho_mlp_save(ho_context* c, const char* path) {
   if (!c || !path) return HO_ERR_ARG;
   if (!c->mlp.ready) return fail(c, HO_ERR_STATE, "no network");
   std::vector<float> flat(ho::kMlpParams);
-  int rc = download_params(c, flat.data(), false);
+  int rc = download_params(c, flat.data());
   if (rc) return rc;
   std::vector<uint16_t> hb(flat.size());
   for (size_t i = 0; i < flat.size(); ++i) {

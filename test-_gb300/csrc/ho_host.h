@@ -211,6 +211,8 @@ struct ho_context {
   size_t rays_cap = 0;
   uint8_t* d_views = nullptr;     // view table of a multi-view call
   size_t views_cap = 0;
+  uint8_t* d_batch = nullptr;     // rows, targets and masks of a gradient call
+  size_t batch_cap = 0;
   // learned mode
   ho::Mlp mlp;
   float* d_desc = nullptr;        // n_elem * 48 element descriptors

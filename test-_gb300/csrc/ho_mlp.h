@@ -32,6 +32,8 @@ struct Mlp {
   // per layer l: W[l] is [in][out] row-major FP32 master; Wb BF16 copy
   float* W[4] = {nullptr, nullptr, nullptr, nullptr};
   void* Wb[4] = {nullptr, nullptr, nullptr, nullptr};
+  // gradients in the flat parameter order (layer 0: 48 rows), then the batch loss
+  float* grads = nullptr;
   float* gW[4] = {nullptr, nullptr, nullptr, nullptr};
   float* mW[4] = {nullptr, nullptr, nullptr, nullptr};
   float* vW[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -53,12 +55,11 @@ struct Mlp {
   int refresh_copies(cudaStream_t s);
   MlpDev dev() const;
   int ensure_ws(int rows);
-  int forward_backward(int B, const void* Xb, const float* Tb, const uint8_t* Vb, int n_valid, float* loss_dev,
+  int forward_backward(int B, const float* Xf, const void* Xb, const float* Tb, const uint8_t* Vb, int n_valid,
                        cudaStream_t s);
   int adam_step(float lr, cudaStream_t s);
   int train(const void* X, const float* T, const uint8_t* V, int64_t n, int steps, int batch, float lr, uint64_t seed,
             std::vector<float>& losses, cudaStream_t s);
-  // pointers into the workspace after forward_backward (for gradient checks)
 };
 
 size_t mlp_infer_smem();

@@ -258,6 +258,12 @@ void ho_destroy(ho_context* c) {
       if (c->order_done[n]) cudaEventDestroy(c->order_done[n]);
     }
     if (c->order_fork) cudaEventDestroy(c->order_fork);
+    if (c->check_stream) {
+      cudaStreamSynchronize(c->check_stream);
+      cudaStreamDestroy(c->check_stream);
+    }
+    if (c->check_fork) cudaEventDestroy(c->check_fork);
+    if (c->check_done) cudaEventDestroy(c->check_done);
     for (cudaEvent_t ev : c->round_events) cudaEventDestroy(ev);
     cudaFree(c->d_pred);
     cudaFree(c->d_cand);

@@ -57,58 +57,69 @@ cudaError_t launch_residuals_n(const float* rec, const uint32_t* flags, int64_t 
   return cudaGetLastError();
 }
 
-// The k-th listed ray: the front list, then, from the next warp on, the list
-// that grows from the back.
-__device__ __forceinline__ bool listed_item(unsigned k, const uint32_t* list, unsigned n_list, const uint32_t* list_end,
-                                            unsigned n_back, unsigned& item) {
-  if (k < n_list) {
-    item = list[k];
+// The rays that one set of check launches works on, and its scratch: the list
+// from the front and from the back (ray_list_kernel), the failures from the
+// front of fail and the rays with a tie partner from its back. Every array has
+// cap entries, cap >= the listed rays.
+struct CheckLists {
+  uint32_t* list;
+  uint32_t* fail;
+  unsigned *n_front, *n_back, *n_fail, *n_tie;  // zeroed by the caller
+  int64_t cap;
+};
+
+// The listed rays as one sequence: the front list, then, from the next warp on,
+// the list that grows from the back. Its length, and whether place k holds one.
+__device__ __forceinline__ unsigned listed_end(const CheckLists& L) { return ((*L.n_front + 31u) & ~31u) + *L.n_back; }
+__device__ __forceinline__ bool listed_item(const CheckLists& L, unsigned k, unsigned& item) {
+  const unsigned n = *L.n_front;
+  if (k < n) {
+    item = L.list[k];
     return true;
   }
-  const unsigned first = (n_list + 31u) & ~31u;
-  if (k < first || k - first >= n_back) return false;
-  item = *(list_end - (k - first));
+  const unsigned first = (n + 31u) & ~31u;
+  if (k < first || k - first >= *L.n_back) return false;
+  item = L.list[L.cap - 1 - (k - first)];
   return true;
 }
 
-// One thread per listed ray (the queued rays with a hit): FP64 check and
-// polish; failures are listed from the front of fail_list, rays that passed
-// with a tie partner from its back (tie_end downwards: a listed ray goes to
-// at most one of the two lists, so they do not meet).
+// One thread per listed ray (rays with a hit; grid-stride): FP64 check and
+// polish; failures and rays that passed with a tie partner are listed (a ray
+// goes to at most one of the two lists, so they do not meet).
 template <int N>
-__global__ void __launch_bounds__(128) check_kernel(TraceParams P, RayState* __restrict__ st,
-                                                    const uint32_t* __restrict__ list,
-                                                    const unsigned* __restrict__ n_list,
-                                                    const uint32_t* __restrict__ list_end,
-                                                    const unsigned* __restrict__ n_back,
-                                                    uint32_t* __restrict__ fail_list, unsigned* __restrict__ n_fail,
-                                                    uint32_t* __restrict__ tie_end, unsigned* __restrict__ n_tie) {
-  unsigned item;
-  bool checked = false, failed = false, polished = false;
-  if (listed_item(blockIdx.x * blockDim.x + threadIdx.x, list, *n_list, list_end, *n_back, item)) {
-    RayState& r = st[item];
-    if (r.best.kind != HO_HIT_MISS) {
-      float3 o, d;
-      float iso;
-      bool iso_on;
-      query_ray(P, P.work[item], o, d, iso, iso_on);
-      checked = true;
-      HitState h = r.best;
-      failed = !fp64_check_polish<N>(P.rec, P.flags, o, d, iso, h, polished);
-      if (failed) {
-        fail_list[atomicAdd(n_fail, 1u)] = item;
-      } else {
-        r.best = h;
-        if (r.tie.kind != HO_HIT_MISS) *(tie_end - atomicAdd(n_tie, 1u)) = item;
+__global__ void __launch_bounds__(128) check_kernel(TraceParams P, RayState* __restrict__ st, CheckLists L) {
+  const unsigned end = listed_end(L);
+  unsigned n_checked = 0, n_failed = 0, n_polished = 0;
+  for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; (k & ~31ull) < end;
+       k += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    unsigned item;
+    bool checked = false, failed = false, polished = false;
+    if (listed_item(L, static_cast<unsigned>(k), item)) {
+      RayState& r = st[item];
+      if (r.best.kind != HO_HIT_MISS) {
+        float3 o, d;
+        float iso;
+        bool iso_on;
+        query_ray(P, P.work[item], o, d, iso, iso_on);
+        checked = true;
+        HitState h = r.best;
+        failed = !fp64_check_polish<N>(P.rec, P.flags, o, d, iso, h, polished);
+        if (failed) {
+          L.fail[atomicAdd(L.n_fail, 1u)] = item;
+        } else {
+          r.best = h;
+          if (r.tie.kind != HO_HIT_MISS) L.fail[L.cap - 1 - atomicAdd(L.n_tie, 1u)] = item;
+        }
       }
     }
+    n_checked += __popc(__ballot_sync(0xffffffffu, checked));
+    n_failed += __popc(__ballot_sync(0xffffffffu, failed));
+    n_polished += __popc(__ballot_sync(0xffffffffu, polished));
   }
-  const unsigned cm = __ballot_sync(0xffffffffu, checked), fm = __ballot_sync(0xffffffffu, failed),
-                 pm = __ballot_sync(0xffffffffu, polished);
   if ((threadIdx.x & 31) == 0) {
-    if (cm) atomicAdd(&P.stats->c[ST_CHECKED], static_cast<unsigned long long>(__popc(cm)));
-    if (fm) atomicAdd(&P.stats->c[ST_CHECK_FAIL], static_cast<unsigned long long>(__popc(fm)));
-    if (pm) atomicAdd(&P.stats->c[ST_POLISHED], static_cast<unsigned long long>(__popc(pm)));
+    if (n_checked) atomicAdd(&P.stats->c[ST_CHECKED], static_cast<unsigned long long>(n_checked));
+    if (n_failed) atomicAdd(&P.stats->c[ST_CHECK_FAIL], static_cast<unsigned long long>(n_failed));
+    if (n_polished) atomicAdd(&P.stats->c[ST_POLISHED], static_cast<unsigned long long>(n_polished));
   }
 }
 
@@ -118,13 +129,11 @@ __global__ void __launch_bounds__(128) check_kernel(TraceParams P, RayState* __r
 // serialise the check's warps. The best hit is polished already; its exact
 // root t is taken again by the same polish (one FP64 evaluation).
 template <int N>
-__global__ void __launch_bounds__(128) tie_kernel(TraceParams P, RayState* __restrict__ st,
-                                                  const uint32_t* __restrict__ tie_end,
-                                                  const unsigned* __restrict__ n_tie) {
-  const unsigned n = *n_tie;
+__global__ void __launch_bounds__(128) tie_kernel(TraceParams P, RayState* __restrict__ st, CheckLists L) {
+  const unsigned n = *L.n_tie;
   unsigned long long weighed = 0, swapped = 0;
   for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const unsigned item = *(tie_end - k);
+    const unsigned item = L.fail[L.cap - 1 - k];
     RayState& r = st[item];
     float3 o, d;
     float iso;
@@ -145,14 +154,12 @@ __global__ void __launch_bounds__(128) tie_kernel(TraceParams P, RayState* __res
 // The failed rays, traced again by the plain cold-start solver (grid-stride
 // over the device-side count); the plain answer replaces the fast one.
 template <int N>
-__global__ void __launch_bounds__(kTraceBlock) fallback_kernel(TraceParams P, RayState* __restrict__ st,
-                                                               const uint32_t* __restrict__ fail_list,
-                                                               const unsigned* __restrict__ n_fail) {
-  const unsigned n = *n_fail;
+__global__ void __launch_bounds__(kTraceBlock) fallback_kernel(TraceParams P, RayState* __restrict__ st, CheckLists L) {
+  const unsigned n = *L.n_fail;
   Work w;
   unsigned long long newton = 0, face = 0;
   for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const unsigned item = fail_list[k];
+    const unsigned item = L.fail[k];
     float3 o, d;
     float iso;
     bool iso_on;
@@ -188,74 +195,61 @@ __global__ void __launch_bounds__(kTraceBlock) fallback_kernel(TraceParams P, Ra
 
 // Without the check: the listed rays' hits are completed (fill_hit).
 template <int N>
-__global__ void __launch_bounds__(128) post_kernel(TraceParams P, RayState* __restrict__ st,
-                                                   const uint32_t* __restrict__ list,
-                                                   const unsigned* __restrict__ n_list,
-                                                   const uint32_t* __restrict__ list_end,
-                                                   const unsigned* __restrict__ n_back) {
-  unsigned item;
-  if (!listed_item(blockIdx.x * blockDim.x + threadIdx.x, list, *n_list, list_end, *n_back, item)) return;
-  HitState h = st[item].best;
-  if (!(h.flags & kFlagPost)) return;
-  float3 o, d;
-  float iso;
-  bool iso_on;
-  query_ray(P, P.work[item], o, d, iso, iso_on);
-  const CoefRef<false> c{P.rec + static_cast<int64_t>(h.elem) * record_floats(N)};
-  float xJ[12], ug[4] = {0.f, 0.f, 0.f, 0.f};
-  geom_eval_raw<N, false>(c, h.xi, xJ);
-  if (h.kind == HO_HIT_ISO || (__ldg(P.flags + h.elem) & 1u))
-    field_eval_raw<N, false>(c.at(3 * block_floats(N)), h.xi, ug);
-  const float J[9] = {xJ[1], xJ[2], xJ[3], xJ[5], xJ[6], xJ[7], xJ[9], xJ[10], xJ[11]};
-  fill_hit(h, J, ug[0], d);
-  st[item].best = h;
+__global__ void __launch_bounds__(128) post_kernel(TraceParams P, RayState* __restrict__ st, CheckLists L) {
+  const unsigned end = listed_end(L);
+  for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < end;
+       k += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    unsigned item;
+    if (!listed_item(L, static_cast<unsigned>(k), item)) continue;
+    HitState h = st[item].best;
+    if (!(h.flags & kFlagPost)) continue;
+    float3 o, d;
+    float iso;
+    bool iso_on;
+    query_ray(P, P.work[item], o, d, iso, iso_on);
+    const CoefRef<false> c{P.rec + static_cast<int64_t>(h.elem) * record_floats(N)};
+    float xJ[12], ug[4] = {0.f, 0.f, 0.f, 0.f};
+    geom_eval_raw<N, false>(c, h.xi, xJ);
+    if (h.kind == HO_HIT_ISO || (__ldg(P.flags + h.elem) & 1u))
+      field_eval_raw<N, false>(c.at(3 * block_floats(N)), h.xi, ug);
+    const float J[9] = {xJ[1], xJ[2], xJ[3], xJ[5], xJ[6], xJ[7], xJ[9], xJ[10], xJ[11]};
+    fill_hit(h, J, ug[0], d);
+    st[item].best = h;
+  }
 }
 
+// threads: of the launch over the listed rays (they are at most L.cap).
 template <int N>
-cudaError_t launch_post_n(const TraceParams& P, RayState* st, const uint32_t* list, const unsigned* n_list,
-                          const uint32_t* list_end, const unsigned* n_back, int64_t n_cap, cudaStream_t s) {
-  post_kernel<N><<<static_cast<unsigned>((n_cap + 32 + 127) / 128), 128, 0, s>>>(P, st, list, n_list, list_end, n_back);
+cudaError_t launch_post_n(const TraceParams& P, RayState* st, const CheckLists& L, int64_t threads, cudaStream_t s) {
+  post_kernel<N><<<static_cast<unsigned>((threads + 32 + 127) / 128), 128, 0, s>>>(P, st, L);
   return cudaGetLastError();
 }
 
-// fail_list holds n_cap entries (n_cap >= the listed rays); n_fail and
-// n_tie are zeroed by the caller.
 template <int N>
-cudaError_t launch_check_n(const TraceParams& P, RayState* st, const uint32_t* list, const unsigned* n_list,
-                           const uint32_t* list_end, const unsigned* n_back, uint32_t* fail_list, unsigned* n_fail, unsigned* n_tie, int64_t n_cap, int sms,
+cudaError_t launch_check_n(const TraceParams& P, RayState* st, const CheckLists& L, int64_t threads, int sms,
                            cudaStream_t s) {
-  uint32_t* tie_end = fail_list + (n_cap - 1);
-  check_kernel<N><<<static_cast<unsigned>((n_cap + 32 + 127) / 128), 128, 0, s>>>(
-      P, st, list, n_list, list_end, n_back, fail_list, n_fail, tie_end, n_tie);
-  tie_kernel<N><<<sms * 2, 128, 0, s>>>(P, st, tie_end, n_tie);
-  fallback_kernel<N><<<sms * 2, kTraceBlock, 0, s>>>(P, st, fail_list, n_fail);
+  check_kernel<N><<<static_cast<unsigned>((threads + 32 + 127) / 128), 128, 0, s>>>(P, st, L);
+  tie_kernel<N><<<sms * 2, 128, 0, s>>>(P, st, L);
+  fallback_kernel<N><<<sms * 2, kTraceBlock, 0, s>>>(P, st, L);
   return cudaGetLastError();
 }
 
-extern template cudaError_t launch_check_n<2>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<4>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<5>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<6>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<7>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<8>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
-extern template cudaError_t launch_check_n<9>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                              const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*,
-                                              int64_t, int, cudaStream_t);
+extern template cudaError_t launch_check_n<2>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<3>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<4>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<5>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<6>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<7>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<8>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
+extern template cudaError_t launch_check_n<9>(const TraceParams&, RayState*, const CheckLists&, int64_t, int,
+                                              cudaStream_t);
 
 extern template cudaError_t launch_residuals_n<2>(const float*, const uint32_t*, int64_t, const float*, const ho_hit*,
                                                   double*, cudaStream_t);
@@ -274,21 +268,13 @@ extern template cudaError_t launch_residuals_n<8>(const float*, const uint32_t*,
 extern template cudaError_t launch_residuals_n<9>(const float*, const uint32_t*, int64_t, const float*, const ho_hit*,
                                                   double*, cudaStream_t);
 
-extern template cudaError_t launch_post_n<2>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<4>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<5>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<6>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<7>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<8>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
-extern template cudaError_t launch_post_n<9>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                             const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<2>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<4>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<5>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<6>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<7>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<8>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
+extern template cudaError_t launch_post_n<9>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
 
 }  // namespace ho

@@ -137,7 +137,7 @@ struct RoundBufs {
   size_t koff_cap = 0;
   uint32_t* tile_sums = nullptr;  // per 4096 keys, for the offsets' scan
   size_t tile_sums_cap = 0;
-  unsigned* ctr = nullptr;   // pairs, batches, next batch, failed FP64 checks
+  unsigned* ctr = nullptr;   // the rounds' and lists' counters (ho_rounds.cu)
   size_t ctr_cap = 0;
   uint32_t* fail = nullptr;  // queue items whose hit failed the FP64 check
   size_t fail_cap = 0;
@@ -228,6 +228,8 @@ struct ho_context {
   // one stream per element order of a mixed-order scene (the orders' round
   // kernels run side by side), forked from and joined to the call's stream
   cudaStream_t order_streams[ho::kMaxModes + 1] = {};
+  cudaStream_t check_stream = nullptr;  // the check of the rounds' rays, beside the tail
+  cudaEvent_t check_fork = nullptr, check_done = nullptr;
   cudaEvent_t order_fork = nullptr, order_done[ho::kMaxModes + 1] = {};
   // batched / learned engine options (ho_set_option)
   int round_chunk = 0;       // pairs per element batch (0: the kernel's pair slots)

@@ -244,44 +244,44 @@ __global__ void round_gather_kernel(TraceParams P, RayState* __restrict__ st, Ro
   }
 }
 
-// Queued rays listed by a predicate (warp-aggregated appends): hits = false,
-// the rays still in flight after the main rounds (for the tail kernel; the
-// count goes to the work counters too); hits = true, the rays with a hit
-// (for the FP64 check): from the front of the list those that its shorter path
-// answers, face hits away from the face's edges, from the back the others, so
-// that a warp of the check mostly runs one path (a 1920 x 1080 picture of 3
-// isovalues, 1.54 M hits: check 4.2 -> 1.9 ms, tie pass 0.51 -> 0.43 ms).
-__global__ void ray_list_kernel(const unsigned* __restrict__ qcount, const RayState* __restrict__ st, bool hits,
-                                uint32_t* __restrict__ list, unsigned* __restrict__ n_list,
-                                uint32_t* __restrict__ list_end, unsigned* __restrict__ n_back, DevStats* stats) {
-  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool live = false, back = false;
-  if (i < *qcount) {
-    live = hits ? st[i].best.kind != HO_HIT_MISS : !st[i].done;
-    if (hits && live) {
+// Lists rays (all queued ones, or the *n_from of `from`) for the passes after the
+// rounds, so that those passes' threads are all busy. flight (or nullptr): the
+// rays still in flight, for the tail (counted in the work counters too). The
+// others' hits go to the check's list: from its front those that the check's
+// shorter path answers, face hits away from the face's edges, from its back the
+// others, so that a warp of the check mostly runs one path (a 1920 x 1080
+// picture of 3 isovalues, 1.54 M hits: check 4.2 -> 1.9 ms, tie pass 0.51 ->
+// 0.43 ms).
+__global__ void ray_list_kernel(const unsigned* __restrict__ n_from, const uint32_t* __restrict__ from,
+                                const RayState* __restrict__ st, uint32_t* __restrict__ flight,
+                                unsigned* __restrict__ n_flight, CheckLists L, DevStats* stats) {
+  const int lane = threadIdx.x & 31;
+  const unsigned n = *n_from;
+  for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; (k & ~31ull) < n;
+       k += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    int to = -1;  // 0: in flight, 1: front, 2: back
+    unsigned i = 0;
+    if (k < n) {
+      i = from ? from[k] : static_cast<unsigned>(k);
       const HitState& b = st[i].best;
-      back = b.kind != HO_HIT_FACE || !normal_on_face(b.face, b.xi);
-      live = !back;
+      if (flight && !st[i].done) to = 0;
+      else if (b.kind != HO_HIT_MISS) to = b.kind == HO_HIT_FACE && normal_on_face(b.face, b.xi) ? 1 : 2;
+    }
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+      const unsigned m = __ballot_sync(kFull, to == w);
+      if (!m) continue;
+      unsigned* ctr = w == 0 ? n_flight : (w == 1 ? L.n_front : L.n_back);
+      const int leader = __ffs(m) - 1;
+      unsigned base = 0;
+      if (lane == leader) {
+        base = atomicAdd(ctr, static_cast<unsigned>(__popc(m)));
+        if (w == 0) atomicAdd(&stats->c[ST_TAIL], static_cast<unsigned long long>(__popc(m)));
+      }
+      const unsigned at = __shfl_sync(kFull, base, leader) + __popc(m & ((1u << lane) - 1u));
+      if (to == w) (w == 0 ? flight[at] : (w == 1 ? L.list[at] : L.list[L.cap - 1 - at])) = i;
     }
   }
-  const unsigned mb = __ballot_sync(kFull, back);
-  if (mb) {
-    const int lane = threadIdx.x & 31, leader = __ffs(mb) - 1;
-    unsigned base = 0;
-    if (lane == leader) base = atomicAdd(n_back, static_cast<unsigned>(__popc(mb)));
-    base = __shfl_sync(kFull, base, leader);
-    if (back) *(list_end - (base + __popc(mb & ((1u << lane) - 1u)))) = i;
-  }
-  const unsigned m = __ballot_sync(kFull, live);
-  if (!m) return;
-  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-  unsigned base = 0;
-  if (lane == leader) {
-    base = atomicAdd(n_list, static_cast<unsigned>(__popc(m)));
-    if (!hits) atomicAdd(&stats->c[ST_TAIL], static_cast<unsigned long long>(__popc(m)));
-  }
-  base = __shfl_sync(kFull, base, leader);
-  if (live) list[base + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
 // Also tallies the round (non-empty rounds and pairs) into the work counters.
@@ -299,9 +299,9 @@ __global__ void round_scatter_kernel(const RoundPair* __restrict__ pairs, const 
   sorted[koff[pkey[k]] + prank[k]] = pairs[k];
 }
 
-// Ctr layout: [0] pairs of the round, [3] failed FP64 checks, [4..5] the
-// tail's list count and cursor, [6..8] the check's front count, tie count and
-// back count,
+// Ctr layout: [0] pairs of the round, [4..5] the tail's list count and cursor,
+// [6..9] the check's front, back, failure and tie counts, [10..13] the same of
+// the check of the tail's rays,
 // and per order n (2..9) the batch count, region start, write cursor of the
 // face batches, take cursor, and count and write cursor of the isosurface
 // batches, which come first in the region.
@@ -427,6 +427,13 @@ static cudaError_t grow(T*& p, size_t& cap, size_t want, size_t size) {
     if (e_ != cudaSuccess) return int(e_); \
   } while (0)
 
+static int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // Scratch for up to n_cap queued rays (all queries of the call), allocated
 // before any stream capture.
 int prepare_rounds(ho_context* c, int64_t n_cap) {
@@ -444,6 +451,9 @@ int prepare_rounds(ho_context* c, int64_t n_cap) {
               sizeof(uint32_t)));
   RT_TRY(grow(rb.ctr, rb.ctr_cap, kCtrWords, sizeof(unsigned)));
   RT_TRY(grow(rb.fail, rb.fail_cap, n, sizeof(uint32_t)));
+  if (!c->check_stream) RT_TRY(cudaStreamCreateWithFlags(&c->check_stream, cudaStreamNonBlocking));
+  if (!c->check_fork) RT_TRY(cudaEventCreateWithFlags(&c->check_fork, cudaEventDisableTiming));
+  if (!c->check_done) RT_TRY(cudaEventCreateWithFlags(&c->check_done, cudaEventDisableTiming));
   if (__builtin_popcount(c->orders) > 1) {  // streams and events of the orders' launches
     if (!c->order_fork) RT_TRY(cudaEventCreateWithFlags(&c->order_fork, cudaEventDisableTiming));
     for (int m = kMinModes; m <= kMaxModes; ++m) {
@@ -471,71 +481,69 @@ int launch_residuals(ho_context* c, int64_t n, const float* rays, const ho_hit* 
   return int(e);
 }
 
-// FP64 check of the rays' hits, plain fallback of the failures; without the
-// check, the hits are only completed.
-static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, int64_t n_cap) {
-  // the rays with a hit, listed into the (now idle) pair-key buffer, so
-  // that the check's threads are all busy
-  uint32_t* list = reinterpret_cast<uint32_t*>(c->rounds.pkey);
-  unsigned* n_list = c->rounds.ctr + 6;
-  unsigned* n_tie = c->rounds.ctr + 7;
-  unsigned* n_back = c->rounds.ctr + 8;
-  uint32_t* list_end = list + (n_cap - 1);
-  RT_TRY(cudaMemsetAsync(c->rounds.ctr + 3, 0, sizeof(unsigned), s));
-  RT_TRY(cudaMemsetAsync(n_list, 0, 3 * sizeof(unsigned), s));
-  ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, R.state, true, list, n_list,
-                                                                             list_end, n_back, P.stats);
-  RT_TRY(cudaGetLastError());
+// Scratch of the check's launches: in the pair-key and failure buffers, or, for
+// the rays that the tail finished (second), in the pair buffer. All are idle
+// after the rounds. The counters are to be zeroed.
+static CheckLists check_lists(ho_context* c, int64_t n_cap, bool second) {
+  RoundBufs& rb = c->rounds;
+  CheckLists L;
+  L.cap = n_cap;
+  L.list = second ? static_cast<uint32_t*>(rb.pairs) : reinterpret_cast<uint32_t*>(rb.pkey);
+  L.fail = second ? static_cast<uint32_t*>(rb.pairs) + n_cap : rb.fail;
+  unsigned* ctr = rb.ctr + (second ? 10 : 6);
+  L.n_front = ctr;
+  L.n_back = ctr + 1;
+  L.n_fail = ctr + 2;
+  L.n_tie = ctr + 3;
+  return L;
+}
+static_assert(2 * sizeof(RoundPair) >= 2 * sizeof(uint32_t), "the pair buffer holds two lists");
+
+// FP64 check of the listed rays' hits, plain fallback of the failures; without
+// the check, the hits are only completed.
+static int enqueue_check(ho_context* c, const TraceParams& P, const RoundParams& R, const CheckLists& L, cudaStream_t s,
+                         int64_t threads) {
+  cudaError_t e;
   if (!c->fp64_check) {
-    c->launches += 2;  // ray list, post
-    cudaError_t e;
+    c->launches += 1;
     switch (c->N) {
-      case 2: e = launch_post_n<2>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 3: e = launch_post_n<3>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 4: e = launch_post_n<4>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 5: e = launch_post_n<5>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 6: e = launch_post_n<6>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 7: e = launch_post_n<7>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 8: e = launch_post_n<8>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
-      case 9: e = launch_post_n<9>(P, R.state, list, n_list, list_end, n_back, n_cap, s); break;
+      case 2: e = launch_post_n<2>(P, R.state, L, threads, s); break;
+      case 3: e = launch_post_n<3>(P, R.state, L, threads, s); break;
+      case 4: e = launch_post_n<4>(P, R.state, L, threads, s); break;
+      case 5: e = launch_post_n<5>(P, R.state, L, threads, s); break;
+      case 6: e = launch_post_n<6>(P, R.state, L, threads, s); break;
+      case 7: e = launch_post_n<7>(P, R.state, L, threads, s); break;
+      case 8: e = launch_post_n<8>(P, R.state, L, threads, s); break;
+      case 9: e = launch_post_n<9>(P, R.state, L, threads, s); break;
       default: e = cudaErrorInvalidValue; break;
     }
     return int(e);
   }
-  c->launches += 4;  // ray list, check, tie rule, fallback
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaError_t e;
+  c->launches += 3;  // check, tie rule, fallback
+  const int sms = sm_count();
   switch (c->N) {
-    case 2:
-      e = launch_check_n<2>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 3:
-      e = launch_check_n<3>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 4:
-      e = launch_check_n<4>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 5:
-      e = launch_check_n<5>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 6:
-      e = launch_check_n<6>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 7:
-      e = launch_check_n<7>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 8:
-      e = launch_check_n<8>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
-    case 9:
-      e = launch_check_n<9>(P, R.state, list, n_list, list_end, n_back, c->rounds.fail, c->rounds.ctr + 3, n_tie, n_cap, sms, s);
-      break;
+    case 2: e = launch_check_n<2>(P, R.state, L, threads, sms, s); break;
+    case 3: e = launch_check_n<3>(P, R.state, L, threads, sms, s); break;
+    case 4: e = launch_check_n<4>(P, R.state, L, threads, sms, s); break;
+    case 5: e = launch_check_n<5>(P, R.state, L, threads, sms, s); break;
+    case 6: e = launch_check_n<6>(P, R.state, L, threads, sms, s); break;
+    case 7: e = launch_check_n<7>(P, R.state, L, threads, sms, s); break;
+    case 8: e = launch_check_n<8>(P, R.state, L, threads, sms, s); break;
+    case 9: e = launch_check_n<9>(P, R.state, L, threads, sms, s); break;
     default: e = cudaErrorInvalidValue; break;
   }
-  RT_TRY(e);
-  return 0;
+  return int(e);
+}
+
+// The check of every queued ray with a hit.
+static int enqueue_check_all(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, int64_t n_cap) {
+  const CheckLists L = check_lists(c, n_cap, false);
+  RT_TRY(cudaMemsetAsync(L.n_front, 0, 4 * sizeof(unsigned), s));
+  ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, nullptr, R.state, nullptr, nullptr,
+                                                                             L, P.stats);
+  RT_TRY(cudaGetLastError());
+  ++c->launches;
+  return enqueue_check(c, P, R, L, s, n_cap);
 }
 
 static RoundParams round_params(ho_context* c, const TraceParams& P) {
@@ -618,10 +626,7 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   round_scatter_kernel<<<gi, 256, 0, s>>>(gathered, rb.pkey, rb.prank, rb.koff, rb.ctr,
                                           const_cast<RoundPair*>(R.pairs), P.stats);
   const unsigned ge = static_cast<unsigned>((n_keys + 255) / 256);
-  int dev = 0, sms = 0;
-  RT_TRY(cudaGetDevice(&dev));
-  RT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const unsigned spread = kSpreadPerSm * static_cast<unsigned>(sms);
+  const unsigned spread = kSpreadPerSm * static_cast<unsigned>(sm_count());
   round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread, rb.ctr);
   round_order_offsets_kernel<<<1, 1, 0, s>>>(rb.ctr);
   round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread,
@@ -670,34 +675,52 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   return 0;
 }
 
-// The tail: every ray still in flight finished by the warp-per-ray kernel;
-// afterwards no round has pairs left (ctr[0] = 0).
-static int enqueue_tail(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, bool learned,
-                        int64_t n_cap) {
+// The tail and the check: every ray still in flight is finished by the
+// warp-per-ray kernel; afterwards no round has pairs left (ctr[0] = 0). The tail
+// is a few long chains that leave most of the device idle, so the check of the
+// rays that the rounds finished runs beside it, on a stream of its own (a branch
+// of the graph in a captured call); the tail's rays are checked after it. The
+// tail is enqueued first: its blocks then have their places, and the check's
+// fill the rest.
+static int enqueue_tail_and_check(ho_context* c, const TraceParams& P, const RoundParams& R, cudaStream_t s, bool learned,
+                                  int64_t n_cap) {
   RoundBufs& rb = c->rounds;
   unsigned* n_list = rb.ctr + 4;
   unsigned* next = rb.ctr + 5;
-  RT_TRY(cudaMemsetAsync(rb.ctr + 4, 0, 2 * sizeof(unsigned), s));
-  round_gather_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(
-      P, R.state, static_cast<RoundPair*>(rb.pairs), rb.pkey, rb.prank, rb.kcount, rb.ctr, 0, true);
-  ray_list_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P.qcount, R.state, false, rb.fail,
-                                                                             n_list, nullptr, nullptr, P.stats);
+  const unsigned gi = static_cast<unsigned>((n_cap + 255) / 256);
+  const CheckLists first = check_lists(c, n_cap, false), second = check_lists(c, n_cap, true);
+  RT_TRY(cudaMemsetAsync(rb.ctr + 4, 0, 10 * sizeof(unsigned), s));
+  round_gather_kernel<<<gi, 256, 0, s>>>(P, R.state, static_cast<RoundPair*>(rb.pairs), rb.pkey, rb.prank, rb.kcount,
+                                         rb.ctr, 0, true);
+  ray_list_kernel<<<gi, 256, 0, s>>>(P.qcount, nullptr, R.state, rb.prank, n_list, first, P.stats);
   RT_TRY(cudaGetLastError());
+  RT_TRY(cudaEventRecord(c->check_fork, s));
   cudaError_t e;
   switch (c->N) {
-    case 2: e = launch_tail_n<2>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 3: e = launch_tail_n<3>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 4: e = launch_tail_n<4>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 5: e = launch_tail_n<5>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 6: e = launch_tail_n<6>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 7: e = launch_tail_n<7>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 8: e = launch_tail_n<8>(P, R.state, rb.fail, n_list, next, learned, s); break;
-    case 9: e = launch_tail_n<9>(P, R.state, rb.fail, n_list, next, learned, s); break;
+    case 2: e = launch_tail_n<2>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 3: e = launch_tail_n<3>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 4: e = launch_tail_n<4>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 5: e = launch_tail_n<5>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 6: e = launch_tail_n<6>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 7: e = launch_tail_n<7>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 8: e = launch_tail_n<8>(P, R.state, rb.prank, n_list, next, learned, s); break;
+    case 9: e = launch_tail_n<9>(P, R.state, rb.prank, n_list, next, learned, s); break;
     default: e = cudaErrorInvalidValue; break;
   }
   RT_TRY(e);
+  RT_TRY(cudaStreamWaitEvent(c->check_stream, c->check_fork, 0));
+  int rc = enqueue_check(c, P, R, first, c->check_stream, n_cap);
+  RT_TRY(cudaEventRecord(c->check_done, c->check_stream));
+  if (rc) return rc;
+  const int64_t few = std::min<int64_t>(n_cap, static_cast<int64_t>(sm_count()) * 1024);
+  ray_list_kernel<<<static_cast<unsigned>((few + 255) / 256), 256, 0, s>>>(n_list, rb.prank, R.state, nullptr, nullptr,
+                                                                           second, P.stats);
+  RT_TRY(cudaGetLastError());
+  rc = enqueue_check(c, P, R, second, s, few);
+  if (rc) return rc;
+  RT_TRY(cudaStreamWaitEvent(s, c->check_done, 0));
   RT_TRY(cudaMemsetAsync(rb.ctr, 0, sizeof(unsigned), s));
-  c->launches += 3;
+  c->launches += 4;
   return 0;
 }
 
@@ -715,14 +738,9 @@ int enqueue_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool lea
     const int rc = enqueue_round(c, P, R, s, learned, n_cap, c->tail_after > 0 ? rounds : 0);
     if (rc) return rc;
   }
-  if (c->tail_after > 0) {
-    const int rc = enqueue_tail(c, P, R, s, learned, n_cap);
-    if (rc) return rc;
-  }
-  {
-    const int rc = enqueue_check(c, P, R, s, n_cap);
-    if (rc) return rc;
-  }
+  const int rc = c->tail_after > 0 ? enqueue_tail_and_check(c, P, R, s, learned, n_cap)
+                                   : enqueue_check_all(c, P, R, s, n_cap);
+  if (rc) return rc;
   round_finish_kernel<<<gi, 256, 0, s>>>(P, R.state, true);
   RT_TRY(cudaGetLastError());
   return 0;
@@ -746,7 +764,7 @@ int finish_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool lear
     if (rc) return rc;
   }
   if (extra) {
-    const int rc = enqueue_check(c, P, R, s, n_cap);
+    const int rc = enqueue_check_all(c, P, R, s, n_cap);
     if (rc) return rc;
     round_finish_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P, R.state, false);
     RT_TRY(cudaGetLastError());

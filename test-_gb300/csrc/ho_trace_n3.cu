@@ -10,9 +10,6 @@ template cudaError_t launch_residuals_n<3>(const float*, const uint32_t*, int64_
                                            double*, cudaStream_t);
 template cudaError_t launch_tail_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*, unsigned*, bool,
                                       cudaStream_t);
-template cudaError_t launch_check_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                       const uint32_t*, const unsigned*, uint32_t*, unsigned*, unsigned*, int64_t, int,
-                                       cudaStream_t);
-template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const uint32_t*, const unsigned*,
-                                      const uint32_t*, const unsigned*, int64_t, cudaStream_t);
+template cudaError_t launch_check_n<3>(const TraceParams&, RayState*, const CheckLists&, int64_t, int, cudaStream_t);
+template cudaError_t launch_post_n<3>(const TraceParams&, RayState*, const CheckLists&, int64_t, cudaStream_t);
 }  // namespace ho

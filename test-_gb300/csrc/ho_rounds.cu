@@ -626,7 +626,9 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   round_scatter_kernel<<<gi, 256, 0, s>>>(gathered, rb.pkey, rb.prank, rb.koff, rb.ctr,
                                           const_cast<RoundPair*>(R.pairs), P.stats);
   const unsigned ge = static_cast<unsigned>((n_keys + 255) / 256);
-  const unsigned spread = kSpreadPerSm * static_cast<unsigned>(sm_count());
+  // with the network's predictions, a solve's restarts depend on what else its
+  // warp runs: full batches for every call size
+  const unsigned spread = learned ? 1u : kSpreadPerSm * static_cast<unsigned>(sm_count());
   round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread, rb.ctr);
   round_order_offsets_kernel<<<1, 1, 0, s>>>(rb.ctr);
   round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread,

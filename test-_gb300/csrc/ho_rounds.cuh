@@ -46,6 +46,18 @@ namespace ho {
 
 constexpr int kRoundBlock = 128;  // 4 warps, one batch each
 constexpr int kSamples = 17;
+// Ended solves after which a warp's step goes on to their phase transitions and
+// the next tasks. Those run straight through a lot of code, and the kernel waits
+// on instruction fetches more than on anything else (2.2 of 6.7 cycles per issue
+// with one transition pass per solver iteration); the lanes that wait for the
+// others cost less. 1920 x 1080, 3 isovalues: call 14.3 ms with a pass per
+// iteration, 14.1 / 13.7 / 13.6 / 13.2 / 13.3 ms for 1 / 4 / 8 / 12 / 16 ended
+// lanes; mixed orders 17.6 -> 17.0 / 16.2 / 15.8 / 15.4 / 15.0 ms; a 3840 x 2160
+// picture of 6 modes 16.3 -> 14.3 ms, four path bounces 12.1 -> 11.3 ms.
+// With the network's predictions a failed warm start goes on from the samples of
+// its pair that have ended so far, so there every end is seen at once, as it would
+// be with a pass per iteration (16 changed 9 answers of 18.7 M).
+constexpr int kEndLanes = 16;
 
 // Pairs per batch (HO_OPT_ROUND_CHUNK, default the slot count): a warp admits
 // a batch's pairs into its slots as earlier pairs finish, so a batch may be
@@ -741,216 +753,228 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
         ++w.steps;
         w.lanes += 32u - __popc(idle) + min(avail, static_cast<unsigned>(__popc(idle)));
       }
-      // -- evaluate: every busy lane evaluates the geometry at its point
+      // -- the lanes' solves, until kEndLanes of them have ended or none runs: every
+      // running lane evaluates the geometry at its point
       const bool act = s.task >= 0;
-      float3 X = make_float3(0.f, 0.f, 0.f);
-      float J[9];
-      float u = 0.f;
-      float3 gr = make_float3(0.f, 0.f, 0.f);
-      // inverse-map iteration of an isosurface solve: the field comes with it
-      const bool on_face = s.kind == TK_FSEED || s.kind == TK_FLEARN;
-      const bool want_field = act && !on_face;
-      float4 r[4];
-      if constexpr (TC) {
-        // every thread's point as a row of the step's MMAs; idle lanes give a
-        // row at xi = 0 whose results are not used
-        const float3 xi = act ? s.xi : make_float3(0.f, 0.f, 0.f);
-        float ar[N], dr[N], as[N], ds[N], at[N], dt[N];
-        basis_val_der<N>(xi.x, ar, dr);
-        basis_val_der<N>(xi.y, as, ds);
-        basis_val_der<N>(xi.z, at, dt);
-        tc_stage_a<N>(T, threadIdx.x, ar, dr);
-        tc_proxy_fence();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (threadIdx.x == 0) tc_issue(T, tmem);
-        const bool done = tc_mbar_wait(&T.mbar, phase);
-        phase ^= 1u;
-        if (__syncthreads_or(!done)) {  // the MMAs did not complete in time: give up the round
-          if (threadIdx.x == 0) atomicOr(&P.stats->status, kStatusRoundGuard);
-          tc_ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-        if (__any_sync(kFull, act)) {
-#pragma unroll 1
-          for (int comp = 0; comp < 3; ++comp) r[comp] = tc_finish_comp<N>(taddr, comp, as, ds, at, dt);
-        }
-        if (__any_sync(kFull, want_field)) r[3] = tc_finish_comp<N>(taddr, 3, as, ds, at, dt);
-      }
-      if constexpr (!TC) {
-        int fixed = 0, ua = 0, va = 0, f = 0;
-        float val = 0.f;
-        if (act && on_face) {
-          f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
-          face_param(f, fixed, val, ua, va);
-        }
-        eval_points<N, false>(el.c, act && !on_face, s.xi, 0, r);
-        eval_points<N, true>(el.c, act && on_face, make_float3(getc(s.xi, ua), getc(s.xi, va), 0.f), f, r);
-      }
-      if (act) {
-        w.flops += !TC && on_face ? face_eval_flops(N) : eval_flops(N, on_face ? 3 : 4);
-        if (!TC && on_face) {
-          X = make_float3(r[0].x, r[1].x, r[2].x);
-          // the columns of the two tangents; the third is not used on a face
-          const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
-          int fixed, ua, va;
-          float val;
-          face_param(f, fixed, val, ua, va);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            J[3 * c] = r[c].y;
-            J[3 * c + 1] = ua == 1 ? r[c].y : r[c].z;
-            J[3 * c + 2] = r[c].z;
-          }
-        } else {
-          X = make_float3(r[0].x, r[1].x, r[2].x);
-          J[0] = r[0].y; J[1] = r[0].z; J[2] = r[0].w;
-          J[3] = r[1].y; J[4] = r[1].z; J[5] = r[1].w;
-          J[6] = r[2].y; J[7] = r[2].z; J[8] = r[2].w;
-        }
-        ++w.geom;
-        if (want_field) {
-          u = r[3].x;
-          gr = make_float3(r[3].y, r[3].z, r[3].w);
-          ++w.field;
-        }
-      }
-      // -- advance the solve
       // end: 0 running, 1 converged / accepted, 2 failed
       int end = 0;
       float sf = 0.f, sdf = 0.f;
       float3 sg = make_float3(0.f, 0.f, 0.f);
-      if (act) {
-        PairSm& p = W.pair(s.pp);
-        if (!on_face) {
-          float K[9];
-          invert3(J, K);
-          ++w.newton;
-          w.flops += kSolveFlops;
-          const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
-                      rz = X.z - (p.o[2] + s.t * p.d[2]);
-          const float d0 = K[0] * rx + K[1] * ry + K[2] * rz;
-          const float d1 = K[3] * rx + K[4] * ry + K[5] * rz;
-          const float d2 = K[6] * rx + K[7] * ry + K[8] * rz;
-          s.xi.x -= d0;
-          s.xi.y -= d1;
-          s.xi.z -= d2;
-          ++s.it;
-          if (fabsf(d0) < 1e-5f && fabsf(d1) < 1e-5f && fabsf(d2) < 1e-5f) {
-            // value and gradient at the converged point, first order
-            sg = make_float3(K[0] * gr.x + K[3] * gr.y + K[6] * gr.z, K[1] * gr.x + K[4] * gr.y + K[7] * gr.z,
-                             K[2] * gr.x + K[5] * gr.y + K[8] * gr.z);
-            sf = (u - (gr.x * d0 + gr.y * d1 + gr.z * d2)) - p.iso;
-            sdf = sg.x * p.d[0] + sg.y * p.d[1] + sg.z * p.d[2];
-            end = 1;
-          } else if (!(fabsf(d0) + fabsf(d1) + fabsf(d2) < FLT_MAX)) {
-            end = 2;
-          } else if (s.it >= s.cap) {
-            end = 2;
+      for (;;) {
+        const bool go = act && end == 0;
+        float3 X = make_float3(0.f, 0.f, 0.f);
+        float J[9];
+        float u = 0.f;
+        float3 gr = make_float3(0.f, 0.f, 0.f);
+        // inverse-map iteration of an isosurface solve: the field comes with it
+        const bool on_face = s.kind == TK_FSEED || s.kind == TK_FLEARN;
+        const bool want_field = go && !on_face;
+        float4 r[4];
+        if constexpr (TC) {
+          // every thread's point as a row of the step's MMAs; idle lanes give a
+          // row at xi = 0 whose results are not used
+          const float3 xi = go ? s.xi : make_float3(0.f, 0.f, 0.f);
+          float ar[N], dr[N], as[N], ds[N], at[N], dt[N];
+          basis_val_der<N>(xi.x, ar, dr);
+          basis_val_der<N>(xi.y, as, ds);
+          basis_val_der<N>(xi.z, at, dt);
+          tc_stage_a<N>(T, threadIdx.x, ar, dr);
+          tc_proxy_fence();
+          tc_fence_before();
+          __syncthreads();
+          tc_fence_after();
+          if (threadIdx.x == 0) tc_issue(T, tmem);
+          const bool done = tc_mbar_wait(&T.mbar, phase);
+          phase ^= 1u;
+          if (__syncthreads_or(!done)) {  // the MMAs did not complete in time: give up the round
+            if (threadIdx.x == 0) atomicOr(&P.stats->status, kStatusRoundGuard);
+            tc_ok = false;
+            break;
           }
-          if (s.warm && end != 0) {
-            if (end == 1) {
-              ++w.accepted;
-            } else {
-              ++w.rejected;
-              atomicAdd(&p.its, s.it);
-              // a sample whose warm start failed starts again from the
-              // nearest converged sample of its pair that it has not tried
-              // yet (stored in an earlier step), each time capped; when none
-              // is left, the plain cold start answers. The cold start is a
-              // chain of up to 50 steps that holds its lane and its pair:
-              // trying every converged neighbour first took hex64_p5
-              // learned from 46.6 to 41.1 ms per call (one neighbour: 46.6;
-              // none: 48.6)
-              int nb = -1;
-              if (s.kind == TK_SAMPLE) {
-                int bd = kSamples;
-                for (unsigned m = ld_ctl(&p.okm) & ~s.tried; m; m &= m - 1u) {
-                  const int j = __ffs(m) - 1, dj = abs(j - s.arg);
-                  if (dj < bd) {
-                    bd = dj;
-                    nb = j;
-                  }
-                }
-              }
-              if (nb >= 0) {
-                s.tried |= 1u << nb;
-                s.xi = ld3(p.sx[nb]);
-                s.cap = P.warm_cap;
-              } else {
-                atomicOr(&p.fl, 8);
-                s.warm = false;
-                s.xi = make_float3(0.f, 0.f, 0.f);
-                s.cap = 50;
-              }
-              s.it = 0;
-                        end = 0;
+          tc_fence_after();
+          const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+          if (__any_sync(kFull, go)) {
+#pragma unroll 1
+            for (int comp = 0; comp < 3; ++comp) r[comp] = tc_finish_comp<N>(taddr, comp, as, ds, at, dt);
+          }
+          if (__any_sync(kFull, want_field)) r[3] = tc_finish_comp<N>(taddr, 3, as, ds, at, dt);
+        }
+        if constexpr (!TC) {
+          int fixed = 0, ua = 0, va = 0, f = 0;
+          float val = 0.f;
+          if (go && on_face) {
+            f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
+            face_param(f, fixed, val, ua, va);
+          }
+          eval_points<N, false>(el.c, go && !on_face, s.xi, 0, r);
+          eval_points<N, true>(el.c, go && on_face, make_float3(getc(s.xi, ua), getc(s.xi, va), 0.f), f, r);
+        }
+        if (go) {
+          w.flops += !TC && on_face ? face_eval_flops(N) : eval_flops(N, on_face ? 3 : 4);
+          if (!TC && on_face) {
+            X = make_float3(r[0].x, r[1].x, r[2].x);
+            // the columns of the two tangents; the third is not used on a face
+            const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
+            int fixed, ua, va;
+            float val;
+            face_param(f, fixed, val, ua, va);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              J[3 * c] = r[c].y;
+              J[3 * c + 1] = ua == 1 ? r[c].y : r[c].z;
+              J[3 * c + 2] = r[c].z;
             }
-          }
-        } else {
-          const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
-          int fixed, ua, va;
-          float val;
-          face_param(f, fixed, val, ua, va);
-          const float tmin = 0.001f, tmax = p.best_t;
-          if (!s.inited) {  // seed: tau from the seed point's position (same evaluation)
-            const float dd = p.d[0] * p.d[0] + p.d[1] * p.d[1] + p.d[2] * p.d[2];
-            float tau = dd > 0.f ? ((X.x - p.o[0]) * p.d[0] + (X.y - p.o[1]) * p.d[1] + (X.z - p.o[2]) * p.d[2]) / dd
-                                 : 0.f;
-            s.t = fminf(fmaxf(tau, tmin), tmax);
-            s.inited = true;
-          }
-          ++w.face;
-          w.flops += kSolveFlops;
-          const bool first = s.kind == TK_FSEED && (p.fl & 16) != 0 && s.arg == 9 * f;
-          const float3 xi0 = s.xi;
-          const float t0 = s.t;
-          const bool late = s.it == kSeedPatience;
-          const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
-                      rz = X.z - (p.o[2] + s.t * p.d[2]);
-          const float m = fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz)));
-          if (m < 1e-4f) {
-            const float pu = getc(s.xi, ua), pv = getc(s.xi, va);
-            end = (pu >= -1.001f && pu <= 1.001f && pv >= -1.001f && pv <= 1.001f && s.t >= tmin && s.t <= tmax) ? 1
-                                                                                                                : 2;
-          } else if (s.it > 5 && m > s.prev * 1.5f) {
-            end = 2;
           } else {
-            s.prev = m;
-            const float A[9] = {J[ua], J[va], -p.d[0], J[3 + ua], J[3 + va], -p.d[1], J[6 + ua], J[6 + va], -p.d[2]};
-            float K[9];
-            invert3(A, K);
-            const float du = -(K[0] * rx + K[1] * ry + K[2] * rz);
-            const float dv = -(K[3] * rx + K[4] * ry + K[5] * rz);
-            const float dtau = -(K[6] * rx + K[7] * ry + K[8] * rz);
-            const float mx = fmaxf(fabsf(du), fmaxf(fabsf(dv), fabsf(dtau)));
-            const float sc = mx > 0.25f ? 0.25f / mx : 1.0f;
-            float nu = getc(s.xi, ua) + du * sc, nv = getc(s.xi, va) + dv * sc;
-            s.t = fminf(fmaxf(s.t + dtau * sc, tmin), tmax);
-            nu = fminf(fmaxf(nu, -1.5f), 1.5f);
-            nv = fminf(fmaxf(nv, -1.5f), 1.5f);
-            setc(s.xi, ua, nu);
-            setc(s.xi, va, nv);
-            setc(s.xi, fixed, val);
-            if (++s.it >= s.cap) end = 2;
+            X = make_float3(r[0].x, r[1].x, r[2].x);
+            J[0] = r[0].y; J[1] = r[0].z; J[2] = r[0].w;
+            J[3] = r[1].y; J[4] = r[1].z; J[5] = r[1].w;
+            J[6] = r[2].y; J[7] = r[2].z; J[8] = r[2].w;
           }
-          // a first seed that ends without a hit, or takes long: none may have one
-          if (first && (end == 2 || (end == 0 && late)) &&
-              face_impossible(P.cull + static_cast<int64_t>(p.elem) * kCullFloats, f, ld3(p.o), ld3(p.d), xi0, X, t0, 0.f,
-                              tmin, tmax)) {
-            atomicAnd(&p.ftodo, ~(1u << f));
-            end = 2;
-          }
-          if (end != 0 && s.kind == TK_FLEARN) {
-            if (end == 1) ++w.accepted;
-            else ++w.rejected;
+          ++w.geom;
+          if (want_field) {
+            u = r[3].x;
+            gr = make_float3(r[3].y, r[3].z, r[3].w);
+            ++w.field;
           }
         }
-        if (end != 0) atomicAdd(&p.its, s.it);
+        // -- advance the solve
+        if (go) {
+          PairSm& p = W.pair(s.pp);
+          if (!on_face) {
+            float K[9];
+            invert3(J, K);
+            ++w.newton;
+            w.flops += kSolveFlops;
+            const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
+                        rz = X.z - (p.o[2] + s.t * p.d[2]);
+            const float d0 = K[0] * rx + K[1] * ry + K[2] * rz;
+            const float d1 = K[3] * rx + K[4] * ry + K[5] * rz;
+            const float d2 = K[6] * rx + K[7] * ry + K[8] * rz;
+            s.xi.x -= d0;
+            s.xi.y -= d1;
+            s.xi.z -= d2;
+            ++s.it;
+            if (fabsf(d0) < 1e-5f && fabsf(d1) < 1e-5f && fabsf(d2) < 1e-5f) {
+              // value and gradient at the converged point, first order
+              sg = make_float3(K[0] * gr.x + K[3] * gr.y + K[6] * gr.z, K[1] * gr.x + K[4] * gr.y + K[7] * gr.z,
+                               K[2] * gr.x + K[5] * gr.y + K[8] * gr.z);
+              sf = (u - (gr.x * d0 + gr.y * d1 + gr.z * d2)) - p.iso;
+              sdf = sg.x * p.d[0] + sg.y * p.d[1] + sg.z * p.d[2];
+              end = 1;
+            } else if (!(fabsf(d0) + fabsf(d1) + fabsf(d2) < FLT_MAX)) {
+              end = 2;
+            } else if (s.it >= s.cap) {
+              end = 2;
+            }
+            if (s.warm && end != 0) {
+              if (end == 1) {
+                ++w.accepted;
+              } else {
+                ++w.rejected;
+                atomicAdd(&p.its, s.it);
+                // a sample whose warm start failed starts again from the
+                // nearest converged sample of its pair that it has not tried
+                // yet (stored in an earlier step), each time capped; when none
+                // is left, the plain cold start answers. The cold start is a
+                // chain of up to 50 steps that holds its lane and its pair:
+                // trying every converged neighbour first took hex64_p5
+                // learned from 46.6 to 41.1 ms per call (one neighbour: 46.6;
+                // none: 48.6)
+                int nb = -1;
+                if (s.kind == TK_SAMPLE) {
+                  int bd = kSamples;
+                  for (unsigned m = ld_ctl(&p.okm) & ~s.tried; m; m &= m - 1u) {
+                    const int j = __ffs(m) - 1, dj = abs(j - s.arg);
+                    if (dj < bd) {
+                      bd = dj;
+                      nb = j;
+                    }
+                  }
+                }
+                if (nb >= 0) {
+                  s.tried |= 1u << nb;
+                  s.xi = ld3(p.sx[nb]);
+                  s.cap = P.warm_cap;
+                } else {
+                  atomicOr(&p.fl, 8);
+                  s.warm = false;
+                  s.xi = make_float3(0.f, 0.f, 0.f);
+                  s.cap = 50;
+                }
+                s.it = 0;
+                          end = 0;
+              }
+            }
+          } else {
+            const int f = s.kind == TK_FSEED ? s.arg / 9 : s.arg;
+            int fixed, ua, va;
+            float val;
+            face_param(f, fixed, val, ua, va);
+            const float tmin = 0.001f, tmax = p.best_t;
+            if (!s.inited) {  // seed: tau from the seed point's position (same evaluation)
+              const float dd = p.d[0] * p.d[0] + p.d[1] * p.d[1] + p.d[2] * p.d[2];
+              float tau = dd > 0.f ? ((X.x - p.o[0]) * p.d[0] + (X.y - p.o[1]) * p.d[1] + (X.z - p.o[2]) * p.d[2]) / dd
+                                   : 0.f;
+              s.t = fminf(fmaxf(tau, tmin), tmax);
+              s.inited = true;
+            }
+            ++w.face;
+            w.flops += kSolveFlops;
+            const bool first = s.kind == TK_FSEED && (p.fl & 16) != 0 && s.arg == 9 * f;
+            const float3 xi0 = s.xi;
+            const float t0 = s.t;
+            const bool late = s.it == kSeedPatience;
+            const float rx = X.x - (p.o[0] + s.t * p.d[0]), ry = X.y - (p.o[1] + s.t * p.d[1]),
+                        rz = X.z - (p.o[2] + s.t * p.d[2]);
+            const float m = fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz)));
+            if (m < 1e-4f) {
+              const float pu = getc(s.xi, ua), pv = getc(s.xi, va);
+              end = (pu >= -1.001f && pu <= 1.001f && pv >= -1.001f && pv <= 1.001f && s.t >= tmin && s.t <= tmax) ? 1
+                                                                                                                  : 2;
+            } else if (s.it > 5 && m > s.prev * 1.5f) {
+              end = 2;
+            } else {
+              s.prev = m;
+              const float A[9] = {J[ua], J[va], -p.d[0], J[3 + ua], J[3 + va], -p.d[1], J[6 + ua], J[6 + va], -p.d[2]};
+              float K[9];
+              invert3(A, K);
+              const float du = -(K[0] * rx + K[1] * ry + K[2] * rz);
+              const float dv = -(K[3] * rx + K[4] * ry + K[5] * rz);
+              const float dtau = -(K[6] * rx + K[7] * ry + K[8] * rz);
+              const float mx = fmaxf(fabsf(du), fmaxf(fabsf(dv), fabsf(dtau)));
+              const float sc = mx > 0.25f ? 0.25f / mx : 1.0f;
+              float nu = getc(s.xi, ua) + du * sc, nv = getc(s.xi, va) + dv * sc;
+              s.t = fminf(fmaxf(s.t + dtau * sc, tmin), tmax);
+              nu = fminf(fmaxf(nu, -1.5f), 1.5f);
+              nv = fminf(fmaxf(nv, -1.5f), 1.5f);
+              setc(s.xi, ua, nu);
+              setc(s.xi, va, nv);
+              setc(s.xi, fixed, val);
+              if (++s.it >= s.cap) end = 2;
+            }
+            // a first seed that ends without a hit, or takes long: none may have one
+            if (first && (end == 2 || (end == 0 && late)) &&
+                face_impossible(P.cull + static_cast<int64_t>(p.elem) * kCullFloats, f, ld3(p.o), ld3(p.d), xi0, X, t0, 0.f,
+                                tmin, tmax)) {
+              atomicAnd(&p.ftodo, ~(1u << f));
+              end = 2;
+            }
+            if (end != 0 && s.kind == TK_FLEARN) {
+              if (end == 1) ++w.accepted;
+              else ++w.rejected;
+            }
+          }
+          if (end != 0) atomicAdd(&p.its, s.it);
+        }
+        if constexpr (TC) break;
+        const unsigned run = __ballot_sync(kFull, act && end == 0);
+        if (run == 0u || __popc(__ballot_sync(kFull, act && end != 0)) >= (L ? 1 : kEndLanes)) break;
+        if (lane == 0) {
+          ++w.steps;
+          w.lanes += __popc(run);
+        }
       }
+      if (TC && !tc_ok) break;
       // every lane has read the pair state of this step (the neighbour
       // restart reads the sample store) before any lane writes to it
       __syncwarp();

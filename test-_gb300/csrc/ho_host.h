@@ -186,7 +186,7 @@ struct ho_context {
   int64_t n_pnodes = 0;
   int pbvh_depth = 0;
   int64_t prim_counts[3] = {0, 0, 0};
-  void* d_pheavy = nullptr;       // queries that the primitive pass hands to its warp-per-query kernel
+  void* d_pheavy = nullptr;       // queries that the primitive pass hands to its second kernel
   size_t pheavy_cap = 0;          // its bytes
   cudaEvent_t pheavy_done = nullptr;  // that kernel's last launch
   ho_hit* d_phits = nullptr;      // hits of calls that asked for none (the primitive pass needs them)

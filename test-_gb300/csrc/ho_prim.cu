@@ -6,9 +6,11 @@
 // engine first; the primitive pass then visits, per query, the primitives
 // whose box the ray meets in ascending (box entry, index) order, each on the
 // segment [0.001, closest hit so far] that starts at the hexahedra's hit,
-// and keeps a primitive hit when it is nearer. One thread per query: the
-// per-primitive solves are short, branchy FP32 Newton loops whose start
-// search the reference defines by exact comparisons. This file is compiled
+// and keeps a primitive hit when it is nearer. One thread per query, until the
+// query has spent kPrimBudget solver iterations; those queries' searches are then
+// dealt over the lanes of warps. The per-primitive solves are short, branchy
+// FP32 Newton loops whose start search the reference defines by exact
+// comparisons. This file is compiled
 // without multiply-add contraction (see ho_prim.cuh).
 #include <cuda_runtime.h>
 
@@ -202,7 +204,7 @@ struct PrimParams {
   int64_t n_queries;
   bool fresh;
   DevStats* stats;
-  struct PrimHeavy* heavy;  // queries handed to the warp-per-query kernel (nullptr: none are)
+  struct PrimHeavy* heavy;  // queries handed to prim_heavy_kernel (nullptr: none are)
   unsigned heavy_cap;       // the most that fit
   unsigned* heavy_ctr;      // their count (it may pass heavy_cap), and the next to take
 };
@@ -228,7 +230,7 @@ struct PrimState {
   float kt;  // last visited key (entry, index)
   int ke;
 };
-// A query handed to the warp-per-query kernel.
+// A query handed to prim_heavy_kernel.
 struct PrimHeavy {
   int32_t q;
   uint32_t iters;
@@ -237,7 +239,7 @@ struct PrimHeavy {
 // Iterations after which a query is handed over. A quad's or a triangle's
 // start search takes 1,000 to 4,000 iterations when it finds nothing; on one
 // thread a ray that passes several such surfaces ran for hundreds of
-// milliseconds after the others had ended.
+// milliseconds after the others had ended. (32, 96 and 1,024 measure within 2%.)
 constexpr uint32_t kPrimBudget = 256;
 // Most queries handed over in a call (40 bytes each); the others run to their
 // end where they are.
@@ -290,16 +292,24 @@ __device__ __forceinline__ void prim_finish(const PrimParams& P, int64_t q, floa
   }
 }
 
+// The j-th of a walk's candidates, from registers.
+__device__ __forceinline__ void walk_entry(const float (&bt)[kPrimCandK], const int (&be)[kPrimCandK], int j, float& ct,
+                                           int& ce) {
+  ct = bt[0];
+  ce = be[0];
+#pragma unroll
+  for (int m = 1; m < kPrimCandK; ++m)
+    if (j == m) {
+      ct = bt[m];
+      ce = be[m];
+    }
+}
+
 // The candidates of a query in (box entry, index) order on [0.001, closest hit
-// so far], from where its walk stands. One thread's form (W = false) hands
-// over after kPrimBudget iterations when it may (returns false, with the place
-// in the list); a warp's form
-// (all lanes with the same arguments; wu: the work that all lanes repeat) runs
-// to the end.
-template <bool W>
+// so far], from where its walk stands. Hands over after kPrimBudget iterations
+// when there is room (returns false, with the place in the list).
 __device__ __forceinline__ bool prim_walk(const PrimParams& P, float3 o, float3 d, PrimState& s, PrimWork& pw,
-                                          PrimWork& wu, unsigned& cand, Work& w, bool& incomplete,
-                                          unsigned* place = nullptr) {
+                                          unsigned& cand, Work& w, bool& incomplete, unsigned& place) {
   const uint32_t iters0 = pw.iters;
   bool asked = false;
   for (;;) {
@@ -307,49 +317,35 @@ __device__ __forceinline__ bool prim_walk(const PrimParams& P, float3 o, float3 
     int be[kPrimCandK];
     bool overflow;
     if (!collect_in<kPrimCandK>(P.nodes, o, d, s.best, s.kt, s.ke, bt, be, overflow, w, PrimKeep{P, o, d, s.best})) {
-      if (!W || (threadIdx.x & 31) == 0) atomicOr(&P.stats->status, kStatusStackOverflow);
+      atomicOr(&P.stats->status, kStatusStackOverflow);
       incomplete = true;
       return true;
     }
     bool done = false;
 #pragma unroll 1
     for (int j = 0; j < kPrimCandK; ++j) {
-      float ct = bt[0];
-      int ce = be[0];
-#pragma unroll
-      for (int m = 1; m < kPrimCandK; ++m)
-        if (j == m) {
-          ct = bt[m];
-          ce = be[m];
-        }
+      float ct;
+      int ce;
+      walk_entry(bt, be, j, ct, ce);
       if (ce == INT_MAX || ct > s.best) {
         done = true;
         break;
       }
-      if (!W && P.heavy && !asked && pw.iters - iters0 > kPrimBudget) {
+      if (P.heavy && !asked && pw.iters - iters0 > kPrimBudget) {
         asked = true;
-        *place = atomicAdd(P.heavy_ctr, 1u);
-        if (*place < P.heavy_cap) return false;
+        place = atomicAdd(P.heavy_ctr, 1u);
+        if (place < P.heavy_cap) return false;
       }
       const PrimRec& p = P.prims[ce];  // read in place: the solvers take it by reference
-      const PrimCull& c = P.cull[ce];
-      const float* start = P.start + 21 * static_cast<int64_t>(ce);
       float te, tx, th;
       float3 xh;
       ++cand;
-      if (pr_slab(o, d, p.lo, p.hi, 0.001f, s.best, te, tx)) {
-        bool hit;
-        if (W)
-          hit = p.kind == kPrimPrism ? pr_hit_prism_warp(p, c, start, P.geom, o, d, 0.001f, s.best, th, xh, pw)
-                                     : pr_hit_surface_warp(p, c, P.geom, o, d, 0.001f, s.best, th, xh, pw, wu);
-        else
-          hit = p.kind == kPrimPrism ? pr_hit_prism(p, c, start, P.geom, o, d, 0.001f, s.best, th, xh, pw)
-                                     : pr_hit_surface(p, c, P.geom, o, d, 0.001f, s.best, th, xh, pw);
-        if (hit && th > 0.001f && th < s.best) {
-          s.best = th;
-          s.win = ce;
-          s.x = xh;
-        }
+      if (pr_slab(o, d, p.lo, p.hi, 0.001f, s.best, te, tx) &&
+          pr_hit(p, P.cull[ce], P.start + 21 * static_cast<int64_t>(ce), P.geom, o, d, 0.001f, s.best, th, xh, pw) &&
+          th > 0.001f && th < s.best) {
+        s.best = th;
+        s.win = ce;
+        s.x = xh;
       }
       s.kt = ct;
       s.ke = ce;
@@ -359,7 +355,7 @@ __device__ __forceinline__ bool prim_walk(const PrimParams& P, float3 o, float3 
 }
 
 __global__ void __launch_bounds__(kPrimThreads, HO_PRIM_MIN_BLOCKS) prim_trace_kernel(PrimParams P) {
-  PrimWork pw, wu;
+  PrimWork pw;
   unsigned cand = 0;
   Work w;
   const int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -377,7 +373,7 @@ __global__ void __launch_bounds__(kPrimThreads, HO_PRIM_MIN_BLOCKS) prim_trace_k
     s.ke = -1;
     bool incomplete = false;
     unsigned place = 0;
-    if (prim_walk<false>(P, o, d, s, pw, wu, cand, w, incomplete, &place)) {
+    if (prim_walk(P, o, d, s, pw, cand, w, incomplete, place)) {
       prim_finish(P, q, d, h, s, pw.iters, incomplete);
     } else {
       PrimHeavy v;
@@ -403,42 +399,195 @@ __global__ void __launch_bounds__(kPrimThreads, HO_PRIM_MIN_BLOCKS) prim_trace_k
   }
 }
 
-// The handed-over queries, a warp each: the starts of a candidate's search run
-// on the lanes (the answer is the one that the loops would find). What bounds
-// it is the evaluation's chain of dependent FP32 operations; what it replaces
-// was bound by the longest query: a picture of 4,138 curved triangles ran
-// 454 ms on one thread a query.
-__global__ void __launch_bounds__(kPrimThreads) prim_heavy_kernel(PrimParams P) {
-  const int lane = threadIdx.x & 31;
-  const unsigned n = min(*P.heavy_ctr, P.heavy_cap);
-  PrimWork pw, wu;  // each lane's own, and what all lanes repeat
+__device__ __forceinline__ float3 shfl_f3(float3 v, int src) {
+  return make_float3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                     __shfl_sync(0xffffffffu, v.z, src));
+}
+
+// The handed-over queries: up to 16 per warp, a lane each, in rounds. In a
+// round every lane walks to its query's next candidate; prisms are solved lane
+// by lane; the start searches of the surface candidates, 36 to 108 independent
+// solves each, are dealt over all lanes, in order and packed (a query's success
+// with the lowest number is the start that the loops of pr_hit_surface would stop
+// at); the Newtons that follow run a lane each. A lane whose query has ended takes the
+// next; with few queries a warp takes fewer, so that all warps have some. What
+// bounds it is the issue rate of the searches' chains and their unequal lengths
+// (18 of at most 30 iterations on average, a pass takes its longest). 4,138
+// curved triangles at 960 x 540 ran 97 ms with a warp to each query, whose lanes
+// mostly waited (8 of 40 searches in a second pass, one lane's Newton on all);
+// 70 / 59 / 51 / 49 / 53 ms with 2 / 4 / 8 / 16 / 32 queries a warp. Six or eight
+// blocks an SM with fewer registers: 59 and 60 ms.
+__global__ void __launch_bounds__(kPrimThreads, 4) prim_heavy_kernel(PrimParams P) {
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ unsigned spent[kPrimThreads];  // iterations for the lane's query
+  const int lane = threadIdx.x & 31, first = threadIdx.x & ~31;
+  const unsigned n = min(*P.heavy_ctr, P.heavy_cap), warps = gridDim.x * (kPrimThreads / 32);
+  const int width = static_cast<int>(min(16u, (n + warps - 1u) / warps));
+  PrimWork pw;
   unsigned cand = 0;
   Work w;
+  bool have = false, drained = lane >= width, overflow = true, incomplete = false;
+  PrimHeavy v;
+  float3 o = make_float3(0.f, 0.f, 0.f), d = o;
+  float bt[kPrimCandK];
+  int be[kPrimCandK], at = kPrimCandK;
   for (;;) {
-    unsigned k = 0;
-    if (lane == 0) k = atomicAdd(P.heavy_ctr + 1, 1u);
-    k = __shfl_sync(0xffffffffu, k, 0);
-    if (k >= n) break;
-    const PrimHeavy v = P.heavy[k];
-    float3 o, d;
-    float iso;
-    bool iso_on;
-    query_ray_from(P.rays, P.n_rays, P.cam, P.iso, P.iso_mask, P.views, P.n_views, v.q, o, d, iso, iso_on);
-    PrimState s = v.s;
-    bool incomplete = false;
-    const uint32_t lane0 = pw.iters, all0 = wu.iters;
-    prim_walk<true>(P, o, d, s, pw, wu, cand, w, incomplete);
-    const uint32_t its = __reduce_add_sync(0xffffffffu, pw.iters - lane0) + wu.iters - all0;
-    if (lane == 0) prim_finish(P, v.q, d, prim_base(P, v.q), s, v.iters + its, incomplete);
+    if (!have && !drained) {
+      const unsigned k = atomicAdd(P.heavy_ctr + 1, 1u);
+      if (k < n) {
+        v = P.heavy[k];
+        float iso;
+        bool iso_on;
+        query_ray_from(P.rays, P.n_rays, P.cam, P.iso, P.iso_mask, P.views, P.n_views, v.q, o, d, iso, iso_on);
+        have = overflow = true;
+        incomplete = false;
+        at = kPrimCandK;
+        spent[threadIdx.x] = v.iters;
+      } else {
+        drained = true;
+      }
+    }
+    if (!__any_sync(kAll, have)) break;
+    // -- the query's next candidate, or its end
+    int ce = -1;
+    bool surface = false;
+    float enter = 0.f, exit = 0.f;
+    if (have) {
+      PrimState& s = v.s;
+      bool end = false;
+      while (ce < 0 && !end) {
+        if (at == kPrimCandK) {
+          if (!overflow) break;
+          if (!collect_in<kPrimCandK>(P.nodes, o, d, s.best, s.kt, s.ke, bt, be, overflow, w,
+                                      PrimKeep{P, o, d, s.best})) {
+            atomicOr(&P.stats->status, kStatusStackOverflow);
+            incomplete = end = true;
+            break;
+          }
+          at = 0;
+        }
+        float ct;
+        int e;
+        walk_entry(bt, be, at, ct, e);
+        if (e == INT_MAX || ct > s.best) {
+          end = true;
+          break;
+        }
+        ++at;
+        ++cand;
+        s.kt = ct;
+        s.ke = e;
+        const PrimRec& p = P.prims[e];
+        if (pr_slab(o, d, p.lo, p.hi, 0.001f, s.best, enter, exit) &&
+            (p.kind == kPrimPrism || pr_may_hit(P.cull[e], o, d, 0.001f, s.best, kPrimTol))) {
+          ce = e;
+          surface = p.kind != kPrimPrism;
+        }
+      }
+      if (ce < 0) {
+        prim_finish(P, v.q, d, prim_base(P, v.q), s, spent[threadIdx.x], incomplete);
+        have = false;
+      }
+    }
+    __syncwarp();
+    bool hit = false;
+    float th = 0.f;
+    float3 xh = make_float3(0.f, 0.f, 0.f);
+    const uint32_t own = pw.iters;
+    if (ce >= 0 && !surface)
+      hit = pr_hit_prism(P.prims[ce], P.cull[ce], P.start + 21 * static_cast<int64_t>(ce), P.geom, o, d, 0.001f, v.s.best,
+                         th, xh, pw);
+    __syncwarp();
+    // -- the surfaces' start searches
+    int base = 0, total = 0;
+    bool started = false;
+    float r = 0.f, t = 0.f;
+    if (surface) {
+      const bool quad = P.prims[ce].kind == kPrimQuad;
+      float3 plane;
+      total = (quad ? 99 : 36) + (pr_plane_point(P.prims[ce], o, d, enter, exit, plane) ? (quad ? 9 : 4) : 0);
+    }
+    const uint32_t before = pw.iters;
+    if (ce >= 0) atomicAdd(&spent[threadIdx.x], before - own);
+    for (;;) {
+      const int rem = total - base;
+      int incl = rem;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int x = __shfl_up_sync(kAll, incl, off);
+        if (lane >= off) incl += x;
+      }
+      const int all = __shfl_sync(kAll, incl, 31);
+      if (all == 0) break;
+      const int excl = incl - rem;
+      int q = 0;  // the query of this lane's solve: the first whose solves go past the lane
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(kAll, incl, q + step - 1) <= lane) q += step;
+      const int k = __shfl_sync(kAll, base, q) + lane - __shfl_sync(kAll, excl, q);
+      const int e = __shfl_sync(kAll, ce, q);
+      const float3 qo = shfl_f3(o, q), qd = shfl_f3(d, q);
+      const float qen = __shfl_sync(kAll, enter, q), qex = __shfl_sync(kAll, exit, q);
+      bool ok = false;
+      float rr = 0.f, ss = 0.f;
+      PrimWork job;
+      if (lane < all) {
+        const PrimRec& p = P.prims[e];
+        const bool quad = p.kind == kPrimQuad;
+        const int starts = quad ? 9 : 4, points = quad ? 11 : 9;
+        float3 x;
+        if (k < points * starts) x = pr_segment_point(qo, qd, qen, qex, k / starts, points - 1);
+        else pr_plane_point(p, qo, qd, qen, qex, x);
+        if (!quad || pr_near(P.cull[e], x, kPrimNear)) {
+          ok = pr_project(p, P.geom, x, k % starts, rr, ss, job) && pr_on_surface(p, P.geom, x, rr, ss, job);
+        }
+      }
+      __syncwarp();
+      const unsigned m = __ballot_sync(kAll, ok);
+      const int hi = min(incl, 32);
+      const bool mine = rem > 0 && excl < 32;
+      const unsigned f = mine ? m & (kAll >> (32 - hi)) & (kAll << excl) : 0u;
+      const int src = f ? __ffs(f) - 1 : 0;
+      const float r1 = __shfl_sync(kAll, rr, src), s1 = __shfl_sync(kAll, ss, src);
+      // counted are the solves up to the success, whatever ran beside them
+      const unsigned fq = __shfl_sync(kAll, f, q);
+      if (job.iters && (fq == 0u || lane < __ffs(fq))) {
+        pw.iters += job.iters;
+        pw.flops += job.flops;
+        atomicAdd(&spent[first + q], job.iters);
+      }
+      if (f) {
+        started = true;
+        r = r1;
+        t = s1;
+        base = total;
+      } else if (mine) {
+        base += hi - excl;
+      }
+    }
+    // -- their Newtons
+    if (surface) {
+      const PrimRec& p = P.prims[ce];
+      const float2 rs = make_float2(r, t);
+      t = 0.5f * (enter + exit);
+      if (started || p.kind != kPrimQuad) t = pr_param(o, d, pr_point(p, P.geom, make_float3(rs.x, rs.y, 0.f)));
+      const uint32_t it0 = pw.iters;
+      hit = pr_surface_newton(p, P.geom, o, d, 0.001f, v.s.best, rs.x, rs.y, t, th, xh, pw);
+      atomicAdd(&spent[threadIdx.x], pw.iters - it0);
+    }
+    if (hit && th > 0.001f && th < v.s.best) {
+      v.s.best = th;
+      v.s.win = ce;
+      v.s.x = xh;
+    }
     __syncwarp();
   }
-  const unsigned long long v[4] = {lane == 0 ? cand : 0u, pw.iters + (lane == 0 ? wu.iters : 0u),
-                                   pw.flops + (lane == 0 ? wu.flops : 0ull), lane == 0 ? w.nodes : 0u};
+  const unsigned long long c[4] = {cand, pw.iters, pw.flops, w.nodes};
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    unsigned long long x = v[k];
+    unsigned long long x = c[k];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(kAll, x, off);
     if (lane == 0 && x) atomicAdd(&P.stats->c[ST_PRIM_CAND + k], x);
   }
 }
@@ -621,7 +770,7 @@ int launch_prims(ho_context* c, const TraceArgs& a, ho_hit* hits, bool fresh, De
     PR_TRY(cudaGetDevice(&dev));
     PR_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t most = (P.n_queries * 32 + kPrimThreads - 1) / kPrimThreads;
-    prim_heavy_kernel<<<static_cast<unsigned>(std::min<int64_t>(most, sms * 8)), kPrimThreads, 0, s>>>(P);
+    prim_heavy_kernel<<<static_cast<unsigned>(std::min<int64_t>(most, sms * 4)), kPrimThreads, 0, s>>>(P);
     PR_TRY(cudaGetLastError());
     PR_TRY(cudaEventRecord(c->pheavy_done, s));
     ++c->launches;

@@ -651,27 +651,6 @@ __device__ __noinline__ bool pr_hit_prism(const PrimRec& p, const PrimCull& c, c
   return false;
 }
 
-// The same by a warp: a lane per start, the first that succeeds.
-__device__ __noinline__ bool pr_hit_prism_warp(const PrimRec& p, const PrimCull& c, const float* __restrict__ start,
-                                               const float* __restrict__ pool, float3 o, float3 d, float tmin,
-                                               float tmax, float& th, float3& xh, PrimWork& w) {
-  float enter, exit;
-  if (!pr_slab(o, d, p.lo, p.hi, tmin, tmax, enter, exit) || !pr_may_hit(c, o, d, enter, exit, kPrimTol)) return false;
-  const int lane = threadIdx.x & 31;
-  float t = 0.f;
-  float3 x = make_float3(0.f, 0.f, 0.f);
-  const bool ok = lane < 7 && pr_prism_solve(p, start, pool, o, d, enter, exit, lane, t, x, w);
-  __syncwarp();
-  const unsigned m = __ballot_sync(0xffffffffu, ok);
-  if (!m) return false;
-  const int src = __ffs(m) - 1;
-  th = __shfl_sync(0xffffffffu, t, src);
-  xh.x = __shfl_sync(0xffffffffu, x.x, src);
-  xh.y = __shfl_sync(0xffffffffu, x.y, src);
-  xh.z = __shfl_sync(0xffffffffu, x.z, src);
-  return true;
-}
-
 // Can any start of a prism begin on the segment [tmin, tmax] of its box? If
 // not, its solver ends without a hit, on any shorter segment too.
 __device__ inline bool pr_prism_begins(const PrimRec& p, const float* __restrict__ start, float3 o, float3 d, float tmin,
@@ -846,44 +825,6 @@ __device__ __noinline__ bool pr_hit_surface(const PrimRec& p, const PrimCull& bo
   }
   if (started || !quad) t = pr_param(o, d, pr_point(p, pool, make_float3(r, s, 0.f)));
   return pr_surface_newton(p, pool, o, d, tmin, tmax, r, s, t, th, xh, w);
-}
-
-// The same by a warp, all lanes with the same arguments: the points' starts
-// are independent, so they run 32 at a time on the lanes, and the first in the
-// order above that succeeds is the one that the loops would stop at.
-__device__ __noinline__ bool pr_hit_surface_warp(const PrimRec& p, const PrimCull& bounds,
-                                                 const float* __restrict__ pool, float3 o, float3 d, float tmin,
-                                                 float tmax, float& th, float3& xh, PrimWork& w, PrimWork& wu) {
-  float enter, exit;
-  if (!pr_slab(o, d, p.lo, p.hi, tmin, tmax, enter, exit) || !pr_may_hit(bounds, o, d, tmin, tmax, kPrimTol)) return false;
-  const int lane = threadIdx.x & 31;
-  const bool quad = p.kind == kPrimQuad;
-  const int n = quad ? 10 : 8, starts = quad ? 9 : 4, all = (n + 1) * starts;
-  float t = 0.5f * (enter + exit), r = 0.f, s = 0.f;
-  bool started = false;
-  float3 plane;
-  const bool test = pr_plane_point(p, o, d, enter, exit, plane);
-  // the plane point's starts come last
-  for (int base = 0; base < all + (test ? starts : 0) && !started; base += 32) {
-    const int k = base + lane;
-    bool ok = false;
-    float rr = 0.f, ss = 0.f;
-    if (k < all + (test ? starts : 0)) {
-      const float3 q = k < all ? pr_segment_point(o, d, enter, exit, k / starts, n) : plane;
-      if (!quad || pr_near(bounds, q, kPrimNear))
-        ok = pr_project(p, pool, q, k % starts, rr, ss, w) && pr_on_surface(p, pool, q, rr, ss, w);
-    }
-    __syncwarp();
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (m) {
-      const int src = __ffs(m) - 1;
-      r = __shfl_sync(0xffffffffu, rr, src);
-      s = __shfl_sync(0xffffffffu, ss, src);
-      started = true;
-    }
-  }
-  if (started || !quad) t = pr_param(o, d, pr_point(p, pool, make_float3(r, s, 0.f)));
-  return pr_surface_newton(p, pool, o, d, tmin, tmax, r, s, t, th, xh, wu);
 }
 
 __device__ inline bool pr_hit(const PrimRec& p, const PrimCull& c, const float* __restrict__ start,

@@ -39,7 +39,7 @@ static_assert(sizeof(PrimRec) == 128, "PrimRec is two 64-byte lines");
 // costs up to 420 (prism) or 4,000 (surface) iterations, against 30 operations
 // here. size < 0: no bounds (a curved triangle accepts any (r, s); a degenerate
 // or non-finite primitive). With the prisms' kept starts and the hand-over to
-// warps (ho_prim.cu), a 960 x 540 picture of 12,000 primitives went from 630 to
+// warps (ho_prim.cu), a 960 x 540 picture of 14,336 primitives went from 630 to
 // 320 ms.
 struct alignas(16) PrimCull {
   float m[9], lo[3], hi[3];
@@ -239,7 +239,7 @@ __device__ __noinline__ void pr_modal_geom(const PrimRec& p, const float* __rest
 // the basis values stay in registers, the recurrences' constants are folded
 // and independent terms overlap. The solvers are chains of these evaluations,
 // and the general form above keeps its basis values in indexed local arrays: a
-// 960 x 540 picture of 12,000 prisms, quads and curved triangles took 320 ms
+// 960 x 540 picture of 14,336 prisms, quads and curved triangles took 320 ms
 // with it and 145 ms with this. Above 5 modes a prism's unrolled code (126
 // coefficients a component at 6) would not pay for its size.
 template <int Kind, int M>

@@ -315,7 +315,7 @@ constexpr unsigned kSpreadPerSm = 16;
 // are fed by a batch's pairs, so a full batch keeps them busiest; but a round
 // that cannot fill the device lasts as long as its longest batch, and a batch of
 // one or two pairs, with the warp to itself, is several times shorter. Calls
-// before (full batches only) and after: 1,024 rays 1.81 -> 1.18 ms, a 256 x 256
+// before (full batches only) and after: 777 rays 1.81 -> 1.18 ms, a 256 x 256
 // picture 3.5 -> 2.5 ms, four path bounces 14.4 -> 12.7 ms; 4 or more batches a
 // resident warp change nothing (1920 x 1080: 15.3 ms either way); 64 an SM:
 // 2.6 ms and 13.0 ms for the second and third.

@@ -329,8 +329,10 @@ __device__ __forceinline__ bool polish_step(const HitState& h, float3 d, float i
 
 // The FP64 check of a hit (a miss always passes) and, when it passes, the
 // polish (file header). Returns whether the hit passed; polished is set when
-// the hit's t, xi and u were refined.
-template <int N>
+// the hit's t, xi and u were refined. F: face hits by the face's own sums (the
+// element's give the same values), and hits without their normal and field value
+// (kFlagPost) are completed.
+template <int N, bool F = true>
 __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint32_t* __restrict__ eflags, float3 o,
                                   float3 d, float iso, HitState& h, bool& polished, double* t64 = nullptr) {
   polished = false;
@@ -340,15 +342,20 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
   const bool has_field = iso_hit || (__ldg(eflags + h.elem) & 1u) != 0;
   // a face hit's fixed coordinate is exactly -1 or 1, and the polish keeps it
   bool on_face = false;
-  if (!iso_hit) {
+  if (F && !iso_hit) {
     int fixed, ua, va;
     float val;
     face_param(h.face, fixed, val, ua, va);
     on_face = getc(h.xi, fixed) == val;
   }
   const auto residual = [&](double t, double x0, double x1, double x2, double (&r)[3], double& u) {
-    if (on_face) fp64_face_residual<N>(rec_all, h.elem, h.face, o, d, t, x0, x1, x2, has_field, r, u);
-    else fp64_residual_vec<N>(rec_all, h.elem, o, d, t, x0, x1, x2, has_field, r, u);
+    if constexpr (F) {
+      if (on_face) {
+        fp64_face_residual<N>(rec_all, h.elem, h.face, o, d, t, x0, x1, x2, has_field, r, u);
+        return;
+      }
+    }
+    fp64_residual_vec<N>(rec_all, h.elem, o, d, t, x0, x1, x2, has_field, r, u);
   };
   double r[3], u;
   residual(h.t, h.xi.x, h.xi.y, h.xi.z, r, u);
@@ -364,7 +371,7 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
   float3 g = make_float3(0.f, 0.f, 0.f);
   float u32 = 0.f;
   auto jacobian_at = [&](float3 xi) {
-    if (on_face) {  // the two tangents and the field's derivatives along them: all that a face hit's steps use
+    if (F && on_face) {  // the two tangents and the field's derivatives along them: all that a face hit's steps use
       int fixed, ua, va;
       float val;
       face_param(h.face, fixed, val, ua, va);
@@ -395,7 +402,7 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
     }
   };
   jacobian_at(h.xi);
-  if (h.flags & kFlagPost) {
+  if (F && (h.flags & kFlagPost)) {
     if (on_face && !normal_on_face(h.face, h.xi)) {  // near another face's edge the normal takes the third column
       float xJ[12];
       geom_eval_raw<N, false>(c, h.xi, xJ);
@@ -452,13 +459,13 @@ __device__ bool fp64_check_polish(const float* __restrict__ rec_all, const uint3
 // an edge), the lower element index, then the lower face index. Returns true
 // when the partner replaced the best hit (flags carried over); the answer
 // carries HO_FLAG_TIE either way.
-template <int N>
+template <int N, bool F = true>
 __device__ __noinline__ bool fp64_tie_rule(const float* __restrict__ rec_all, const uint32_t* __restrict__ eflags, float3 o,
                               float3 d, float iso, HitState& best, double t_best, HitState tie) {
   best.flags |= HO_FLAG_TIE;
   bool polished;
   double t_tie;
-  if (!fp64_check_polish<N>(rec_all, eflags, o, d, iso, tie, polished, &t_tie)) return false;
+  if (!fp64_check_polish<N, F>(rec_all, eflags, o, d, iso, tie, polished, &t_tie)) return false;
   const double eps = 1e-7 * fmax(1.0, fabs(t_best));
   bool wins;
   if (t_tie < t_best - eps) wins = true;

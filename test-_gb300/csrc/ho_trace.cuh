@@ -497,6 +497,16 @@ __device__ HitState plain_trace(const TraceParams& P, float3 o, float3 d, float 
   return best;
 }
 
+// Does the plain form check face hits by the face's own sums (fp64_check_polish)?
+// Both forms give the same hits. The face's needs 1 / N of the operations, but it
+// adds a second copy of the sums to a kernel that is out of registers: its stack
+// frame grows by 112 bytes, and whether that costs more than the sums save was
+// measured per order. 24^3 elements, two 960 x 540 pictures, ms with the
+// element's and with the face's sums: 27.3 / 24.2 at 2 modes, 39.1 / 39.1, 54.9 /
+// 55.7, 101.1 / 98.6, 134.5 / 142.8 at 6, 225.7 / 217.1, 293.7 / 283.9, 558 / 583
+// at 9; hex64_p5 283 / 301, hex48_mixed 1,450 / 1,530 (three pictures).
+constexpr bool plain_face_check(int n) { return n != 6 && n != 9; }
+
 // Plain form: the reference's structure on the GPU — one thread per query
 // (camera rays: a warp covers an 8x4 pixel tile), no queue, no lane-parallel
 // solves, no prediction.
@@ -534,11 +544,11 @@ __global__ void __launch_bounds__(kTraceBlock) plain_kernel(TraceParams P, int64
     // plain solver is the fallback itself, so a failing hit is only flagged
     if (P.fp64) {
       double t64;
-      if (!fp64_check_polish<N>(P.rec, P.flags, o, d, iso, best, polished, &t64)) {
+      if (!fp64_check_polish<N, plain_face_check(N)>(P.rec, P.flags, o, d, iso, best, polished, &t64)) {
         best.flags |= HO_FLAG_FP64_FAIL;
       } else if (tie.kind != HO_HIT_MISS) {
         tie_seen = 1;
-        tie_swapped = fp64_tie_rule<N>(P.rec, P.flags, o, d, iso, best, t64, tie) ? 1 : 0;
+        tie_swapped = fp64_tie_rule<N, plain_face_check(N)>(P.rec, P.flags, o, d, iso, best, t64, tie) ? 1 : 0;
       }
     }
   }

@@ -376,13 +376,16 @@ int ho_set_mode(ho_context* ctx, int mode);
  *                     (HO_FLAG_TIE, ho_stats.fp64_ties). 0: off (the
  *                     solvers' own answers).
  * HO_OPT_ROUND_CHUNK  pairs per element batch of the round kernel (1..4096).
- *                     Unset: at most the kernel's pair slots (20 per warp up
- *                     to 7 modes per direction, 12 at 8, 8 at 9, times 4 warps
- *                     in the tensor-core form: the value that ho_get_option
- *                     gives; 32 for face searches on elements with a
- *                     convergence certificate), fewer while a round has too
- *                     few pairs to give 16 warps of every SM a batch;
- *                     ho_autotune picks a fixed one.
+ *                     Unset, or set to the value that ho_get_option gives
+ *                     while unset (the kernel's pair slots at the scene's
+ *                     largest order: 20 per warp up to 7 modes per direction,
+ *                     12 at 8, 8 at 9, times 4 warps in the tensor-core
+ *                     form): at most the pair slots of each element's order
+ *                     (32, 22 and 14 for face searches on elements with a
+ *                     convergence certificate), in batched mode fewer while
+ *                     a round has too few pairs to give 16 warps of every SM
+ *                     a batch. Any other value is a fixed size for every
+ *                     order and round; ho_autotune may pick one.
  * HO_OPT_TENSOR      0 (default): the FP32 CUDA-core round kernel for every
  *                     order; 1: elements of up to 8 modes per direction are
  *                     intersected by the tensor-core round kernel (tcgen05
@@ -457,9 +460,10 @@ int ho_get_option(ho_context* ctx, int option, int64_t* value);
 /* Autotuner of the batched / learned engine (no reference counterpart): times
  * the given render (device buffers only, CUDA events on the context's stream,
  * one warm-up and one timed call per candidate) for HO_AUTOTUNE_N element
- * batch sizes (0.5, 1, 2, 4 and 8 times the kernel's pair slots), keeps the
- * fastest as HO_OPT_ROUND_CHUNK and returns it in *chunk_out; ms_out (may be
- * NULL) receives the candidates' times. Uses the current mode. */
+ * batch sizes (0.5, 1, 2, 4 and 8 times the kernel's pair slots; 1 is the
+ * unset option's rule), keeps the fastest as HO_OPT_ROUND_CHUNK, where a fixed
+ * size has to be over 2% faster than the rule, and returns it in *chunk_out;
+ * ms_out (may be NULL) receives the candidates' times. Uses the current mode. */
 #define HO_AUTOTUNE_N 5
 int ho_autotune(ho_context* ctx, const ho_camera* cam, const float* isovalues, int n_iso, int width, int height,
                 int iso_zero_disables, int64_t* chunk_out, int64_t* candidates_out, float* ms_out);

@@ -1046,7 +1046,7 @@ int ho_autotune(ho_context* c, const ho_camera* cam, const float* iso, int n_iso
   CK(cudaEventCreate(&ev0), "cudaEventCreate");
   CK(cudaEventCreate(&ev1), "cudaEventCreate");
   const int keep = c->round_chunk;
-  float best_ms = 0.f;
+  float best_ms = 0.f, rule_ms = 0.f;
   int64_t best = keep;
   for (int k = 0; k < HO_AUTOTUNE_N && rc == HO_OK; ++k) {
     c->round_chunk = static_cast<int>(cand[k]);
@@ -1063,11 +1063,15 @@ int ho_autotune(ho_context* c, const ho_camera* cam, const float* iso, int n_iso
     if (rc != HO_OK) break;
     if (ms_out) ms_out[k] = ms;
     if (candidates_out) candidates_out[k] = cand[k];
+    if (cand[k] == slots) rule_ms = ms;
     if (k == 0 || ms < best_ms) {
       best_ms = ms;
       best = cand[k];
     }
   }
+  // the slots' candidate is the unset option's rule, which smaller calls need
+  // too: a fixed size has to beat it by more than two timings of one differ
+  if (rule_ms <= 1.02f * best_ms) best = slots;
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
   c->round_chunk = rc == HO_OK ? static_cast<int>(best) : keep;

@@ -232,7 +232,7 @@ struct ho_context {
   cudaEvent_t check_fork = nullptr, check_done = nullptr;
   cudaEvent_t order_fork = nullptr, order_done[ho::kMaxModes + 1] = {};
   // batched / learned engine options (ho_set_option)
-  int round_chunk = 0;       // pairs per element batch (0: the kernel's pair slots)
+  int round_chunk = 0;       // pairs per element batch (0 or the kernel's pair slots: by each round's pairs)
   int warm_cap = 4;          // round kernel: iterations of a warm-started solve before its cold restart
   int round_count = 16;      // rounds enqueued before the completion check (at most)
   int tail_after = 4;        // rounds before the warp-per-ray tail finishes every ray (0: no tail)

@@ -310,7 +310,14 @@ constexpr int kCtrOrderNb = 16, kCtrOrderOff = 26, kCtrOrderCur = 36, kCtrOrderN
 
 // Batches per SM that a round's pairs are spread over, before batches grow.
 constexpr unsigned kSpreadPerSm = 16;
-// Pairs per batch of a key: HO_OPT_ROUND_CHUNK, else the slots, or fewer while
+// HO_OPT_ROUND_CHUNK where it asks for a fixed batch size, else 0. The size that
+// the option reports while unset asks for the rule below, so that a program that
+// puts an option's value back, or the autotuner when no fixed size is faster,
+// does not take the rule from later, smaller calls.
+static int fixed_chunk(const ho_context* c) {
+  return c->round_chunk == round_batch_default(c->N, c->use_tc) ? 0 : c->round_chunk;
+}
+// Pairs per batch of a key: the fixed size, else the slots, or fewer while
 // the round has less than `spread` full batches (16 warps an SM). A warp's lanes
 // are fed by a batch's pairs, so a full batch keeps them busiest; but a round
 // that cannot fill the device lasts as long as its longest batch, and a batch of
@@ -629,9 +636,10 @@ static int enqueue_round(ho_context* c, const TraceParams& P, const RoundParams&
   // with the network's predictions, a solve's restarts depend on what else its
   // warp runs: full batches for every call size
   const unsigned spread = learned ? 1u : kSpreadPerSm * static_cast<unsigned>(sm_count());
-  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread, rb.ctr);
+  const int chunk = fixed_chunk(c);
+  round_batch_count_kernel<<<ge, 256, 0, s>>>(rb.kcount, c->d_cord, c->d_cull, n_elem, chunk, c->use_tc, spread, rb.ctr);
   round_order_offsets_kernel<<<1, 1, 0, s>>>(rb.ctr);
-  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, c->round_chunk, c->use_tc, spread,
+  round_batch_kernel<<<ge, 256, 0, s>>>(rb.kcount, rb.koff, c->d_cord, c->d_cull, n_elem, chunk, c->use_tc, spread,
                                         const_cast<RoundBatch*>(R.batches), rb.ctr);
   RT_TRY(cudaGetLastError());
   c->launches += 7 + __builtin_popcount(c->orders);

@@ -545,8 +545,8 @@ __device__ inline bool pr_may_hit(const PrimCull& c, float3 o, float3 d, float t
     const float w = slack * (fabsf(mx) + fabsf(my) + fabsf(mz));
     const float a = mx * o.x + my * o.y + mz * o.z, b = mx * d.x + my * d.y + mz * d.z;
     const float lo = c.lo[k] - w - a, hi = c.hi[k] + w - a;
-    if (fabsf(b) < 1e-20f) {
-      if (lo > 0.f || hi < 0.f) return false;
+    if (fabsf(b) < FLT_MIN) {  // parallel, or 1 / b may not be finite (a short direction goes with a large t)
+      if (b == 0.f && (lo > 0.f || hi < 0.f)) return false;
       continue;
     }
     const float inv = 1.0f / b, t0 = lo * inv, t1 = hi * inv;

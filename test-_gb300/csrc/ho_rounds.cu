@@ -392,9 +392,9 @@ __global__ void round_batch_kernel(const uint32_t* __restrict__ kcount, const ui
   }
 }
 
-// The queued rays' answers into the call's outputs; count: tally the grazing
-// hits (once per call: a second write-out after extra rounds does not).
-__global__ void round_finish_kernel(TraceParams P, const RayState* __restrict__ st, bool count) {
+// The queued rays' answers into the call's outputs, and the count of the grazing
+// hits.
+__global__ void round_finish_kernel(TraceParams P, const RayState* __restrict__ st) {
   const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= *P.qcount) return;
   const int64_t q = P.work[item];
@@ -404,12 +404,10 @@ __global__ void round_finish_kernel(TraceParams P, const RayState* __restrict__ 
   query_ray(P, q, o, d, iso, iso_on);
   const HitState& b = st[item].best;
   write_result(P, q, d, b, static_cast<uint32_t>(st[item].its));
-  if (count) {
-    const unsigned act = __activemask();
-    const unsigned g = __ballot_sync(act, is_grazing(b, d));
-    if (g && static_cast<int>(threadIdx.x & 31) == __ffs(act) - 1)
-      atomicAdd(&P.stats->c[ST_GRAZING], static_cast<unsigned long long>(__popc(g)));
-  }
+  const unsigned act = __activemask();
+  const unsigned g = __ballot_sync(act, is_grazing(b, d));
+  if (g && static_cast<int>(threadIdx.x & 31) == __ffs(act) - 1)
+    atomicAdd(&P.stats->c[ST_GRAZING], static_cast<unsigned long long>(__popc(g)));
 }
 
 // Grow-only device buffer of `want` elements of `size` bytes.
@@ -734,8 +732,9 @@ static int enqueue_tail_and_check(ho_context* c, const TraceParams& P, const Rou
   return 0;
 }
 
-// The state init, `rounds` rounds (then the tail, when on) and the final
-// write-out of the queued rays.
+// The state init and `rounds` rounds, then, with the tail, the tail, the check
+// and the final write-out of the queued rays. Without it rays may still be in
+// flight after the rounds, and finish_rounds ends the call.
 int enqueue_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool learned, int64_t n_cap, int rounds) {
   const RoundParams R = round_params(c, P);
   const unsigned gi = static_cast<unsigned>((n_cap + 255) / 256);
@@ -748,19 +747,21 @@ int enqueue_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool lea
     const int rc = enqueue_round(c, P, R, s, learned, n_cap, c->tail_after > 0 ? rounds : 0);
     if (rc) return rc;
   }
-  const int rc = c->tail_after > 0 ? enqueue_tail_and_check(c, P, R, s, learned, n_cap)
-                                   : enqueue_check_all(c, P, R, s, n_cap);
+  if (c->tail_after == 0) return 0;
+  const int rc = enqueue_tail_and_check(c, P, R, s, learned, n_cap);
   if (rc) return rc;
-  round_finish_kernel<<<gi, 256, 0, s>>>(P, R.state, true);
+  round_finish_kernel<<<gi, 256, 0, s>>>(P, R.state);
   RT_TRY(cudaGetLastError());
   return 0;
 }
 
-// After the enqueued rounds ran: while the last round still found pairs, run
-// one more round (with a read-back each), then write the results again.
+// After the enqueued rounds ran: without the tail, one more round while the last
+// one still found pairs (with a read-back each), then the check and the final
+// write-out. The check polishes a ray's hit, and a ray in flight compares its
+// next candidates with that hit, so no ray is checked before all are done: its
+// answer would depend on how many rounds the call before had needed.
 int finish_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool learned, int64_t n_cap) {
   const RoundParams R = round_params(c, P);
-  bool extra = false;
   for (int guard = 0; guard < 100000; ++guard) {
     unsigned last = 0;
     unsigned long long rounds = 0;
@@ -769,17 +770,14 @@ int finish_rounds(ho_context* c, const TraceParams& P, cudaStream_t s, bool lear
     RT_TRY(cudaStreamSynchronize(s));
     c->rounds_needed = static_cast<int>(rounds);
     if (last == 0) break;
-    extra = true;
     const int rc = enqueue_round(c, P, R, s, learned, n_cap, 0);
     if (rc) return rc;
   }
-  if (extra) {
-    const int rc = enqueue_check_all(c, P, R, s, n_cap);
-    if (rc) return rc;
-    round_finish_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P, R.state, false);
-    RT_TRY(cudaGetLastError());
-    ++c->launches;
-  }
+  if (c->tail_after > 0) return 0;
+  const int rc = enqueue_check_all(c, P, R, s, n_cap);
+  if (rc) return rc;
+  round_finish_kernel<<<static_cast<unsigned>((n_cap + 255) / 256), 256, 0, s>>>(P, R.state);
+  RT_TRY(cudaGetLastError());
   return 0;
 }
 

@@ -416,6 +416,9 @@ int ho_set_mode(ho_context* ctx, int mode);
  *                     round's intersection launches (event nodes of the graph)
  *                     and ho_stats.round_kernel_ns / round_launches report
  *                     their device time.
+ * HO_OPT_CERTIFIED    (read only) hexahedra of the built scene that have a
+ *                     convergence certificate: their isosurface searches can
+ *                     be excluded and their face seeds run in stages.
  * HO_ERR_ARG for an unknown option, HO_ERR_RANGE for a value out of range. */
 #define HO_OPT_GRAPH 1
 #define HO_OPT_ROUNDS 2
@@ -427,6 +430,7 @@ int ho_set_mode(ho_context* ctx, int mode);
 #define HO_OPT_GPU_FIT 8
 #define HO_OPT_LAST_FIT_GPU 9
 #define HO_OPT_WARM_CAP 10
+#define HO_OPT_CERTIFIED 11
 int ho_set_option(ho_context* ctx, int option, int64_t value);
 /* Path tracing with Lambertian bounces (replaces: render_kernel at spp
  * samples and depth max_depth, FEM-AABB/raytracer.cu:410-476, with

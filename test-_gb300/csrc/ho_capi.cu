@@ -1011,6 +1011,19 @@ int ho_set_option(ho_context* c, int option, int64_t value) {
   }
 }
 
+// Elements of the built scene with a certificate (delta >= 0).
+static int certified_count(ho_context* c, int64_t* value) {
+  std::vector<float> delta(static_cast<size_t>(c->built ? c->n_elem : 0));
+  *value = 0;
+  if (delta.empty()) return HO_OK;
+  CK(cudaMemcpy2DAsync(delta.data(), sizeof(float), c->d_cull + 12, ho::kCullFloats * sizeof(float), sizeof(float),
+                       delta.size(), cudaMemcpyDeviceToHost, c->stream),
+     "read certificates");
+  CK(cudaStreamSynchronize(c->stream), "sync");
+  for (float d : delta) *value += d >= 0.f ? 1 : 0;
+  return HO_OK;
+}
+
 int ho_get_option(ho_context* c, int option, int64_t* value) {
   if (!c || !value) return HO_ERR_ARG;
   switch (option) {
@@ -1026,6 +1039,7 @@ int ho_get_option(ho_context* c, int option, int64_t* value) {
     case HO_OPT_ROUND_CHUNK:
       *value = c->round_chunk > 0 ? c->round_chunk : ho::round_batch_default(c->N > 0 ? c->N : 2, c->use_tc);
       return HO_OK;
+    case HO_OPT_CERTIFIED: return certified_count(c, value);
     default: return fail(c, HO_ERR_ARG, "unknown option " + std::to_string(option));
   }
 }

@@ -77,6 +77,10 @@ __device__ __forceinline__ void train_mma(const bf16* A, int lda, const bf16* B,
   }
 }
 
+// Columns of the FP32 sums that the rows' pass leaves per block and row half:
+// the bias gradients of the four layers, then the loss.
+constexpr int kSumCols = 3 * kMlpHidden + kMlpOut + 1;
+
 struct TrainArgs {
   const bf16* w[4];
   const float* b[4];
@@ -87,6 +91,8 @@ struct TrainArgs {
   const float* t;
   const uint8_t* valid;
   float* loss;
+  float* sums;  // [2 * row_blocks][kSumCols]
+  int row_blocks;
   int rows;
   float inv_n;
 };
@@ -96,7 +102,9 @@ struct TrainArgs {
 // every layer's gradient before its activation, with the weights in shared
 // memory and the activations' slopes in registers (a thread owns the same rows
 // and columns of every layer, forward and backward). Eight warps: 2 row halves
-// x 4 groups of 32 columns. Bias gradients are summed from the FP32 values.
+// x 4 groups of 32 columns. Bias gradients and the loss are summed from the FP32
+// values, a block's part of each kept apart and added up in a fixed order
+// (train_weights_kernel), so a call gives the same bits every time.
 // What bounds it is the chain of six small products and their barriers; the
 // products are 0.6 GFLOP at 4,096 rows. As separate launches per layer (product,
 // bias and activation, slope, column sums) the pass ran 28 kernels, 200 us at
@@ -116,7 +124,7 @@ __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
   for (int i = tid; i < kMlpHidden * kMlpOut; i += 256) S.w3[i / kMlpOut][i % kMlpOut] = __bfloat162float(P.w[3][i]);
   for (int i = tid; i < 3 * kMlpHidden; i += 256) S.b[i / kMlpHidden][i % kMlpHidden] = P.b[i / kMlpHidden][i % kMlpHidden];
   if (tid < kMlpOut) S.b3[tid] = P.b[3][tid];
-  float sum[3][4][2], sum3[2] = {0.f, 0.f}, loss = 0.f;
+  float sum[3][4][2], sum3 = 0.f, loss = 0.f;
 #pragma unroll
   for (int l = 0; l < 3; ++l)
 #pragma unroll
@@ -182,7 +190,7 @@ __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
         gr = 2.f * e * P.inv_n;
         loss += e * e * P.inv_n;
       }
-      sum3[0] += gr;
+      sum3 += gr;
       const bf16 gq = __float2bfloat16(gr);
       S.dy[r][j] = __bfloat162float(gq);
       if (r < live) P.dz[3][(row0 + r) * kMlpOut + j] = gq;
@@ -221,6 +229,7 @@ __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
       if (l > 0) __syncthreads();
     }
   }
+  float* sums = P.sums + (2 * static_cast<int64_t>(blockIdx.x) + (warp >> 2)) * kSumCols;
 #pragma unroll
   for (int l = 0; l < 3; ++l)
 #pragma unroll
@@ -230,16 +239,22 @@ __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
         float v = sum[l][nt][e];
 #pragma unroll
         for (int off = 4; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (g == 0) atomicAdd(P.gb[l] + n0 + 8 * nt + 2 * t4 + e, v);
+        if (g == 0) sums[kMlpHidden * l + n0 + 8 * nt + 2 * t4 + e] = v;
       }
-  {
-    float v = sum3[0];
+  // the output layer's bias and the loss: the warps' parts through S.dy, which
+  // the last tile has read before its last barrier
+  float v = sum3;
 #pragma unroll
-    for (int off = 8; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane < kMlpOut) atomicAdd(P.gb[3] + lane, v);
+  for (int off = 8; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
-    if (lane == 0) atomicAdd(P.loss, loss);
+  for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
+  if (lane < kMlpOut) S.dy[warp][lane] = v;
+  if (lane == 0) S.dy[8 + warp][0] = loss;
+  __syncthreads();
+  if ((warp & 3) == 0 && lane <= kMlpOut) {
+    float t = 0.f;
+    for (int k = 0; k < 4; ++k) t += lane < kMlpOut ? S.dy[warp + k][lane] : S.dy[8 + warp + k][0];
+    sums[3 * kMlpHidden + lane] = t;
   }
 }
 
@@ -247,16 +262,31 @@ __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
 // tile x of the 12 tiles of 64 x 64 (of 64 x 8 for the output layer) and every
 // gridDim.y-th chunk of 256 rows from chunk y on, read whole (16 bytes a load) before
 // its products; 8 warps of 16 x 32 outputs. Few output tiles and long sums: the
-// split over the rows is what fills the device. (Four launches of one layer
+// split over the rows is what fills the device; below 1,024 rows two parts at
+// most, whose sum does not depend on which comes first. Tile 12: the sums that
+// the rows' pass left, a warp a column, in a fixed order. (Four launches of one layer
 // each, whose operands were read two bytes at a time across rows, took 123 us
 // at 4,096 rows; this one takes 7 us.)
-constexpr int kGradChunk = 256, kGradPad = 72;
+constexpr int kGradChunk = 256, kGradPad = 72, kGradTiles = 12;
 __global__ void __launch_bounds__(256) train_weights_kernel(TrainArgs P, float* __restrict__ g0, float* __restrict__ g1,
                                                             float* __restrict__ g2, float* __restrict__ g3) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* As = reinterpret_cast<bf16*>(smem_raw);
   bf16* Ds = As + kGradChunk * kGradPad;
   const int tile = blockIdx.x;
+  if (tile == kGradTiles) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int c = blockIdx.y * 8 + warp; c < kSumCols; c += 8 * gridDim.y) {
+      float v = 0.f;
+      for (int k = lane; k < 2 * P.row_blocks; k += 32) v += P.sums[static_cast<int64_t>(k) * kSumCols + c];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      if (lane == 0)
+        *(c < 3 * kMlpHidden ? P.gb[c / kMlpHidden] + c % kMlpHidden
+                             : (c < kSumCols - 1 ? P.gb[3] + c - 3 * kMlpHidden : P.loss)) = v;
+    }
+    return;
+  }
   const int l = tile < 2 ? 0 : (tile < 6 ? 1 : (tile < 10 ? 2 : 3));
   const int q = tile - (l == 0 ? 0 : (l == 1 ? 2 : (l == 2 ? 6 : 10)));
   const int im = l == 0 ? 0 : (l == 3 ? 64 * q : 64 * (q >> 1)), in = l == 3 ? 0 : 64 * (q & 1);
@@ -427,6 +457,8 @@ void Mlp::release() {
   }
   cudaFree(grads);
   grads = nullptr;
+  cudaFree(sums);
+  sums = nullptr;
   cudaFree(ws);
   ws = nullptr;
   ws_rows = 0;
@@ -522,6 +554,10 @@ int Mlp::forward_backward(int B, const float* Xf, const void* Xb, const float* T
   }
   MLP_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   MLP_TRY(cudaError_t(ensure_ws(B)));
+  if (!sums) {
+    MLP_TRY(cudaMalloc(&sums, static_cast<size_t>(2) * sms * kSumCols * sizeof(float)));
+    sums_blocks = sms;
+  }
   TrainArgs P;
   bf16* f = static_cast<bf16*>(ws);
   P.h[0] = Xf ? f : static_cast<bf16*>(const_cast<void*>(Xb));
@@ -542,9 +578,12 @@ int Mlp::forward_backward(int B, const float* Xf, const void* Xb, const float* T
   P.inv_n = 1.0f / std::max(1, n_valid);
   MLP_TRY(cudaMemsetAsync(grads, 0, (kMlpParams + 1) * sizeof(float), s));
   const int tiles = (B + kTrainRows - 1) / kTrainRows, chunks = (B + kGradChunk - 1) / kGradChunk;
-  train_rows_kernel<<<std::min(tiles, sms), 256, sizeof(TrainSmem), s>>>(P);
+  P.sums = sums;
+  P.row_blocks = std::min(tiles, sums_blocks);
+  train_rows_kernel<<<P.row_blocks, 256, sizeof(TrainSmem), s>>>(P);
   MLP_TRY(cudaGetLastError());
-  train_weights_kernel<<<dim3(12, std::min(chunks, 32)), 256, kGradSmem, s>>>(P, gW[0], gW[1], gW[2], gW[3]);
+  train_weights_kernel<<<dim3(kGradTiles + 1, std::min(chunks, B < 1024 ? 2 : 32)), 256, kGradSmem, s>>>(
+      P, gW[0], gW[1], gW[2], gW[3]);
   return int(cudaGetLastError());
 }
 

@@ -34,6 +34,8 @@ struct Mlp {
   void* Wb[4] = {nullptr, nullptr, nullptr, nullptr};
   // gradients in the flat parameter order (layer 0: 48 rows), then the batch loss
   float* grads = nullptr;
+  float* sums = nullptr;  // the training pass's per-block parts of bias gradients and loss
+  int sums_blocks = 0;    // blocks that it has room for
   float* gW[4] = {nullptr, nullptr, nullptr, nullptr};
   float* mW[4] = {nullptr, nullptr, nullptr, nullptr};
   float* vW[4] = {nullptr, nullptr, nullptr, nullptr};

@@ -27,6 +27,7 @@ int fail(ho_context* c, int code, const std::string& msg) {
 }
 
 int cuda_fail(ho_context* c, int e, const char* what) {
+  cudaGetLastError();  // the next call's launches are not to find this error
   return fail(c, HO_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(static_cast<cudaError_t>(e)));
 }
 

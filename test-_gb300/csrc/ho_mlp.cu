@@ -530,6 +530,7 @@ int Mlp::ensure_ws(int rows) {
   if (rows <= ws_rows) return 0;
   cudaFree(ws);
   ws = nullptr;
+  ws_rows = 0;
   // X (64 wide), H1..H3 and dZ0..dZ2 (128 wide), dY (8 wide), in BF16
   MLP_TRY(cudaMalloc(&ws, static_cast<size_t>(rows) * (kMlpInPad + 6 * kMlpHidden + kMlpOut) * sizeof(bf16)));
   ws_rows = rows;

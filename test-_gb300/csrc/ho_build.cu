@@ -237,7 +237,14 @@ int launch_setup(ho_context* c) {
 //    2 beta / (1 - beta), while the segment from xi to xi* stays in the cube.
 //    So from any start with |xi| <= S where rho + q (S + rho) <= R (the cold
 //    start 0 is one) the iterates approach xi*: where they stop, they are at
-//    xi*. No sample of a certified element converges anywhere else.
+//    xi*. No cold-started sample of a certified element converges anywhere else,
+//    and none from a start within S. A network-started sample that fails goes
+//    on from its converged neighbours, and those starts may lie outside S (|xi|
+//    up to rho, beyond it where one neighbour is extrapolated): such a solve
+//    may, for all that is shown here, end at another point that maps to x, but
+//    that one lies outside the cube. So what an excluded search of network
+//    starts could still have bracketed is no isosurface point of the element:
+//    on the segment, the field at the points of the cube clears the isovalue.
 // The cube reaches at least to 1.5, the clamp of the face Newton's iterates.
 // The field there is its trilinear part, exactly interpolated by the test,
 // plus the higher modes, at most H = sum |c_ijk| V_i V_j V_k over |xi| <= rho.

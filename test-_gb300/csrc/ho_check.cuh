@@ -19,18 +19,6 @@
 
 namespace ho {
 
-// True when the hit passes the FP64 check (a miss always passes).
-template <int N>
-__device__ bool fp64_check(const TraceParams& P, float3 o, float3 d, float iso, const HitState& h) {
-  if (h.kind == HO_HIT_MISS) return true;
-  const bool iso_hit = h.kind != HO_HIT_FACE;
-  double r, u;
-  fp64_residuals<N>(P.rec, h.elem, o, d, h.t, h.xi, iso_hit, r, u);
-  if (!iso_hit) return r <= kCheckFaceTol;
-  if (r > kCheckIsoPosTol) return false;
-  return fabs(u - static_cast<double>(iso)) <= kCheckIsoFieldTol;
-}
-
 // The check's residuals for given hits (ho_hit_residuals): per hit the
 // position residual and the field value at its xi.
 template <int N>

@@ -742,10 +742,12 @@ __device__ bool find_iso_warp(const Elem<N, SM>& e, float3 o, float3 d, float t0
 }
 
 // True when the isosurface search of a candidate's segment [te, tx] cannot
-// find a sign change, from the element's certificate (cull_kernel in
-// ho_build.cu has the proof): every sample whose Newton solve converges has
-// xi within delta of y = K (x - x0), which is linear in t, and a field value
-// within H of the trilinear interpolant of the element's corner values there.
+// find a sign change that is an isosurface point of the element, from the
+// element's certificate (cull_kernel in ho_build.cu has the proof, and what it
+// leaves open for restarted network starts): every sample whose Newton solve
+// converges has xi within delta of y = K (x - x0), which is linear in t, and a
+// field value within H of the trilinear interpolant of the element's corner
+// values there.
 // So u - iso keeps one sign over the segment when those bounds clear the
 // isovalue on one side over the boxes around its four quarters (a trilinear
 // function on a box has its extremes at the box's corners), and the 17
@@ -1192,14 +1194,7 @@ __device__ void visit_candidate(const Elem<N, SM>& e, const float* __restrict__ 
       float3 x;
       float J[9];
       geom_eval<N>(e, xi, x, J, w);
-      const float3 dr = make_float3(J[0], J[3], J[6]), ds = make_float3(J[1], J[4], J[7]),
-                   dt = make_float3(J[2], J[5], J[8]);
-      float3 n;
-      if (fabsf(xi.x) > 0.9f) n = cross3(ds, dt);
-      else if (fabsf(xi.y) > 0.9f) n = cross3(dr, dt);
-      else n = cross3(dr, ds);
-      n = normalize3(n);
-      if (n.x * d.x + n.y * d.y + n.z * d.z > 0.f) n = make_float3(-n.x, -n.y, -n.z);
+      const float3 n = face_normal(J, xi, d);
       note_tie(best, best.t, th, tie);
       best.t = th;
       best.elem = eidx;
@@ -1398,7 +1393,7 @@ __device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox,
       best.flags &= ~kFlagPost;
       best.xi = xi;
       best.n = n;
-      float4 r[4];  // the field at the root, as the round kernel's post evaluation
+      float4 r[4];  // the field at the root: what fill_hit gives the round kernel's hits
       eval_comps<N, SM>(e.c, xi, 3, 4, r);
       best.u = r[3].x;
     }
@@ -1410,18 +1405,12 @@ __device__ void visit_warp(const Elem<N, SM>& e, const float* __restrict__ fbox,
   wu.cyc[3] += clock64() - c0;
   if (fh) {
     if (th > 0.001f && th < best.t) {
-      // geometry (and field) at the hit, as the round kernel's post evaluation
+      // geometry (and field) at the hit: what fill_hit gives the round kernel's hits
       float4 r[4];
       eval_comps<N, SM>(e.c, xi, 0, e.has_field ? 4 : 3, r);
       ++wu.geom;
-      const float3 dr = make_float3(r[0].y, r[1].y, r[2].y), ds = make_float3(r[0].z, r[1].z, r[2].z),
-                   dt = make_float3(r[0].w, r[1].w, r[2].w);
-      float3 n;
-      if (fabsf(xi.x) > 0.9f) n = cross3(ds, dt);
-      else if (fabsf(xi.y) > 0.9f) n = cross3(dr, dt);
-      else n = cross3(dr, ds);
-      n = normalize3(n);
-      if (n.x * d.x + n.y * d.y + n.z * d.z > 0.f) n = make_float3(-n.x, -n.y, -n.z);
+      const float J[9] = {r[0].y, r[0].z, r[0].w, r[1].y, r[1].z, r[1].w, r[2].y, r[2].z, r[2].w};
+      const float3 n = face_normal(J, xi, d);
       note_tie(best, best.t, th, tie);
       best.t = th;
       best.elem = eidx;

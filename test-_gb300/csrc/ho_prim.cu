@@ -236,12 +236,13 @@ struct PrimHeavy {
   uint32_t iters;
   PrimState s;
 };
+static_assert(sizeof(PrimHeavy) == 36, "what a handed-over query takes, below");
 // Iterations after which a query is handed over. A quad's or a triangle's
 // start search takes 1,000 to 4,000 iterations when it finds nothing; on one
 // thread a ray that passes several such surfaces ran for hundreds of
 // milliseconds after the others had ended. (32, 96 and 1,024 measure within 2%.)
 constexpr uint32_t kPrimBudget = 256;
-// Most queries handed over in a call (40 bytes each); the others run to their
+// Most queries handed over in a call (36 bytes each); the others run to their
 // end where they are.
 constexpr int64_t kPrimHeavyMost = int64_t(1) << 22;
 

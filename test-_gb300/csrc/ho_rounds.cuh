@@ -902,7 +902,7 @@ __global__ void __launch_bounds__(kRoundBlock) round_kernel(RoundParams P) {
                   s.cap = 50;
                 }
                 s.it = 0;
-                          end = 0;
+                end = 0;
               }
             }
           } else {

@@ -108,7 +108,7 @@ struct TrainArgs {
 // What bounds it is the chain of six small products and their barriers; the
 // products are 0.6 GFLOP at 4,096 rows. As separate launches per layer (product,
 // bias and activation, slope, column sums) the pass ran 28 kernels, 200 us at
-// 4,096 rows; this one takes 18 us.
+// 4,096 rows; this one takes 16 us (19 with its bias gradients by atomics).
 __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) train_rows_kernel(TrainArgs P) {
 // most, whose sum does not depend on which comes first. Tile 12: the sums that
 // the rows' pass left, a warp a column, in a fixed order. (Four launches of one layer
 // each, whose operands were read two bytes at a time across rows, took 123 us
-// at 4,096 rows; this one takes 7 us.)
+// at 4,096 rows; this one takes 10 us, 7 of them without tile 12.)
 constexpr int kGradChunk = 256, kGradPad = 72, kGradTiles = 12;
 __global__ void __launch_bounds__(256) train_weights_kernel(TrainArgs P, float* __restrict__ g0, float* __restrict__ g1,
                                                             float* __restrict__ g2, float* __restrict__ g3) {
